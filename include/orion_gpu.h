@@ -44,8 +44,8 @@ extern "C" {
 #define ORION_SWEEP_PLANES 0   /* one launch per hyperplane */
 #define ORION_SWEEP_GRID 1     /* one cooperative launch, bounded grid barrier per hyperplane */
 #define ORION_SWEEP_CLUSTER 2  /* thread-block clusters (8 or 16 CTAs), cluster barrier per hyperplane */
-#define ORION_SWEEP_TILES 3    /* one launch per pass: 32x4-line tiles, each waiting only on its upstream
-                                  neighbour tiles' progress (bounded waits); the default */
+#define ORION_SWEEP_TILES 3    /* one launch per pass: tiles of up to 112 grid lines, each waiting only on its
+                                  upstream neighbour tiles' increments (bounded waits); the default */
 
 /* BC types (src/bc/PhysicalBC.cpp:576-613) */
 #define ORION_BC_INTERFACE (-1)

@@ -80,14 +80,12 @@ struct DeviceLists {
   int* cl_nplanes = nullptr;                     // hyperplanes of each group
   long long spin_limit = 1LL << 21;              // polls before a grid barrier gives up (about a second)
   // tile wavefront sweeps (sweep_tiles.cuh): per direction the tile list in
-  // ticket order, and one control block (ticket + progress per tile) reset
-  // before every pass
+  // ticket order, and the ticket counters (the last CTA of a pass clears them)
   bool tiles_on = false;
   void* sweep_tiles[2] = {nullptr, nullptr};     // SweepTile lists, forward / backward
   int n_sweep_tiles[2] = {0, 0};
-  void* tile_ctl = nullptr;                      // TileCtl with max(n_sweep_tiles) progress words
-  size_t tile_ctl_bytes = 0;
-  int tile_k = 4;                                // k rows per tile (32 j rows)
+  void* tile_ctl = nullptr;                      // TileCtl
+  int tile_lines = 0;                            // lines of the largest tile
   int max_planes = 0;
   long long* halo_src = nullptr;
   long long* halo_dst = nullptr;
@@ -180,6 +178,7 @@ struct orion_case_s {
   std::vector<orion::BlockDev<float>> bd32;
   void* d_blocks = nullptr;
   orion::DeviceLists L;
+  int sweep_arrays = -1;  // whose arrays the sweeps' shared memory holds: 1 the tile form's, 0 the plane-major ones, -1 neither
   orion::ShardLists shard;
   long long total_interior = 0;
   cudaGraphExec_t graph = nullptr;
@@ -228,6 +227,7 @@ struct StageOps {
   int (*step)(orion_case_t, bool with_q);
   int (*init_flow)(orion_case_t, uint64_t seed, double amp);
   int (*skew_static)(orion_case_t, int block);
+  int (*sweep_arrays)(orion_case_t, bool tiles);
   int (*persistent_grid)(orion_case_t);
   int (*schedule)(orion_case_t, int form, int cluster_size);
   int (*prim_shadow)(orion_case_t, int block);

@@ -1,5 +1,7 @@
 // Device-side descriptors shared by the kernels and the host runtime.
 #pragma once
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 namespace orion {
@@ -60,11 +62,19 @@ struct BlockDev {
   // Coefficients of the flux splitting that do not involve the swept increment
   // (computed once per step, off the sweeps' critical path):
   S* sk_nrm;              // 9 (static): unit normal nx_n,ny_n,nz_n of the point's xi, eta, zeta metrics
-  S* sk_nbq;              // 8: u, v, w, H, c^2, (gamma-1)/2 v^2, c, 2 mu/(|Re| rho vol + 1e-30) of the point as
-                          // somebody's neighbour
+  S* sk_nbq;              // 6: u, v, w, H, c^2, (gamma-1)/2 v^2 of the point as somebody's neighbour
   S* sk_pair;             // 30: per face neighbour q (lower i,j,k, upper i,j,k): l1, x1, x2, ct_n, rv/2
-  S* sk_gm;               // 3 (static): |grad xi|, |grad eta|, |grad zeta| of the point's metrics
-  S* sk_inv;              // 3 (static): 1 / max(|grad .|, 1e-30)
+  // The tile form's own copies (sweep_tiles.cuh), in the order its tiles walk
+  // them: tile, wave, 16-byte piece, line.  They share memory with the
+  // plane-major arrays above: only the form in use keeps its arrays.
+  char* tl_own;           // static metrics, diagonal coefficient and masked RHS
+  char* tl_nb;            // the state a neighbour's term needs, and the increment being swept
+  char* tl_edge;          // increments handed from tile to tile
+  long long nrec;         // edge records
+  int tJ;                 // tiles along j
+  const int4* t_j;        // per j: tile column, line within it, its width
+  const int4* t_k;        // per k: tile row, line within it, its height
+  const long long* t_base;  // first slot of tile (a, b) at b * tJ + a
   // the parameters of the block's case: kernels read them here, with the
   // block's other fields (no further dependent load), so one launch can
   // cover the blocks of several cases (orion_group_*)

@@ -1168,24 +1168,55 @@ __global__ void k_skew_static(const BlockDev<S>* __restrict__ blocks, int b) {
       B.sk_nrm[(3 * d) * B.ncomp + c] = nx * inv_mag;
       B.sk_nrm[(3 * d + 1) * B.ncomp + c] = ny * inv_mag;
       B.sk_nrm[(3 * d + 2) * B.ncomp + c] = nz * inv_mag;
-      // the unclamped magnitude the spectral radius uses, and the reciprocal of the clamped one
-      B.sk_gm[d * B.ncomp + c] = sqrt_s(nx * nx + ny * ny + nz * nz);
-      B.sk_inv[d * B.ncomp + c] = inv_mag;
     }
   }
 }
 
-// Prep: gather prim, mu into the skewed layout; rhs = dq with physical-BC
-// windows zeroed (set_boundary_dq_zero + the AoS copy, StateUpdater.cpp:447-570);
-// diagonal coefficient 1/(1/dt + sum of radii) (get_diag_coeff :267-295), the
-// same in all four sweeps.
-template <typename S, typename T, bool PAIRS = true>
+// What the sweeps need of one point besides its RHS: the diagonal coefficient
+// 1/(1/dt + sum of radii) (get_diag_coeff, StateUpdater.cpp:267-295), the same
+// in all four sweeps, and its quantities as a neighbour in
+// compute_flux_splitting (:217-253) and visc_spectral_radius (:194-207).
+template <typename T>
+struct PrepPoint {
+  T coed, H, c2, af, c, vcoef;
+  __device__ __forceinline__ void form(const ParamsDev& P, T rho, T u, T v, T w, T p, const T km[9], T mu, T vol, T dt) {
+    const T gamma = T(P.gamma), reynolds = T(P.reynolds);
+    const T ra = spectral_radius<T>(rho, u, v, w, p, gamma, km[0], km[1], km[2]);
+    const T rb = spectral_radius<T>(rho, u, v, w, p, gamma, km[3], km[4], km[5]);
+    const T rc = spectral_radius<T>(rho, u, v, w, p, gamma, km[6], km[7], km[8]);
+    T rva = T(0), rvb = T(0), rvc = T(0);
+    vcoef = T(0);
+    T rm = rho, pm = p;
+    if (rm < T(1e-30)) rm = T(1e-30);
+    if (pm < T(1e-30)) pm = T(1e-30);
+    if (P.nvis == 1) {
+      if (vol < T(1e-30)) vol = T(1e-30);
+      const T rm_vol = rm * vol;
+      vcoef = T(2) * mu / (tabs(reynolds) * rm_vol + T(1.0e-30));
+      rva = visc_spectral_radius<T>(rho, mu, vol, reynolds, km[0], km[1], km[2]);
+      rvb = visc_spectral_radius<T>(rho, mu, vol, reynolds, km[3], km[4], km[5]);
+      rvc = visc_spectral_radius<T>(rho, mu, vol, reynolds, km[6], km[7], km[8]);
+    }
+    const T rad_sum = ra + rb + rc + rva + rvb + rvc;
+    const T term = (T(1) / dt) + rad_sum;
+    coed = T(1) / term;
+    const T v2 = u * u + v * v + w * w;
+    c2 = gamma * pm / rm;
+    H = (gamma / (gamma - T(1))) * (pm / rm) + T(0.5) * v2;
+    af = T(0.5) * (gamma - T(1)) * v2;
+    c = tsqrt(c2);
+  }
+};
+
+// Prep of the plane-major forms: gather prim, mu into the skewed layout; rhs =
+// dq with physical-BC windows zeroed (set_boundary_dq_zero + the AoS copy,
+// StateUpdater.cpp:447-570).
+template <typename S, typename T>
 __global__ void __launch_bounds__(256, PointwiseMinBlocks<T>::n) k_lusgs_prep(const BlockDev<S>* __restrict__ blocks, const Chunk* __restrict__ chunks) {
   const Chunk ch = chunks[blockIdx.x];
   const BlockDev<S> B = blocks[ch.block];
   const ParamsDev& P = B.prm;
   const long long np = B.npad, nc = B.ncomp;
-  const T gamma = T(P.gamma), reynolds = T(P.reynolds);
   for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
     const long long c = ch.start + t;
     const int nat = B.sk_nat[c];
@@ -1194,56 +1225,24 @@ __global__ void __launch_bounds__(256, PointwiseMinBlocks<T>::n) k_lusgs_prep(co
     const S* pr = FluxSrc<S>::prim(B);
     const T rho = (T)pr[nat], u = (T)pr[np + nat], v = (T)pr[2 * np + nat], w = (T)pr[3 * np + nat],
             p = (T)pr[4 * np + nat];
-    if (PAIRS) {  // the operands of k_sweep_pairs
-      B.sk_prim[c] = (S)rho;
-      B.sk_prim[nc + c] = (S)u;
-      B.sk_prim[2 * nc + c] = (S)v;
-      B.sk_prim[3 * nc + c] = (S)w;
-      B.sk_prim[4 * nc + c] = (S)p;
-    }
+    B.sk_prim[c] = (S)rho;  // the operands of k_sweep_pairs
+    B.sk_prim[nc + c] = (S)u;
+    B.sk_prim[2 * nc + c] = (S)v;
+    B.sk_prim[3 * nc + c] = (S)w;
+    B.sk_prim[4 * nc + c] = (S)p;
     T km[9];
     for (int m = 0; m < 9; ++m) km[m] = (T)B.sk_metrics[m * nc + c];
-    const T ra = spectral_radius<T>(rho, u, v, w, p, gamma, km[0], km[1], km[2]);
-    const T rb = spectral_radius<T>(rho, u, v, w, p, gamma, km[3], km[4], km[5]);
-    const T rc = spectral_radius<T>(rho, u, v, w, p, gamma, km[6], km[7], km[8]);
-    T rva = T(0), rvb = T(0), rvc = T(0);
     const T mu = (T)B.mu[nat];
-    if (PAIRS) B.sk_mu[c] = (S)mu;
-    T vcoef = T(0);
-    if (P.nvis == 1) {
-      T vol = (T)B.sk_vol[c];
-      if (vol < T(1e-30)) vol = T(1e-30);
-      {  // the neighbour factor of visc_spectral_radius (StateUpdater.cpp:194-207)
-        T rc = rho;
-        if (rc < T(1e-30)) rc = T(1e-30);
-        const T rm_vol = rc * vol;
-        vcoef = T(2) * mu / (tabs(reynolds) * rm_vol + T(1.0e-30));
-      }
-      rva = visc_spectral_radius<T>(rho, mu, vol, reynolds, km[0], km[1], km[2]);
-      rvb = visc_spectral_radius<T>(rho, mu, vol, reynolds, km[3], km[4], km[5]);
-      rvc = visc_spectral_radius<T>(rho, mu, vol, reynolds, km[6], km[7], km[8]);
-    }
-    const T rad_sum = ra + rb + rc + rva + rvb + rvc;
-    const T term = (T(1) / (T)B.dt[nat]) + rad_sum;
-    B.sk_coed[c] = (S)(T(1) / term);
-    // the point's quantities as a neighbour in compute_flux_splitting (StateUpdater.cpp:217-253)
-    {
-      T rm = rho, pm = p;
-      const T v2 = u * u + v * v + w * w;
-      if (rm < T(1e-30)) rm = T(1e-30);
-      if (pm < T(1e-30)) pm = T(1e-30);
-      const T c2 = gamma * pm / rm;
-      const T H = (gamma / (gamma - T(1))) * (pm / rm) + T(0.5) * v2;
-      const T af = T(0.5) * (gamma - T(1)) * v2;
-      B.sk_nbq[c] = (S)u;
-      B.sk_nbq[nc + c] = (S)v;
-      B.sk_nbq[2 * nc + c] = (S)w;
-      B.sk_nbq[3 * nc + c] = (S)H;
-      B.sk_nbq[4 * nc + c] = (S)c2;
-      B.sk_nbq[5 * nc + c] = (S)af;
-      B.sk_nbq[6 * nc + c] = (S)tsqrt(c2);
-      B.sk_nbq[7 * nc + c] = (S)vcoef;
-    }
+    B.sk_mu[c] = (S)mu;
+    PrepPoint<T> q;
+    q.form(P, rho, u, v, w, p, km, mu, (T)B.sk_vol[c], (T)B.dt[nat]);
+    B.sk_coed[c] = (S)q.coed;
+    B.sk_nbq[c] = (S)u;
+    B.sk_nbq[nc + c] = (S)v;
+    B.sk_nbq[2 * nc + c] = (S)w;
+    B.sk_nbq[3 * nc + c] = (S)q.H;
+    B.sk_nbq[4 * nc + c] = (S)q.c2;
+    B.sk_nbq[5 * nc + c] = (S)q.af;
   }
 }
 
@@ -1814,12 +1813,50 @@ __device__ __forceinline__ void block_reduce_res(double& sum, double& mx, long l
 #ifndef ORION_FINISH_MINB
 #define ORION_FINISH_MINB 4
 #endif
-template <typename S, bool DO_RES, int NT>
+// Where interior point (ii, jj, kk) is in the block's tile arrays
+// (sweep_tiles.cuh): slot of its wave's first line, its line, lines per wave.
+struct TileSlot {
+  long long wave;
+  int line, nl;
+  // its first piece in an array of `pieces` per point; pieces nl apart
+  template <typename V>
+  __device__ __forceinline__ V* run(char* base, int pieces) const {
+    return reinterpret_cast<V*>(base) + wave * pieces + line;
+  }
+};
+template <typename S>
+__device__ __forceinline__ TileSlot tile_slot(const BlockDev<S>& B, int ii, int jj, int kk) {
+  const int4 a = __ldg(B.t_j + jj), b = __ldg(B.t_k + kk);  // {tile column, line in it, width}, {tile row, ...}
+  const int nl = a.z * b.z;
+  return TileSlot{__ldg(B.t_base + b.x * B.tJ + a.x) + (long long)(ii + a.y + b.y) * nl, b.y * a.z + a.y, nl};
+}
+// The swept increment of a point.
+__device__ __forceinline__ void tile_increment(const BlockDev<float>& B, const TileSlot& at, float d[5]) {
+  const float4* const p = at.run<float4>(B.tl_nb, 3);
+  const float4 a = __ldcs(p + 2 * at.nl);
+  d[0] = a.x;
+  d[1] = a.y;
+  d[2] = a.z;
+  d[3] = a.w;
+  d[4] = __ldcs(reinterpret_cast<const float*>(p + at.nl) + 3);
+}
+__device__ __forceinline__ void tile_increment(const BlockDev<double>& B, const TileSlot& at, double d[5]) {
+  const double2* const p = at.run<double2>(B.tl_nb, 8);
+  const double2 a = __ldcs(p + 5 * at.nl), b = __ldcs(p + 6 * at.nl);
+  d[0] = a.x;
+  d[1] = a.y;
+  d[2] = b.x;
+  d[3] = b.y;
+  d[4] = __ldcs(reinterpret_cast<const double*>(p + 7 * at.nl));
+}
+
+template <typename S, bool DO_RES, bool TILES, int NT>
 __global__ void __launch_bounds__(NT, ORION_FINISH_MINB) k_sweep_finish(const BlockDev<S>* __restrict__ blocks,
                                                      const Chunk* __restrict__ chunks, ResPartial* __restrict__ partials) {
   // Natural order (interior index n = i + ni*(j + nj*k)): prim, dq, vol, dt
   // and the mask are read and written coalesced; only the swept increment is
-  // gathered from the plane-major layout, at c = koff[s*nk + k] + (j - jlo(s,k)).
+  // gathered, from its tile slot or from the plane-major layout at
+  // c = koff[s*nk + k] + (j - jlo(s,k)).
   const Chunk ch = chunks[blockIdx.x];
   const BlockDev<S> B = blocks[ch.block];
   const ParamsDev& P = B.prm;
@@ -1831,13 +1868,19 @@ __global__ void __launch_bounds__(NT, ORION_FINISH_MINB) k_sweep_finish(const Bl
     const int n32 = (int)n, r32 = n32 / B.ni;
     const int ii = n32 - r32 * B.ni, jj = r32 % B.nj, kk = r32 / B.nj;
     const long long idx = lin(B, NG + ii, NG + jj, NG + kk);
-    const int sp = ii + jj + kk;
-    const int jlo = sp - kk - (B.ni - 1) > 0 ? sp - kk - (B.ni - 1) : 0;
-    const long long c = (long long)__ldg(B.koff + (long long)sp * B.nk + kk) + (jj - jlo);
+    S sw[5];
+    if (TILES) {
+      tile_increment(B, tile_slot(B, ii, jj, kk), sw);
+    } else {
+      const int sp = ii + jj + kk;
+      const int jlo = sp - kk - (B.ni - 1) > 0 ? sp - kk - (B.ni - 1) : 0;
+      const long long c = (long long)__ldg(B.koff + (long long)sp * B.nk + kk) + (jj - jlo);
+      for (int m = 0; m < 5; ++m) sw[m] = __ldcs(B.sk_dq + m * nc + c);
+    }
     double dq[5];
     const bool masked = B.bcmask[idx] != 0;
     for (int m = 0; m < 5; ++m) {
-      const S v = masked ? (S)0 : __ldcs(B.sk_dq + m * nc + c);
+      const S v = masked ? (S)0 : sw[m];
       B.dq[m * np + idx] = v;
       dq[m] = (double)v;
     }

@@ -80,8 +80,12 @@ size_t block_bytes(const HostBlock& b, size_t ssz) {
   add((npl * b.kdim + 1) * 4);  // koff
   add(nc * 4);                  // sk_nat
   add(6 * nc * 4);              // sk_nb
-  add(80 * nc * ssz);           // sk_metrics 9, sk_vol, sk_prim 5, sk_mu, sk_coed, sk_rhs 5, sk_dq 5, sk_nrm 9, sk_nbq 8,
-                                // sk_pair 30, sk_gm 3, sk_inv 3
+  const TilePlan p = make_tile_plan(b.idim, b.jdim, b.kdim, ssz);
+  add(16 * (size_t)(b.jdim + b.kdim));  // t_j, t_k
+  add(8 * p.base.size());               // t_base
+  // one area for the form in use: sk_metrics 9, sk_vol, sk_prim 5, sk_mu, sk_coed, sk_rhs 5, sk_dq 5, sk_nrm 9,
+  // sk_nbq 6, sk_pair 30, or the tile arrays
+  add(std::max((size_t)kPlaneComps * nc * ssz, tile_array_bytes(p.slots, p.records, ssz)));
   return align_up(s, 256);
 }
 
@@ -118,7 +122,18 @@ void carve_block(char* base, const HostBlock& b, BlockDev<S>& d) {
   d.koff = reinterpret_cast<int*>(take(((size_t)npl * b.kdim + 1) * 4));
   d.sk_nat = reinterpret_cast<int*>(take(nc * 4));
   d.sk_nb = reinterpret_cast<int*>(take(6 * nc * 4));
-  S* sk = reinterpret_cast<S*>(take(80 * nc * sizeof(S)));
+  const TilePlan p = make_tile_plan(b.idim, b.jdim, b.kdim, sizeof(S));
+  const TileBytes tb = tile_bytes(sizeof(S));
+  d.t_j = reinterpret_cast<int4*>(take(16 * (size_t)(b.jdim + b.kdim)));
+  d.t_k = d.t_j + b.jdim;
+  d.t_base = reinterpret_cast<long long*>(take(8 * p.base.size()));
+  d.tJ = p.nJ();
+  d.nrec = p.records;
+  char* area = take(std::max((size_t)kPlaneComps * nc * sizeof(S), tile_array_bytes(p.slots, p.records, sizeof(S))));
+  d.tl_own = area;
+  d.tl_nb = d.tl_own + align_up(tb.own * (size_t)p.slots, 256);
+  d.tl_edge = d.tl_nb + align_up(tb.nb * (size_t)p.slots, 256);
+  S* sk = reinterpret_cast<S*>(area);
   d.sk_metrics = sk;
   d.sk_vol = sk + 9 * nc;
   d.sk_prim = sk + 10 * nc;
@@ -128,9 +143,7 @@ void carve_block(char* base, const HostBlock& b, BlockDev<S>& d) {
   d.sk_dq = sk + 22 * nc;
   d.sk_nrm = sk + 27 * nc;
   d.sk_nbq = sk + 36 * nc;
-  d.sk_pair = sk + 44 * nc;
-  d.sk_gm = sk + 74 * nc;
-  d.sk_inv = sk + 77 * nc;
+  d.sk_pair = sk + 42 * nc;
   d.prm = ParamsDev{};  // set by the caller: the case's parameters
   d.ni = b.idim;
   d.nj = b.jdim;
@@ -299,72 +312,70 @@ int build_line_tiles(orion_case_t c) {
   return 0;
 }
 
-// Tile wavefront sweeps: tiles of 32 x TK grid lines (TK per precision,
-// TileShape), per direction in ticket order.  A tile's start in steps is
-// 32 J + TK K behind its
-// block's first tile, and its upstream tiles (J-1, K) and (J, K-1) start
-// strictly earlier, so ordering by start offset (ties by block, then J) is a
-// dependency-respecting order for every block at once.
+// Tile wavefront sweeps: every block's tiles (tile_plan.hpp), per direction in
+// ticket order.  A tile's first point is `start` waves behind its block's
+// first, and the tiles it waits for start strictly earlier, so ordering by
+// start (ties by block) respects the dependencies of every block at once.
 int build_sweep_tiles(orion_case_t c) {
   auto& L = c->L;
-  constexpr int TJ = 32;
-  const int TK = c->prec == ORION_PREC_FP64 ? TileShape<double>::TK : TileShape<float>::TK;
-  L.tile_k = TK;
-  int maxn = 0;
-  for (int dir = 0; dir < 2; ++dir) {
-    struct Item {
-      int start, block, J, K;
-    };
-    std::vector<Item> items;
-    std::vector<int> first(c->nblocks + 1, 0);
-    for (int b = 0; b < c->nblocks; ++b) {
-      const auto& h = c->hb[b];
-      const int nJ = (h.jdim + TJ - 1) / TJ, nK = (h.kdim + TK - 1) / TK;
-      for (int K = 0; K < nK; ++K)
-        for (int J = 0; J < nJ; ++J) items.push_back(Item{TJ * J + TK * K, b, J, K});
-    }
-    std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
-      if (a.start != b.start) return a.start < b.start;
-      if (a.block != b.block) return a.block < b.block;
-      return a.J < b.J;
-    });
-    // slot of (block, J, K)
-    std::vector<long long> base(c->nblocks + 1, 0);
-    std::vector<int> nJs(c->nblocks);
-    for (int b = 0; b < c->nblocks; ++b) {
-      const auto& h = c->hb[b];
-      nJs[b] = (h.jdim + TJ - 1) / TJ;
-      base[b + 1] = base[b] + (long long)nJs[b] * ((h.kdim + TK - 1) / TK);
-    }
-    std::vector<int> slot_of((size_t)base[c->nblocks], -1);
-    for (size_t q = 0; q < items.size(); ++q)
-      slot_of[(size_t)(base[items[q].block] + (long long)items[q].K * nJs[items[q].block] + items[q].J)] = (int)q;
-    std::vector<SweepTile> tiles(items.size());
-    for (size_t q = 0; q < items.size(); ++q) {
-      const Item& it = items[q];
-      const auto& h = c->hb[it.block];
-      SweepTile& w = tiles[q];
-      w = SweepTile{};
-      w.block = it.block;
-      w.jb = dir == 0 ? it.J * TJ : h.jdim - 1 - it.J * TJ;
-      w.kb = dir == 0 ? it.K * TK : h.kdim - 1 - it.K * TK;
-      const long long bb = base[it.block];
-      w.up_j = it.J > 0 ? slot_of[(size_t)(bb + (long long)it.K * nJs[it.block] + it.J - 1)] : -1;
-      w.up_k = it.K > 0 ? slot_of[(size_t)(bb + (long long)(it.K - 1) * nJs[it.block] + it.J)] : -1;
-      if ((w.up_j >= 0 && w.up_j >= (int)q) || (w.up_k >= 0 && w.up_k >= (int)q))
-        return fail(ORION_E_INVALID, "sweep tile order does not respect the dependencies");
-    }
-    int rc;
-    SweepTile* d = nullptr;
-    if ((rc = dev_upload(c, &d, tiles, true))) return rc;
-    L.sweep_tiles[dir] = d;
-    L.n_sweep_tiles[dir] = (int)tiles.size();
-    maxn = std::max(maxn, (int)tiles.size());
+  const size_t ssz = c->prec == ORION_PREC_FP64 ? 8 : 4;
+  std::vector<SweepTile> all;
+  L.tile_lines = 0;
+  for (int b = 0; b < c->nblocks; ++b) {
+    const auto& h = c->hb[b];
+    const TilePlan p = make_tile_plan(h.idim, h.jdim, h.kdim, ssz);
+    const int nJ = p.nJ(), nK = p.nK();
+    for (int K = 0; K < nK; ++K)
+      for (int J = 0; J < nJ; ++J) {
+        const size_t t = (size_t)K * nJ + J;
+        SweepTile w{};
+        w.block = b;
+        w.jw = p.jw(J);
+        w.kh = p.kh(K);
+        w.jb = p.jb[J];
+        w.kb = p.kb[K];
+        w.base = p.base[t];
+        if (J > 0) {
+          w.w[0] = p.jw(J - 1);
+          w.base_j[0] = p.base[t - 1];
+          w.edge_j[0] = p.ej[t - 1];
+        }
+        if (J + 1 < nJ) {
+          w.w[1] = p.jw(J + 1);
+          w.base_j[1] = p.base[t + 1];
+          w.edge_j[1] = p.ej[t];
+        }
+        if (K > 0) {
+          w.h[0] = p.kh(K - 1);
+          w.base_k[0] = p.base[t - nJ];
+          w.edge_k[0] = p.ek[t - nJ];
+        }
+        if (K + 1 < nK) {
+          w.h[1] = p.kh(K + 1);
+          w.base_k[1] = p.base[t + nJ];
+          w.edge_k[1] = p.ek[t];
+        }
+        L.tile_lines = std::max(L.tile_lines, w.jw * w.kh);
+        all.push_back(w);
+      }
   }
-  L.tile_ctl_bytes = offsetof(TileCtl, progress) + sizeof(unsigned int) * (size_t)maxn;
-  unsigned char* ctl = nullptr;
+  for (int dir = 0; dir < 2; ++dir) {
+    for (auto& w : all) {
+      const auto& h = c->hb[w.block];
+      w.start = dir == 0 ? w.jb + w.kb : (h.jdim - w.jb - w.jw) + (h.kdim - w.kb - w.kh);
+    }
+    std::stable_sort(all.begin(), all.end(), [](const SweepTile& x, const SweepTile& y) {
+      return x.start != y.start ? x.start < y.start : x.block < y.block;
+    });
+    SweepTile* d = nullptr;
+    int rc;
+    if ((rc = dev_upload(c, &d, all, true))) return rc;
+    L.sweep_tiles[dir] = d;
+    L.n_sweep_tiles[dir] = (int)all.size();
+  }
+  TileCtl* ctl = nullptr;
   int rc;
-  if ((rc = dev_alloc(c, &ctl, L.tile_ctl_bytes))) return rc;
+  if ((rc = dev_alloc(c, &ctl, 1))) return rc;
   L.tile_ctl = ctl;
   return 0;
 }
@@ -411,6 +422,17 @@ int build_lists(orion_case_t c, const std::vector<long long>& prim_off, const Ex
       plane_major_neighbours(h, koffs[b], nat, nbv);
       void* dnb = b64 ? (void*)b64->sk_nb : (void*)b32->sk_nb;
       CUDA_TRY(cudaMemcpyAsync(dnb, nbv.data(), nbv.size() * 4, cudaMemcpyHostToDevice, c->stream));
+      // natural order -> tile slots
+      const TilePlan p = make_tile_plan(h.idim, h.jdim, h.kdim, b64 ? 8 : 4);
+      std::vector<int4> tjk;
+      for (int a = 0; a < p.nJ(); ++a)
+        for (int x = 0; x < p.jw(a); ++x) tjk.push_back(make_int4(a, x, p.jw(a), 0));
+      for (int a = 0; a < p.nK(); ++a)
+        for (int x = 0; x < p.kh(a); ++x) tjk.push_back(make_int4(a, x, p.kh(a), 0));
+      const void* dt = b64 ? (const void*)b64->t_j : (const void*)b32->t_j;
+      const void* db = b64 ? (const void*)b64->t_base : (const void*)b32->t_base;
+      CUDA_TRY(cudaMemcpyAsync((void*)dt, tjk.data(), tjk.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
+      CUDA_TRY(cudaMemcpyAsync((void*)db, p.base.data(), p.base.size() * 8, cudaMemcpyHostToDevice, c->stream));
     }
     // kSweepThreads points per sweep chunk, one per thread
     const int nt = kSweepThreads;
@@ -636,6 +658,14 @@ int field_info(orion_case_t c, int block, int field, void** dptr, int* ncomp, bo
 // ============================================================================
 // C ABI
 // ============================================================================
+// Makes the sweeps' shared memory hold the arrays of the form about to run.
+// Every change of form does this at once; what is left for the launches is a
+// member of a group that runs another form than its own, and a wait that gave up.
+static int use_sweep_arrays(orion_case_t c, bool tiles) {
+  if (c->sweep_arrays == (tiles ? 1 : 0)) return 0;
+  return ops_for(c->prec).sweep_arrays(c, tiles);
+}
+
 static int capture_step(orion_case_t c, cudaGraph_t* g) {
   CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   int rc = ops_for(c->prec).step(c, c->prec == ORION_PREC_FP64);
@@ -830,6 +860,7 @@ static int create_case(int nglobal, const orion_block_desc_t* blocks, const int*
   if ((rc = build_lists(c.get(), prim_off, plan))) return rc;
   rc = ops_for(precision).set_attributes();
   if (!rc) rc = ops_for(precision).persistent_grid(c.get());
+  if (!rc) rc = use_sweep_arrays(c.get(), c->L.tiles_on);
   if (rc) return rc;
   // creation-time copies and memsets are ordered on the case's stream
   CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -972,6 +1003,7 @@ static int apply_schedule(orion_case_t c, const orion_schedule_t& s) {
     if ((rc = build_line_tiles(c))) return rc;
   }
   rc = ops_for(c->prec).schedule(c, s.sweep_form, s.cluster_size);
+  if (!rc && !c->group) rc = use_sweep_arrays(c, c->L.tiles_on);
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   return rc;
 }
@@ -1126,7 +1158,7 @@ int orion_case_sweep_schedule(orion_case_t c, int out[5]) {
   out[0] = L.tiles_on ? 3 : (L.cl_size > 0 ? 2 : (L.persist_grid > 0 ? 1 : 0));
   out[1] = L.tiles_on ? L.n_sweep_tiles[0] : (L.cl_size > 0 ? L.cl_count : L.persist_grid);
   out[2] = L.cl_size;
-  out[3] = L.tiles_on ? 32 * L.tile_k : L.sweep_nt;
+  out[3] = L.tiles_on ? kTileThreads : L.sweep_nt;
   out[4] = L.max_planes;
   return 0;
 }
@@ -1284,7 +1316,10 @@ int orion_compute_inviscid_rhs(orion_case_t c) {
   return dispatch(c, [&](const StageOps& o) { return o.inviscid(c); });
 }
 int orion_update_solution(orion_case_t c) {
-  return dispatch(c, [&](const StageOps& o) { return o.update(c, false); });
+  return dispatch(c, [&](const StageOps& o) {
+    const int rc = use_sweep_arrays(c, c->L.tiles_on);
+    return rc ? rc : o.update(c, false);
+  });
 }
 
 static int read_hist(orion_case_t c, long long first, int n, orion_residual_t* out) {
@@ -1329,6 +1364,7 @@ static int launch_steps(orion_case_t c, int nsteps) {
   if (c->shard.nranks > 1)
     return fail(ORION_E_INVALID, "a shard steps through the per-stage entry points and the shard exchanges");
   int rc = ensure_graph(c);
+  if (!rc && !c->L.group) rc = use_sweep_arrays(c, c->L.tiles_on);  // a group's: its members' (orion_group_submit)
   if (rc) return rc;
   for (int s = 0; s < nsteps; ++s) CUDA_TRY(cudaGraphLaunch(c->graph, c->stream));
   c->steps_done += nsteps;
@@ -1349,11 +1385,19 @@ static int sweep_status(orion_case_t c) {
   int ctl[2] = {0, 0};
   CUDA_TRY(cudaMemcpy(ctl, c->L.sweep_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
   if (ctl[1]) {
+    c->sweep_arrays = -1;  // edge records may hold increments nobody read
     CUDA_TRY(cudaMemsetAsync(c->L.sweep_ctl, 0, sizeof(ctl), c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     return fail(ORION_E_TIMEOUT, "a bounded wait of the implicit sweeps (grid barrier or tile progress) gave up waiting");
   }
   return 0;
+}
+
+static int group_status(orion_group_t g) {
+  const int rc = sweep_status(g->proxy);
+  if (rc == ORION_E_TIMEOUT)
+    for (auto c : g->members) c->sweep_arrays = -1;
+  return rc;
 }
 
 int orion_step(orion_case_t c, int nsteps, orion_residual_t* hist) {
@@ -1436,7 +1480,7 @@ int orion_case_poll(orion_case_t c, orion_residual_t* out, int cap, int* n) {
     cudaGetLastError();
     return fail(ORION_E_CUDA, std::string("case stream: ") + cudaGetErrorString(q));
   }
-  int rc = sweep_status(c->group ? c->group->proxy : c);
+  int rc = c->group ? group_status(c->group) : sweep_status(c);
   if (rc) return rc;
   const int take = std::min(cap, c->pending_n);
   for (int s = 0; s < take; ++s) {
@@ -1834,15 +1878,13 @@ int build_group(orion_group_t g, orion_case_t px) {
       std::vector<SweepTile> st;
       if ((rc = download(c, st, static_cast<const SweepTile*>(M.sweep_tiles[dir]), (size_t)M.n_sweep_tiles[dir])))
         return rc;
-      const int sb = (int)stiles[dir].size();
       for (auto x : st) {
         x.block += bo;
-        if (x.up_j >= 0) x.up_j += sb;
-        if (x.up_k >= 0) x.up_k += sb;
         stiles[dir].push_back(x);
       }
     }
     max_planes = std::max(max_planes, M.max_planes);
+    L.tile_lines = std::max(L.tile_lines, M.tile_lines);
   }
   // upload
   if ((rc = dev_upload(px, &L.pad_chunks, pad))) return rc;
@@ -1886,18 +1928,17 @@ int build_group(orion_group_t g, orion_case_t px) {
     if ((rc = dev_upload(px, &L.sweep_chunks[dir], ch))) return rc;
     L.sweep_off[dir] = off;
     SweepTile* d = nullptr;
+    std::stable_sort(stiles[dir].begin(), stiles[dir].end(),
+                     [](const SweepTile& x, const SweepTile& y) { return x.start < y.start; });
     if ((rc = dev_upload(px, &d, stiles[dir]))) return rc;
     L.sweep_tiles[dir] = d;
     L.n_sweep_tiles[dir] = (int)stiles[dir].size();
   }
   L.sweep_nt = kSweepThreads;
   {
-    const int mx = std::max(L.n_sweep_tiles[0], L.n_sweep_tiles[1]);
-    unsigned char* ctl = nullptr;
-    if ((rc = dev_alloc(px, &ctl, offsetof(TileCtl, progress) + sizeof(unsigned int) * (size_t)std::max(mx, 1))))
-      return rc;
+    TileCtl* ctl = nullptr;
+    if ((rc = dev_alloc(px, &ctl, 1))) return rc;
     L.tile_ctl = ctl;
-    L.tile_k = mem[0]->L.tile_k;
     int* sctl = nullptr;
     if ((rc = dev_alloc(px, &sctl, 4))) return rc;
     L.sweep_ctl = sctl;
@@ -1993,8 +2034,10 @@ int orion_group_submit(orion_group_t g, int nsteps) {
     }
   }
   if (nsteps == 0) return 0;
-  int rc = launch_steps(g->proxy, nsteps);
-  if (rc) return rc;
+  int rc = 0;
+  for (auto c : g->members)
+    if ((rc = use_sweep_arrays(c, g->proxy->L.tiles_on))) return rc;
+  if ((rc = launch_steps(g->proxy, nsteps))) return rc;
   for (auto c : g->members) {
     c->steps_done += nsteps;
     if ((rc = enqueue_hist_copy(c, nsteps))) return rc;
@@ -2005,7 +2048,7 @@ int orion_group_submit(orion_group_t g, int nsteps) {
 int orion_group_sync(orion_group_t g) {
   if (!g) return fail(ORION_E_INVALID, "null group");
   CUDA_TRY(cudaStreamSynchronize(g->proxy->stream));
-  return sweep_status(g->proxy);
+  return group_status(g);
 }
 
 int orion_group_step_launches(orion_group_t g, int* n) {

@@ -26,13 +26,10 @@ struct Stages {
     return rc;
   }
 
-  // dynamic shared memory the tile sweeps may ask for (prefetch buffers and
-  // the row-base cache of blocks of up to about 2,500 hyperplanes)
-  static constexpr size_t kTileSmemMax = 160 * 1024;
-
   static int set_line_attributes() {
     const int b = (int)kLineSmemBudget;
-    const int tb = (int)kTileSmemMax;
+    // the ring of a tile of kTileLines lines and its halo at most
+    const int tb = (int)tile_smem_bytes<T>(kTileMaxLines);
     CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_LUSGS_FWD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb));
     CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_LUSGS_BWD, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb));
     CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_GS, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb));
@@ -286,10 +283,10 @@ struct Stages {
     c->L.persist_grid = 0;
     c->L.cl_size = 0;
     c->L.tiles_on = false;
-    // default: one programmatic-dependent launch per hyperplane (the fastest
-    // form the autotuner measured on the configurations, both precisions)
+    // default: the tile wavefront (the fastest form the autotuner measured on
+    // the configurations, both precisions)
     const char* env = getenv("ORION_SWEEP");
-    const std::string mode = env ? std::string(env) : std::string("planes");
+    const std::string mode = env ? std::string(env) : std::string("tiles");
     const char* lim = getenv("ORION_SWEEP_SPIN_LIMIT");  // bound of the sweeps' device waits
     if (lim) c->L.spin_limit = atoll(lim);
     if (mode == "tiles") {
@@ -348,31 +345,27 @@ struct Stages {
     return 0;
   }
 
-  // One pass of the tile wavefront: reset the tickets and progress words, then
-  // one CTA per tile.
+  // One pass of the tile wavefront, one CTA per tile.
   template <int MODE, int DIR>
   static int tile_pass(orion_case_t c) {
     auto& L = c->L;
     const int d = DIR > 0 ? 0 : 1;
     const int n = L.n_sweep_tiles[d];
     if (n <= 0) return 0;
-    CUDA_TRY(cudaMemsetAsync(L.tile_ctl, 0, offsetof(TileCtl, progress) + sizeof(unsigned int) * (size_t)n,
-                             c->stream));
     SweepCtl* sc = static_cast<SweepCtl*>(L.sweep_ctl);
-    const size_t smem = tile_smem_bytes<T, MODE>(L.max_planes);
-    if (smem > kTileSmemMax) return fail(ORION_E_UNSUPPORTED, "block too long for the tile sweeps' row-base cache");
-    k_sweep_tiles<S, T, MODE, DIR><<<n, 32 * TileShape<T>::TK + 32, smem, c->stream>>>(
-        blocks(c), static_cast<const SweepTile*>(L.sweep_tiles[d]), n, static_cast<TileCtl*>(L.tile_ctl),
-        &sc->error, L.spin_limit);
+    const size_t smem = tile_smem_bytes<T>(L.tile_lines);
+    k_sweep_tiles<S, T, MODE, DIR><<<n, kTileThreads + 64, smem, c->stream>>>(
+        blocks(c), static_cast<const SweepTile*>(L.sweep_tiles[d]), n, L.tile_lines,
+        static_cast<TileCtl*>(L.tile_ctl), &sc->error, L.spin_limit);
     return 0;
   }
 
   static int update(orion_case_t c, bool fuse_residual) {
     auto& L = c->L;
     if (L.tiles_on) {
-      k_lusgs_prep<S, T, false><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks);
+      k_tile_prep<S, T><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks);
     } else {
-      k_lusgs_prep<S, T, true><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks);
+      k_lusgs_prep<S, T><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks);
       k_sweep_pairs<S, T><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks);
     }
     if (L.tiles_on) {
@@ -394,19 +387,40 @@ struct Stages {
       if (!rc) rc = sweep<SW_GS>(c, 1);
       if (rc) return rc;
     }
-    if (fuse_residual) {
-      k_sweep_finish<S, true, kThreads><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks,
-                                                                                     L.partials);
-      residual_final(c);
-    } else {
-      k_sweep_finish<S, false, kThreads><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks,
-                                                                                      L.partials);
+    auto finish = fuse_residual ? (L.tiles_on ? k_sweep_finish<S, true, true, kThreads> : k_sweep_finish<S, true, false, kThreads>)
+                                : (L.tiles_on ? k_sweep_finish<S, false, true, kThreads> : k_sweep_finish<S, false, false, kThreads>);
+    finish<<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks, L.partials);
+    if (fuse_residual) residual_final(c);
+    return 0;
+  }
+
+  // Gives the sweeps' shared arrays to the tile form or to the plane-major
+  // ones: the new owner's static operands are rebuilt from the metrics (every
+  // other field is written by each step); the tile form's slots without a
+  // point start as zeros, its edge records empty.
+  static int sweep_arrays(orion_case_t c, bool tiles) {
+    c->sweep_arrays = tiles ? 1 : 0;
+    for (int b = 0; b < c->nblocks; ++b) {
+      if (tiles) {
+        char *area, *edge;
+        long long nrec;
+        if constexpr (sizeof(S) == 8) area = c->bd64[b].tl_own, edge = c->bd64[b].tl_edge, nrec = c->bd64[b].nrec;
+        else area = c->bd32[b].tl_own, edge = c->bd32[b].tl_edge, nrec = c->bd32[b].nrec;
+        CUDA_TRY(cudaMemsetAsync(area, 0, (size_t)(edge - area), c->stream));
+        CUDA_TRY(cudaMemsetAsync(edge, 0xff, tile_bytes(sizeof(S)).rec * (size_t)nrec, c->stream));
+      }
+      sweep_static(c, b);
     }
     return 0;
   }
 
+  static void sweep_static(orion_case_t c, int b) {
+    if (c->sweep_arrays == 1) k_tile_static<S><<<148 * 4, kThreads, 0, c->stream>>>(blocks(c), b);
+    else if (c->sweep_arrays == 0) k_skew_static<S><<<148 * 4, kThreads, 0, c->stream>>>(blocks(c), b);
+  }
+
   static int skew_static(orion_case_t c, int b) {
-    k_skew_static<S><<<148 * 4, kThreads, 0, c->stream>>>(blocks(c), b);
+    sweep_static(c, b);
     if constexpr (sizeof(S) == 4)
       k_metric_shadow<<<148 * 4, kThreads, 0, c->stream>>>(reinterpret_cast<const BlockDev<float>*>(blocks(c)), b);
     return 0;
@@ -475,6 +489,7 @@ StageOps make_ops() {
   o.step = &X::step;
   o.init_flow = &X::init_flow;
   o.skew_static = &X::skew_static;
+  o.sweep_arrays = &X::sweep_arrays;
   o.persistent_grid = &X::persistent_grid;
   o.schedule = &X::schedule;
   o.prim_shadow = &X::prim_shadow;

@@ -1,496 +1,762 @@
 // Tile wavefront form of the LU-SGS / symmetric Gauss-Seidel sweeps
 // (StateUpdater::lusgs_sweep and gs_pr_sweep, src/solver/StateUpdater.cpp:297-445).
 //
-// The increment-independent coefficients of every neighbour term (the
-// neighbour's spectral radius through this point's metric, the split
-// eigenvalues, the viscous radius) are formed in place from the neighbour's
-// prepared state (u, v, w, H, c^2, af, c, viscous factor) and this point's
-// static metric magnitudes, so a pass reads per point only its own operands,
-// its neighbours' prepared state and increments, and writes its increment.
+// One launch per pass.  A CTA owns a tile of jw x kh grid lines along i of one
+// block, one thread per line, and walks it wave by wave: on wave
+// w = i + tj + tk the thread of line (tj, tk) updates its point i (forward
+// passes take the waves upwards, backward passes downwards).  A wave lies on
+// one i+j+k hyperplane, so the order is the reference's lexicographic one
+// exactly: a point reads its "behind" neighbours (lower i, j, k forward, upper
+// backward) after they were updated in this pass and its "ahead" neighbours
+// before.
 //
-// One launch per pass.  A CTA owns a tile of 32 x TK grid lines along i of one
-// block (32 consecutive j, TK consecutive k) and walks it: at local step t the
-// thread of line (tj, tk) updates the point i = t - tj - tk (mirrored on the
-// backward passes).  All points a CTA touches at one step lie on one i+j+k
-// hyperplane, and within a k row they are consecutive in the plane-major
-// layout, so every warp reads and writes 32 consecutive elements.
+// What bounds it.  Small cases: the length of the chain, (ni + nj + nk) waves
+// per pass, so a wave has to be short: everything a wave reads is in shared
+// memory before it starts, and one CTA barrier ends it.  Large cases: DRAM and,
+// in FP64, the FP64 pipe, so each operand is read once per pass.  The arrays
+// are laid out in the order the tile walks them (tile, wave, 16-byte piece,
+// line), so a wave of a tile is one contiguous run and comes in by one bulk
+// copy per array (a copy costs its issuing warp about 100 cycles whatever its
+// size; one per piece made the copies the longest part of an FP32 step); the
+// compute threads issue no loads from global memory.  A slot no point has (the ramps at both ends, and
+// one wave beyond each) holds zeros, and so has the ring for a line outside the
+// block, so the six neighbour terms are formed without a branch.
 //
-// Dependencies are the reference's lexicographic order exactly: a point reads
-// its "behind" neighbours (lower i, j, k on forward passes, upper on backward
-// ones) after they were updated in this pass, and its "ahead" neighbours
-// before.  Inside a tile the behind-j and behind-k neighbours were updated one
-// step earlier by the adjacent threads (shared memory, one barrier per step),
-// the behind-i neighbour by the same thread (registers).  Across tiles a CTA
-// waits on the progress counter of its upstream neighbour tile in j and in k,
-// which runs 32 (resp. TK) steps ahead; the ahead neighbours are only updated
-// by the downstream tiles after this tile has published that it read them.
+// Across tiles a CTA needs the fresh increments of its behind-j and behind-k
+// neighbour tiles.  The producing thread stores each into an edge record as
+// soon as it has it; a warp of the consuming CTA polls the record itself,
+// word by word against a value no increment can have (kEdgeEmpty), and puts
+// the record back to empty after reading.  So a hop between tiles costs one
+// L2 store and one L2 load: no fence, no progress counter, and no reset
+// between passes.  The ahead neighbours' old increments are plain loads: the
+// tile that owns one only overwrites it after it has received this tile's
+// fresh value of the same i, which is stored after the old one was read.
 //
-// Tiles are claimed through a ticket counter in a dependency-respecting order,
-// so a CTA only ever waits on tiles held by CTAs that are already running:
-// the launch needs no co-residency guarantee.  Every wait is bounded: after
-// spin_limit polls it raises the shared error word and the CTA returns; every
-// other waiting CTA sees the word and returns too (the host reports
-// ORION_E_TIMEOUT).
+// Tiles are claimed through a ticket counter in an order in which a tile's
+// behind tiles come first, so a CTA only ever waits on CTAs that are already
+// running; the launch needs no co-residency.  Every wait is bounded: after
+// spin_limit polls the error word is raised, every wait of the launch gives
+// up, the passes finish on whatever data is there (in bounds), and the host
+// reports ORION_E_TIMEOUT and empties the edge records.
 #pragma once
 
 #include <cstddef>
 
 #include "kernels.cuh"
+#include "tile_plan.hpp"
 
 namespace orion {
 
-// One tile of one pass.  (jb, kb) is the tile's first line in sweep order:
-// the lowest (j, k) on forward passes, the highest on backward passes.
+constexpr int kTileThreads = (kTileMaxLines + 31) / 32 * 32;  // compute threads, one a line
+
+// 16-byte pieces per point of the tile layout (tl_own: met, dyn; tl_nb: nb), FP32 / FP64:
+//   met  {kx ky kz |k|} per direction                     / {kx ky}{kz |k|} per direction, {1/|k| x 2}{1/|k| -}
+//   dyn  {coed r0 r1 r2}{r3 r4 - -}                       / {coed r0}{r1 r2}{r3 r4}
+//   nb   {u v w H}{c visc af dq4}{dq0..3}                 / {u v}{w H}{c^2 af}{c visc}{1/2c^2 1/2c}{dq0 dq1}{dq2 dq3}{dq4 -}
+//
+// `ring` waves of nb are kept in shared memory: at step t waves t-1 (behind) to
+// t+1 (ahead) are in use and waves up to t + ring - 2 on their way; own
+// operands (met, dyn) of waves t to t + ring - 2.  FP32: six waves and two CTAs
+// an SM (193x97x65, 8 blocks: 1.93 ms a step, five waves 1.98; eight waves and
+// one CTA an SM the same, and 4% slower on 385x257x129).  FP64: one CTA an SM,
+// so that the six terms of a point overlap in registers (183 to 196; at two CTAs
+// and 168 registers a pass of 97x49x33 took 0.73 ms in place of 0.40).
+#ifndef ORION_TILE_RING_F32
+#define ORION_TILE_RING_F32 6
+#endif
+#ifndef ORION_TILE_RING_F64
+#define ORION_TILE_RING_F64 5
+#endif
+template <typename T> struct TileLayout;
+template <> struct TileLayout<float> {
+  static constexpr int met = 3, dyn = 2, nb = 3, own = met + dyn, rec = 8, minb = 2, ring = ORION_TILE_RING_F32;
+};
+template <> struct TileLayout<double> {
+  static constexpr int met = 8, dyn = 3, nb = 8, own = met + dyn, rec = 8, minb = 1, ring = ORION_TILE_RING_F64;
+};
+
+// One tile, in ticket order of one direction.
 struct SweepTile {
   int block;
-  int jb, kb;
-  int up_j, up_k;  // ticket slots of the upstream tiles in j and k (-1: none)
-  int pad[3];
+  int start;             // waves its first point is behind the block's first (list order)
+  int jw, kh;
+  int w[2];              // widths jw of the tiles at j-1 and j+1, 0: none
+  int h[2];              // heights kh of the tiles at k-1 and k+1, 0: none
+  int jb, kb;            // first line
+  long long base;        // slot of wave 0, line 0 in the block's tile arrays
+  long long base_j[2];   // of the tiles at j-1, j+1
+  long long base_k[2];
+  long long edge_j[2];   // first edge record shared with the tile at j-1, j+1 (kh per i)
+  long long edge_k[2];   // at k-1, k+1 (jw per i)
 };
 
-// Per-launch control: ticket counter then one progress word per tile slot
-// (steps completed), zeroed before every pass.
+// Ticket and exit counters of one launch; the last CTA to leave clears both.
 struct TileCtl {
-  unsigned int ticket;
-  unsigned int pad;
-  unsigned int progress[1];
+  unsigned int ticket, done;
 };
 
-// Polls are plain volatile loads: an acquire load at GPU scope would discard
-// the SM's L1 contents at every poll.  Nothing a tile reads through L1 is
-// written during the pass; the increments other tiles write are read with
-// ld.global.cg (L2, the point of coherence), and the producer publishes its
-// progress only after a fence that makes them visible there.
-__device__ __forceinline__ unsigned int ld_poll_u32(const unsigned int* p) { return *(const volatile unsigned int*)p; }
-
-__device__ __forceinline__ void publish_u32(unsigned int* p, unsigned int v) {
-  __threadfence();
-  *(volatile unsigned int*)p = v;
-}
-
-// Waits (bounded) until *p >= need; `known` caches the last value seen.
-// Returns false when this wait or another CTA's gave up.
-__device__ __forceinline__ bool tile_wait(const unsigned int* p, unsigned int need, unsigned int& known, int* err,
-                                          long long spin_limit) {
-  if (known >= need) return true;
-  long long it = 0;
-  while (true) {
-    const unsigned int v = ld_poll_u32(p);
-    if (v >= need) {
-      known = v;
-      return true;
-    }
-    if (*(volatile int*)err) return false;
-    if (++it > spin_limit) {
-      atomicExch(err, 1);
-      return false;
-    }
-    __nanosleep(32);
-  }
-}
-
-// Compact index of (s, kk, jj) is row_base(s, kk) + jj.
-__device__ __forceinline__ long long row_base(const int* __restrict__ koff, int ni, int nk, int s, int kk) {
-  const int v = s - kk - (ni - 1);
-  return (long long)__ldg(koff + (long long)s * nk + kk) - (v > 0 ? v : 0);
-}
-
-// Bound of a compute warp's wait for the control warp (about four seconds).
-constexpr long long kComputeWaitCycles = 8000000000LL;
-
-__device__ __forceinline__ void compute_barrier(int nthreads) {
-  asm volatile("bar.sync 1, %0;\n" ::"r"(nthreads) : "memory");
-}
-
-// Prefetch distance (steps) and tile height of each precision: FP32 tiles are
-// 32 x 4 lines and read their operands three steps ahead, FP64 tiles 32 x 2
-// lines two steps ahead (the prefetch buffers live in shared memory).
-#ifndef ORION_TILE_K_F32
-#define ORION_TILE_K_F32 4
-#endif
-#ifndef ORION_TILE_PD_F32
-#define ORION_TILE_PD_F32 3
-#endif
-#ifndef ORION_TILE_K_F64
-#define ORION_TILE_K_F64 2
-#endif
-#ifndef ORION_TILE_PD_F64
-#define ORION_TILE_PD_F64 2
-#endif
-template <typename T> struct TileShape;
-template <> struct TileShape<float> { static constexpr int TK = ORION_TILE_K_F32, PD = ORION_TILE_PD_F32; };
-template <> struct TileShape<double> { static constexpr int TK = ORION_TILE_K_F64, PD = ORION_TILE_PD_F64; };
-
-// Fields a point's owner prefetches: static operands (coed, own: rhs or the
-// forward increment, metrics 9, |grad| 3, 1/|grad| 3) for itself, and the
-// neighbour-visible state (u, v, w, H, c^2, af, c, viscous factor, and on the
-// GS passes the old increment) for the adjacent threads.
-constexpr int kTileStatics = 21;
-template <int MODE> __host__ __device__ constexpr int tile_ring_fields() { return MODE == SW_GS ? 13 : 8; }
-
-// Dynamic shared memory of one tile CTA with `npl` hyperplanes at most.
-// Edge records: the state (8) and increment (5) of a neighbour in another
-// tile, per step slot, for the first and last lane of every k row (j edges)
-// and every lane of the first and last k row (k edges).
-constexpr int kTileEdgeFields = 13;
-template <int TK> __host__ __device__ constexpr int tile_edge_records() { return 2 * TK + 64; }
-
-template <typename T, int MODE>
-constexpr size_t tile_smem_bytes(int npl) {
-  constexpr int TK = TileShape<T>::TK, PD = TileShape<T>::PD;
-  return (size_t)((PD + 1) * kTileStatics + (PD + 2) * tile_ring_fields<MODE>()) * TK * 32 * sizeof(T) +
-         (size_t)(PD + 1) * tile_edge_records<TK>() * kTileEdgeFields * sizeof(T) +
-         (size_t)(TK + 2) * npl * sizeof(int);
-}
-
+// Dynamic shared memory of tiles of `lines` lines at most: the ring (per wave
+// [piece][line], then [piece][32 behind and 32 ahead halo lines]), the fresh
+// increments of two waves ([piece][line, halo line]) and the own operands
+// ([piece][line]).
 template <typename T>
-__device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
+constexpr size_t tile_smem_bytes(int lines) {
+  using L = TileLayout<T>;
+  return (size_t)(L::ring * L::nb + 2 * ((5 * sizeof(T) + 15) / 16)) * 16 * (size_t)(lines + 64) +
+         (size_t)(L::ring - 1) * L::own * 16 * (size_t)lines;
+}
+
+// ---------------------------------------------------------------------------
+// edge records: five increments and the empty value (all bits set).  No
+// arithmetic result has that pattern except a NaN with its sign flipped, which
+// the producer stores as another NaN.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void edge_store(float* r, const float v[5]) {
+  unsigned b[5];
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    b[m] = __float_as_uint(v[m]);
+    if (b[m] == 0xffffffffu) b[m] = 0x7fffffffu;
+  }
+  asm volatile("st.relaxed.gpu.global.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"l"(r), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3])
+               : "memory");
+  asm volatile("st.relaxed.gpu.global.b32 [%0], %1;\n" ::"l"(r + 4), "r"(b[4]) : "memory");
+}
+__device__ __forceinline__ void edge_store(double* r, const double v[5]) {
+  unsigned long long b[5];
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    b[m] = (unsigned long long)__double_as_longlong(v[m]);
+    if (b[m] == ~0ull) b[m] = 0x7fffffffffffffffull;
+  }
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1,%2};\n" ::"l"(r), "l"(b[0]), "l"(b[1]) : "memory");
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1,%2};\n" ::"l"(r + 2), "l"(b[2]), "l"(b[3]) : "memory");
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;\n" ::"l"(r + 4), "l"(b[4]) : "memory");
+}
+__device__ __forceinline__ void edge_load(const float* r, unsigned b[5]) {
+  asm volatile("ld.relaxed.gpu.global.v4.b32 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
+               : "l"(r)
+               : "memory");
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];\n" : "=r"(b[4]) : "l"(r + 4) : "memory");
+}
+__device__ __forceinline__ void edge_load(const double* r, unsigned long long b[5]) {
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0,%1}, [%2];\n" : "=l"(b[0]), "=l"(b[1]) : "l"(r) : "memory");
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0,%1}, [%2];\n" : "=l"(b[2]), "=l"(b[3]) : "l"(r + 2) : "memory");
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];\n" : "=l"(b[4]) : "l"(r + 4) : "memory");
+}
+__device__ __forceinline__ void edge_clear(float* r) {
+  asm volatile("st.relaxed.gpu.global.v4.b32 [%0], {%1,%1,%1,%1};\n" ::"l"(r), "r"(0xffffffffu) : "memory");
+  asm volatile("st.relaxed.gpu.global.b32 [%0], %1;\n" ::"l"(r + 4), "r"(0xffffffffu) : "memory");
+}
+__device__ __forceinline__ void edge_clear(double* r) {
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1,%1};\n" ::"l"(r), "l"(~0ull) : "memory");
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1,%1};\n" ::"l"(r + 2), "l"(~0ull) : "memory");
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;\n" ::"l"(r + 4), "l"(~0ull) : "memory");
+}
+template <typename T> struct EdgeBits;
+template <> struct EdgeBits<float> { using type = unsigned; };
+template <> struct EdgeBits<double> { using type = unsigned long long; };
+template <typename U>
+__device__ __forceinline__ bool edge_full(const U b[5]) {
+  const U e = ~U(0);
+  return b[0] != e && b[1] != e && b[2] != e && b[3] != e && b[4] != e;
+}
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned int s = (unsigned int)__cvta_generic_to_shared(smem);
-  if (sizeof(T) == 4)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// MODE: SW_LUSGS_FWD (forward, behind = lower, uses q 0..2), SW_LUSGS_BWD
-// (backward, behind = upper, uses q 3..5), SW_GS with DIR +1 / -1 (all six).
-//
-// 32*TK compute threads and one control warp.  The compute warps separate
-// their steps with a named barrier of their own; before step t they wait (in
-// shared memory) until the control warp has seen the upstream tiles far
-// enough along.  The control warp publishes the compute warps' completed
-// steps (fence, then the progress word) and polls the upstream progress, so
-// neither the fence nor the polls are on the compute warps' path.  When a
-// wait gives up, the control warp raises the error word and releases every
-// remaining step: the compute warps finish the tile on whatever data is there
-// (every access stays in bounds) and the host reports ORION_E_TIMEOUT.
-//
-// Each compute thread copies its own points' operands PD steps ahead with
-// cp.async into shared memory: the static operands into a (PD+1)-slot buffer
-// of its own, the neighbour-visible state into a (PD+2)-slot ring the adjacent
-// threads read at step t from slot t-1 (behind neighbours) and t+1 (ahead).
-// New increments of the behind neighbours come from the previous step
-// (registers for i, s_dq for j and k).  Neighbours in other tiles are
-// prefetched with the same lead into per-step edge records; a step's operands
-// are fetched only once the upstream tiles allow that step, so the compute of
-// a step never waits on memory.  The row bases of the tile's k rows (and the
-// rows on either side) are cached in shared memory for every hyperplane.
-template <typename S, typename T, int MODE, int DIR>
-__global__ void __launch_bounds__(32 * TileShape<T>::TK + 32) k_sweep_tiles(const BlockDev<S>* __restrict__ blocks,
-                                                                           const SweepTile* __restrict__ tiles,
-                                                                           int ntiles, TileCtl* __restrict__ ctl,
-                                                                           int* __restrict__ err, long long spin_limit) {
-  static_assert(sizeof(S) == sizeof(T), "the tile sweeps keep operands in their storage precision");
-  constexpr int TJ = 32, TK = TileShape<T>::TK, PD = TileShape<T>::PD;
-  constexpr int NSS = PD + 1, NSR = PD + 2, NR = tile_ring_fields<MODE>(), NS = kTileStatics;
-  constexpr int Q0 = MODE == SW_LUSGS_BWD ? 3 : 0;
-  constexpr int Q1 = MODE == SW_LUSGS_FWD ? 3 : 6;
-  // behind neighbours (updated in this pass) are q = QB .. QB+2
-  constexpr int QB = DIR > 0 ? 0 : 3;
-  __shared__ int s_slot;
-  __shared__ int s_ready;  // steps whose upstream data is ready (control -> compute)
-  __shared__ int s_done;   // steps the compute warps have completed (compute -> control)
-  __shared__ T s_dq[2][5][TK][TJ];  // each thread's increment of the last two steps
-  const int tj = threadIdx.x & 31, tk = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {
-    s_slot = (int)atomicAdd(&ctl->ticket, 1u);
-    s_ready = 0;
-    s_done = 0;
-  }
-  __syncthreads();
-  const int slot = s_slot;
-  if (slot >= ntiles) return;
-  const SweepTile W = tiles[slot];
-  const BlockDev<S>& Bd = blocks[W.block];
-  const ParamsDev& P = Bd.prm;
-  const int ni = Bd.ni;
-  const int nsteps = ni + TJ + TK - 2;
-
-  if (tk == TK) {  // ---------------- control warp ----------------
-    if (tj != 0) return;
-    const int up_j = W.up_j, up_k = W.up_k;
-    unsigned int* const mine = &ctl->progress[slot];
-    // steps allowed by an upstream tile that has completed p steps and runs `lag` ahead
-    auto allowed = [&](int up, int lag) -> int {
-      if (up < 0) return nsteps;
-      const int p = (int)ld_poll_u32(&ctl->progress[up]);
-      return p >= nsteps ? nsteps : max(0, p - lag + 1);
-    };
-    int ready = 0, published = 0;
-    long long idle = 0;
-    while (published < nsteps) {
-      bool moved = false;
-      if (ready < nsteps) {
-        const int r = min(allowed(up_j, TJ), allowed(up_k, TK));
-        if (r > ready) {
-          ready = r;
-          *(volatile int*)&s_ready = ready;
-          moved = true;
-        }
-      }
-      const int d = *(volatile int*)&s_done;
-      if (d > published) {
-        publish_u32(mine, (unsigned int)d);
-        published = d;
-        moved = true;
-      }
-      if (moved) {
-        idle = 0;
-        continue;
-      }
-      if (*(volatile int*)err || ++idle > spin_limit) {  // give up: release the compute warps, stop publishing
-        if (!*(volatile int*)err) atomicExch(err, 1);
-        *(volatile int*)&s_ready = nsteps;
-        return;
-      }
-      __nanosleep(32);
+// mbarrier of one ring wave: one arrival (the copying warp's, with the wave's
+// byte count), completed by the bulk copies.
+__device__ __forceinline__ void mbar_init(unsigned long long* m) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"((unsigned)__cvta_generic_to_shared(m)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned long long* m, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"((unsigned)__cvta_generic_to_shared(m)),
+               "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ bool mbar_try(unsigned m, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(m), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// A copy of this CTA's own always arrives; the bound is there all the same.
+__device__ __forceinline__ void mbar_wait(unsigned m, unsigned parity, int* err) {
+  for (int it = 0; !mbar_try(m, parity); ++it)
+    if (it > (1 << 24)) {
+      atomicExch(err, 1);
+      return;
     }
-    return;
-  }
+}
+__device__ __forceinline__ void bulk_copy(void* smem, const void* gmem, unsigned bytes, unsigned long long* m) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(smem)),
+               "l"(gmem), "r"(bytes), "r"((unsigned)__cvta_generic_to_shared(m))
+               : "memory");
+}
 
-  // ---------------- compute warps ----------------
-  extern __shared__ __align__(16) unsigned char tile_smem[];
-  T(*s_stat)[NS][TK][TJ] = reinterpret_cast<T(*)[NS][TK][TJ]>(tile_smem);
-  T(*s_ring)[NR][TK][TJ] = reinterpret_cast<T(*)[NR][TK][TJ]>(tile_smem + sizeof(T) * NSS * NS * TK * TJ);
-  constexpr int NE = tile_edge_records<TK>(), NEF = kTileEdgeFields;
-  T(*s_edge)[NE][NEF] = reinterpret_cast<T(*)[NE][NEF]>(tile_smem + sizeof(T) * (NSS * NS + NSR * NR) * TK * TJ);
-  int* s_rowb = reinterpret_cast<int*>(tile_smem + sizeof(T) * ((NSS * NS + NSR * NR) * TK * TJ + NSS * NE * NEF));
-  const long long nc = Bd.ncomp;
-  const int nj = Bd.nj, nk = Bd.nk, npl = Bd.nplanes;
-  S* const skdq = Bd.sk_dq;
-  const S* const skcoed = Bd.sk_coed;
-  const S* const skrhs = Bd.sk_rhs;
-  const S* const sknbq = Bd.sk_nbq;
-  const S* const skmet = Bd.sk_metrics;
-  const S* const skgm = Bd.sk_gm;
-  const S* const skinv = Bd.sk_inv;
-  const int jj = W.jb + DIR * tj, kk = W.kb + DIR * tk;
-  const bool row = jj >= 0 && jj < nj && kk >= 0 && kk < nk;
-  const T gm1 = T(P.gamma) - T(1);
-  const int nvis = P.nvis;
-  // row bases of k rows kb - DIR .. kb + DIR*TK: compact index of (s, kk_r, jj) = s_rowb[r * npl + s] + jj
-  {
-    const int* const koff = Bd.koff;
-    for (int e = threadIdx.x; e < (TK + 2) * npl; e += 32 * TK) {
-      const int r = e / npl, sp = e - r * npl;
-      const int kr = W.kb + DIR * (r - 1);
-      s_rowb[e] = (kr >= 0 && kr < nk) ? (int)row_base(koff, ni, nk, sp, kr) : 0;
-    }
-  }
-  // rows of this thread (r = tk + 1) and its k neighbours (r = tk, tk + 2)
-  const int* const rb_own = s_rowb + (tk + 1) * npl;
-  const int* const rb_lo = s_rowb + (DIR > 0 ? tk : tk + 2) * npl;  // row kk - 1
-  const int* const rb_hi = s_rowb + (DIR > 0 ? tk + 2 : tk) * npl;  // row kk + 1
-  auto valid = [&](int u) { return row && u >= 0 && u < ni; };
-  auto ii_of = [&](int u) { return DIR > 0 ? u : ni - 1 - u; };
-  compute_barrier(32 * TK);  // row bases ready
+// ---------------------------------------------------------------------------
+// one point's own operands and one neighbour's term, per precision; all
+// operands in shared memory
+// ---------------------------------------------------------------------------
+template <typename T, int MODE> struct TilePoint;
 
-  // edge increments in flight: loaded at prefetch time, stored to the edge
-  // record at the end of the step
-  T edq[4][5];
-  T* edq_dst[4] = {nullptr, nullptr, nullptr, nullptr};
-  // waits (bounded) until the upstream tiles allow step x
-  auto wait_ready = [&](int x) {
-    if (*(volatile int*)&s_ready <= x) {  // bounded: the control warp releases or gives up well before this
-      const long long t0 = clock64();
-      while (*(volatile int*)&s_ready <= x) {
-        if (clock64() - t0 > kComputeWaitCycles) {
-          atomicExch(err, 1);
-          break;
-        }
-      }
-    }
-  };
-  // copies the operands of this thread's point at sweep position u into the
-  // buffers of step slot `step` (the upstream tiles must allow that step)
-  auto prefetch = [&](int u, int step) {
-    if (!valid(u)) return;
-    const int ii = ii_of(u);
-    const long long c = (long long)rb_own[ii + jj + kk] + jj;
-    T(*st)[TK][TJ] = s_stat[step % NSS];
-    T(*rg)[TK][TJ] = s_ring[step % NSR];
-    cp_async_elem(&st[0][tk][tj], skcoed + c);
+// FP32 (mixed path).  With the neighbour's spectral radius taken through this
+// point's metric k, the split eigenvalues of compute_flux_splitting
+// (StateUpdater.cpp:217-265) give 2 l1 - l4 - l5 = 0 and l4 - l5 = 2 c |k|
+// identically, so x1 = 0, x2 = |k| / 2 and every 1/|k| cancels:
+//   2 fs0 = a d0 - D,  2 fsm = a dm + km dh - um D,  2 fs4 = a d4 + ct dh - H D
+// with ct = k.u, D = ct d0 - k.d, dh = af d0 - (gamma-1)(u.d - d4) and
+// a = ct +- (|ct| + c |k| + visc |k|^2) carrying the viscous radius too.  About
+// 30 operations a neighbour and no division, against 70 with the coefficients
+// formed one by one; the rounding noise of x1 is gone.
+template <int MODE>
+struct TilePoint<float, MODE> {
+  float4 m[3];
+  float4 y0;  // coed and rhs 0..2
+  float2 y1;  // rhs 3, 4
+  // own operands of a wave ([piece][nl]); in the backward LU-SGS pass the
+  // forward increment, from the wave's ring plane, takes the RHS's place
+  __device__ __forceinline__ void load(const uint4* own, int nl, int l, const uint4* plane) {
+    const float4* const p = reinterpret_cast<const float4*>(own) + l;
 #pragma unroll
-    for (int m = 0; m < 5; ++m)
-      cp_async_elem(&st[1 + m][tk][tj], (MODE == SW_LUSGS_BWD ? (const S*)skdq : skrhs) + m * nc + c);
-#pragma unroll
-    for (int m = 0; m < 9; ++m) cp_async_elem(&st[6 + m][tk][tj], skmet + m * nc + c);
+    for (int d = 0; d < 3; ++d) m[d] = p[d * nl];
+    if (MODE == SW_LUSGS_BWD) {
+      const float4* const q = reinterpret_cast<const float4*>(plane) + l;
+      y0 = q[2 * nl];
+      y1.x = reinterpret_cast<const float*>(q + nl)[3];
+      y1.y = reinterpret_cast<const float*>(p + 3 * nl)[0];
+    } else {
+      y0 = p[3 * nl];
+      y1 = *reinterpret_cast<const float2*>(p + 4 * nl);
+    }
+  }
+  // neighbour across direction d, lower or upper: its first ring piece (ps
+  // apart), and its fresh increment, or the ring's old one
+  template <bool FRESH>
+  __device__ __forceinline__ void term(int d, bool upper, const uint4* first, int ps, const uint4* fresh, int sl, int slot,
+                                       float g1, int, float acc[5]) const {
+    const float4* p = reinterpret_cast<const float4*>(first);
+    const float4 A = p[0];
+    float4 B = p[ps], D;
+    if (FRESH) {
+      D = reinterpret_cast<const float4*>(fresh)[slot];
+      B.w = reinterpret_cast<const float*>(fresh + sl)[slot];
+    } else {
+      D = p[2 * ps];
+    }
+    const float4 k = m[d];
+    const float ct = k.x * A.x + k.y * A.y + k.z * A.z;
+    const float rr = fabsf(ct) + B.x * k.w, vr = B.y * (k.w * k.w);
+    const float a = upper ? (MODE == SW_GS ? ct - (rr + vr) : ct - rr + vr) : ct + (rr + vr);
+    const float kd = k.x * D.y + k.y * D.z + k.z * D.w;
+    const float DC = ct * D.x - kd;
+    const float dh = B.z * D.x - g1 * (A.x * D.y + A.y * D.z + A.z * D.w - B.w);
+    const float s = (MODE == SW_GS && upper) ? -1.f : 1.f;
+    acc[0] += s * (a * D.x - DC);
+    acc[1] += s * (a * D.y + k.x * dh - A.x * DC);
+    acc[2] += s * (a * D.z + k.y * dh - A.y * DC);
+    acc[3] += s * (a * D.w + k.z * dh - A.z * DC);
+    acc[4] += s * (a * B.w + ct * dh - A.w * DC);
+  }
+  __device__ __forceinline__ void result(const float acc[5], float v[5]) const {
+    if (MODE == SW_LUSGS_BWD) {
+      const float h = 0.5f * y1.y;
+      v[0] = y0.x - acc[0] * h;
+      v[1] = y0.y - acc[1] * h;
+      v[2] = y0.z - acc[2] * h;
+      v[3] = y0.w - acc[3] * h;
+      v[4] = y1.x - acc[4] * h;
+    } else {
+      v[0] = (0.5f * acc[0] - y0.y) * y0.x;
+      v[1] = (0.5f * acc[1] - y0.z) * y0.x;
+      v[2] = (0.5f * acc[2] - y0.w) * y0.x;
+      v[3] = (0.5f * acc[3] - y1.x) * y0.x;
+      v[4] = (0.5f * acc[4] - y1.y) * y0.x;
+    }
+  }
+  static __device__ __forceinline__ void fresh_store(uint4* fresh, int sl, int slot, const float v[5]) {
+    reinterpret_cast<float4*>(fresh)[slot] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float*>(fresh + sl)[slot] = v[4];
+  }
+  // p: the point's first nb piece, pieces cs bytes apart
+  static __device__ __forceinline__ void store(char* p, int cs, const float v[5]) {
+    *reinterpret_cast<float4*>(p + 2 * cs) = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float*>(p + cs)[3] = v[4];
+  }
+};
+
+// a / b, correctly rounded, from r = RN(1/b): two Newton corrections of the
+// quotient with an exact remainder (Markstein, IBM J. Res. Dev. 34, 1990: with
+// r correctly rounded and q within one ulp, RN(q + r (a - b q)) = RN(a / b)).
+// The first correction brings q = RN(a r) within one ulp, the second is the
+// theorem's step.  Exact while a remainder stays normal: quotient_rcp gives 0,
+// and quotient 0, for a denominator beyond 1e+-290.
+__device__ __forceinline__ double quotient(double a, double b, double r) {
+  double q = a * r;
+  q = __fma_rn(__fma_rn(-b, q, a), r, q);
+  return __fma_rn(__fma_rn(-b, q, a), r, q);
+}
+__device__ __forceinline__ double quotient_rcp(double b) {
+  return (b > 1.0e-290 && b < 1.0e290) ? __drcp_rn(b) : 0.0;
+}
+
+// FP64 (plain path): the reference's operations in the reference's order; the
+// two divisions of the pair's coefficients share the reciprocals prepared once
+// per point.
+template <int MODE>
+struct TilePoint<double, MODE> {
+  double k[9], gm[3], inv[3], coed, y[5];
+  __device__ __forceinline__ void load(const uint4* own, int nl, int l, const uint4* plane) {
+    const double2* const p = reinterpret_cast<const double2*>(own) + l;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      cp_async_elem(&st[15 + d][tk][tj], skgm + d * nc + c);
-      cp_async_elem(&st[18 + d][tk][tj], skinv + d * nc + c);
+      const double2 a = p[2 * d * nl], b = p[(2 * d + 1) * nl];
+      k[3 * d] = a.x;
+      k[3 * d + 1] = a.y;
+      k[3 * d + 2] = b.x;
+      gm[d] = b.y;
     }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) cp_async_elem(&rg[k][tk][tj], sknbq + k * nc + c);
-    if (MODE == SW_GS) {
-#pragma unroll
-      for (int m = 0; m < 5; ++m) cp_async_elem(&rg[8 + m][tk][tj], (const S*)skdq + m * nc + c);
-    }
-    // neighbours in other tiles: state by cp.async, increment (written during
-    // this pass by the upstream tile, or not yet by the downstream one) from
-    // L2 into registers, stored at the end of the step
-    const int s = ii + jj + kk;
-    T(*ed)[NEF] = s_edge[step % NSS];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      // e: 0 behind-j, 1 ahead-j, 2 behind-k, 3 ahead-k
-      const bool isj = e < 2, behind = (e & 1) == 0;
-      if (isj ? (behind ? tj != 0 : tj != TJ - 1) : (behind ? tk != 0 : tk != TK - 1)) continue;
-      if (MODE == SW_LUSGS_FWD && !behind) continue;  // these passes read behind neighbours only
-      if (MODE == SW_LUSGS_BWD && !behind) continue;
-      const bool lower = behind == (DIR > 0);  // natural lower neighbour (j-1 or k-1)
-      const int nd = isj ? jj + (lower ? -1 : 1) : kk + (lower ? -1 : 1);
-      if (nd < 0 || nd >= (isj ? nj : nk)) continue;
-      const int sn = lower ? s - 1 : s + 1;
-      const long long n = isj ? (long long)rb_own[sn] + nd : (long long)(lower ? rb_lo : rb_hi)[sn] + jj;
-      const int rec = isj ? (behind ? 0 : 1) * TK + tk : 2 * TK + (behind ? 0 : 1) * 32 + tj;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) cp_async_elem(&ed[rec][k], sknbq + k * nc + n);
-      T* const slotp = &ed[rec][8];
-#pragma unroll
-      for (int m = 0; m < 5; ++m) edq[e][m] = (T)__ldcg(skdq + m * nc + n);
-      edq_dst[e] = slotp;
-    }
-  };
-  auto store_edges = [&]() {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (!edq_dst[e]) continue;
-#pragma unroll
-      for (int m = 0; m < 5; ++m) edq_dst[e][m] = edq[e][m];
-      edq_dst[e] = nullptr;
-    }
-  };
-  {
-    const int u0 = -tj - tk;
-    wait_ready(min(PD, nsteps) - 1);
-#pragma unroll
-    for (int p = 0; p < PD; ++p) {
-      prefetch(u0 + p, p);
-      cp_async_commit();
-      store_edges();
+    const double2 a = p[6 * nl];
+    inv[0] = a.x;
+    inv[1] = a.y;
+    inv[2] = reinterpret_cast<const double*>(p + 7 * nl)[0];
+    if (MODE == SW_LUSGS_BWD) {
+      coed = reinterpret_cast<const double*>(p + 8 * nl)[0];
+      const double2* const q = reinterpret_cast<const double2*>(plane) + l;
+      const double2 e = q[5 * nl], h = q[6 * nl];
+      y[0] = e.x;
+      y[1] = e.y;
+      y[2] = h.x;
+      y[3] = h.y;
+      y[4] = reinterpret_cast<const double*>(q + 7 * nl)[0];
+    } else {
+      const double2 e = p[8 * nl], h = p[9 * nl], w = p[10 * nl];
+      coed = e.x;
+      y[0] = e.y;
+      y[1] = h.x;
+      y[2] = h.y;
+      y[3] = w.x;
+      y[4] = w.y;
     }
   }
+  template <bool FRESH>
+  __device__ __forceinline__ void term(int d, bool upper, const uint4* first, int ps, const uint4* fresh, int sl, int slot,
+                                       double g1, int nvis, double acc[5]) const {
+    const double2* p = reinterpret_cast<const double2*>(first);
+    const double2 uv = p[0], wh = p[ps], ca = p[2 * ps], cv = p[3 * ps], rc = p[4 * ps];
+    const double2* f = FRESH ? reinterpret_cast<const double2*>(fresh) + slot : p + 5 * ps;
+    const int fs = FRESH ? sl : ps;
+    const double2 d01 = f[0], d23 = f[fs];
+    const double dn[5] = {d01.x, d01.y, d23.x, d23.y,
+                          FRESH ? reinterpret_cast<const double*>(fresh + 2 * sl)[slot]
+                                : reinterpret_cast<const double*>(f + 2 * fs)[0]};
+    const double nq[6] = {uv.x, uv.y, wh.x, wh.y, ca.x, ca.y};
+    const double kx = k[3 * d], ky = k[3 * d + 1], kz = k[3 * d + 2];
+    const double c2 = ca.x, cm = cv.x;
+    // the neighbour's state as seen through this point's metric: spectral
+    // radius, split eigenvalues and viscous radius (calc_spectral_radius,
+    // compute_flux_splitting, calc_visc_spectral_radius,
+    // StateUpdater.cpp:175-265)
+    const double ct = uv.x * kx + uv.y * ky + wh.x * kz + 0.0;
+    const double r = fabs(ct) + cm * gm[d];
+    const double gmc = gm[d] < 1.0e-30 ? 1.0e-30 : gm[d];
+    const double sr = upper ? -r : r;
+    double l1 = ct, l4 = ct + cm * gmc, l5 = ct - cm * gmc;
+    l1 = 0.5 * (l1 + sr);
+    l4 = 0.5 * (l4 + sr);
+    l5 = 0.5 * (l5 + sr);
+    double pc[5], nrm[3];
+    pc[0] = l1;
+    pc[1] = quotient(2.0 * l1 - l4 - l5, 2.0 * c2, rc.x);
+    pc[2] = quotient(l4 - l5, 2.0 * cm, rc.y);
+    pc[3] = ct * inv[d];
+    pc[4] = nvis == 1 ? 0.5 * (cv.y * (kx * kx + ky * ky + kz * kz)) : 0.0;
+    nrm[0] = kx * inv[d];
+    nrm[1] = ky * inv[d];
+    nrm[2] = kz * inv[d];
+    split_term<double, MODE>(upper ? 3 : 0, g1, nvis, dn, nq, pc, nrm, acc);
+  }
+  __device__ __forceinline__ void result(const double acc[5], double v[5]) const {
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+      if (MODE == SW_LUSGS_BWD) v[m] = y[m] - acc[m] * coed;
+      else if (MODE == SW_LUSGS_FWD) v[m] = (-y[m] + acc[m]) * coed;
+      else v[m] = (acc[m] + -y[m]) * coed;
+    }
+  }
+  static __device__ __forceinline__ void fresh_store(uint4* fresh, int sl, int slot, const double v[5]) {
+    reinterpret_cast<double2*>(fresh)[slot] = make_double2(v[0], v[1]);
+    reinterpret_cast<double2*>(fresh + sl)[slot] = make_double2(v[2], v[3]);
+    reinterpret_cast<double*>(fresh + 2 * sl)[slot] = v[4];
+  }
+  static __device__ __forceinline__ void store(char* p, int cs, const double v[5]) {
+    *reinterpret_cast<double2*>(p + 5 * cs) = make_double2(v[0], v[1]);
+    *reinterpret_cast<double2*>(p + 6 * cs) = make_double2(v[2], v[3]);
+    *reinterpret_cast<double*>(p + 7 * cs) = v[4];
+  }
+};
 
-  T prev[5] = {T(0), T(0), T(0), T(0), T(0)};  // this thread's increment of the previous step (behind-i)
-  for (int t = 0; t < nsteps; ++t) {
-    cp_async_wait<PD - 2>();   // this thread's copies up to step t+1 have landed
-    compute_barrier(32 * TK);  // everybody's copies up to step t+1 and step t-1's increments are visible
-    if (threadIdx.x == 0 && t > 0) {
-      __threadfence_block();
-      *(volatile int*)&s_done = t;
-    }
-    const int u = t - tj - tk;  // position along i in sweep order
-    if (t + PD < nsteps) {
-      wait_ready(t + PD);
-      prefetch(u + PD, t + PD);
-    }
-    cp_async_commit();
-    if (valid(u)) {
-      const T(*st)[TK][TJ] = s_stat[t % NSS];
-      const int ii = ii_of(u);
-      const int s = ii + jj + kk;
-      const long long c = (long long)rb_own[s] + jj;
-      bool has[6];
-      has[0] = ii > 0;
-      has[1] = jj > 0;
-      has[2] = kk > 0;
-      has[3] = ii < ni - 1;
-      has[4] = jj < nj - 1;
-      has[5] = kk < nk - 1;
-      const int pb = (t - 1) & 1;
-      const T(*rgb)[TK][TJ] = s_ring[(t + NSR - 1) % NSR];
-      const T(*rga)[TK][TJ] = s_ring[(t + 1) % NSR];
-      T rhs0[5] = {T(0), T(0), T(0), T(0), T(0)};
-      // lower neighbours first (i, j, k), then upper (i, j, k): the reference's order
-#pragma unroll
-      for (int q = Q0; q < Q1; ++q) {
-        if (!has[q]) continue;
-        const int d = q % 3;
-        const bool behind = q >= QB && q < QB + 3;
-        T dn[5], nq[8];
-        // source of the neighbour: this thread (i), the adjacent thread (j, k)
-        // in this tile, or another tile (global memory)
-        const bool in_tile = d == 0 || (d == 1 ? (behind ? tj > 0 : tj < TJ - 1) : (behind ? tk > 0 : tk < TK - 1));
-        if (in_tile) {
-          const int sj = d == 1 ? (behind ? tj - 1 : tj + 1) : tj;
-          const int sk = d == 2 ? (behind ? tk - 1 : tk + 1) : tk;
-          const T(*rg)[TK][TJ] = behind ? rgb : rga;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) nq[k] = rg[k][sk][sj];
-          if (behind) {
-            if (d == 0) {
-#pragma unroll
-              for (int m = 0; m < 5; ++m) dn[m] = prev[m];
-            } else {
-#pragma unroll
-              for (int m = 0; m < 5; ++m) dn[m] = s_dq[pb][m][sk][sj];
-            }
-          } else {
-#pragma unroll
-            for (int m = 0; m < 5; ++m) dn[m] = rg[8 + m][sk][sj];
-          }
-        } else {
-          // neighbour in another tile: its record, prefetched with this step's operands
-          const int rec = d == 1 ? (behind ? 0 : 1) * TK + tk : 2 * TK + (behind ? 0 : 1) * 32 + tj;
-          const T* ed = s_edge[t % NSS][rec];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) nq[k] = ed[k];
-#pragma unroll
-          for (int m = 0; m < 5; ++m) dn[m] = ed[8 + m];
-        }
-        // the neighbour's state as seen through this point's metric: spectral
-        // radius, split eigenvalues and viscous radius (calc_spectral_radius,
-        // compute_flux_splitting, calc_visc_spectral_radius,
-        // StateUpdater.cpp:175-265), in the reference's operation order
-        T pc[5], nrm[3];
-        const T kx = st[6 + 3 * d][tk][tj], ky = st[7 + 3 * d][tk][tj], kz = st[8 + 3 * d][tk][tj];
-        const T gmr = st[15 + d][tk][tj], inv = st[18 + d][tk][tj];
-        const T c2 = nq[4], cm = nq[6];
-        const T ct = nq[0] * kx + nq[1] * ky + nq[2] * kz + T(0);
-        const T r = tabs(ct) + cm * gmr;
-        const T gmc = gmr < T(1.0e-30) ? T(1.0e-30) : gmr;
-        const T sign = q < 3 ? T(1) : T(-1);
-        T l1 = ct;
-        T l4 = ct + cm * gmc;
-        T l5 = ct - cm * gmc;
-        l1 = T(0.5) * (l1 + sign * r);
-        l4 = T(0.5) * (l4 + sign * r);
-        l5 = T(0.5) * (l5 + sign * r);
-        pc[0] = l1;
-        pc[1] = (T(2) * l1 - l4 - l5) / (T(2) * c2);
-        pc[2] = (l4 - l5) / (T(2) * cm);
-        pc[3] = (ct - T(0)) * inv;
-        pc[4] = nvis == 1 ? T(0.5) * (nq[7] * (kx * kx + ky * ky + kz * kz)) : T(0);
-        nrm[0] = kx * inv;
-        nrm[1] = ky * inv;
-        nrm[2] = kz * inv;
-        split_term<T, MODE>(q, gm1, nvis, dn, nq, pc, nrm, rhs0);
-      }
-      const T coed = st[0][tk][tj];
-#pragma unroll
-      for (int m = 0; m < 5; ++m) {
-        const T ownv = st[1 + m][tk][tj];
-        const T own = MODE == SW_LUSGS_BWD ? ownv : -ownv;
-        S v;
-        if (MODE == SW_LUSGS_FWD) v = (S)((own + rhs0[m]) * coed);
-        else if (MODE == SW_LUSGS_BWD) v = (S)(own - rhs0[m] * coed);
-        else v = (S)((rhs0[m] + own) * coed);
-        skdq[m * nc + c] = v;
-        s_dq[t & 1][m][tk][tj] = (T)v;
-        prev[m] = (T)v;
-      }
-    }
-    store_edges();
-  }
-  cp_async_wait<0>();
-  compute_barrier(32 * TK);
+// MODE: SW_LUSGS_FWD (lower neighbours), SW_LUSGS_BWD (upper), SW_GS with DIR
+// +1 / -1 (all six).  Warps: kTileThreads compute threads, one warp for the
+// behind halo lines, and one that starts the bulk copies and, on the GS passes,
+// brings the ahead halo lines.
+//
+// Step t handles wave t (forward) or W-1-t.  At its start wave t + FN is sent
+// for; the compute threads wait for wave t+1, update wave t from ring waves
+// t-1 and t+1 and the fresh increments of t-1; the behind warp delivers its
+// lines' fresh increments of wave t (read at t+1).
+template <typename S, typename T, int MODE, int DIR>
+__global__ void __launch_bounds__(kTileThreads + 64, TileLayout<T>::minb)
+    k_sweep_tiles(const BlockDev<S>* __restrict__ blocks, const SweepTile* __restrict__ tiles, int ntiles, int lines,
+                  TileCtl* __restrict__ ctl, int* __restrict__ err, long long spin_limit) {
+  static_assert(sizeof(S) == sizeof(T), "the tile sweeps keep operands in their storage precision");
+  using L = TileLayout<T>;
+  using U = typename EdgeBits<T>::type;
+  constexpr int R = L::ring, NB = L::nb, FN = R - 2;
+  // own pieces copied (the last of the run stay: the backward LU-SGS pass reads no RHS)
+  constexpr int OWN = L::met + (MODE == SW_LUSGS_BWD ? 1 : L::dyn);
+  constexpr bool LOWER = MODE != SW_LUSGS_BWD, UPPER = MODE != SW_LUSGS_FWD;
+  constexpr int FP = (5 * (int)sizeof(T) + 15) / 16;  // 16-byte units of a slot's fresh increment
+  extern __shared__ __align__(128) uint4 ring[];      // R planes, fresh [2][FP][sl], own [R - 1][own][lines]
+  __shared__ unsigned long long s_full[R];
+  __shared__ int s_slot;
+  const int sl = lines + 64;
+  const int plane = NB * sl, fplane = FP * sl, oplane = L::own * lines;
+  uint4* const fresh = ring + R * plane;
+  uint4* const own = fresh + 2 * fplane;
   if (threadIdx.x == 0) {
-    __threadfence_block();
-    *(volatile int*)&s_done = nsteps;
+    s_slot = (int)atomicAdd(&ctl->ticket, 1u);
+#pragma unroll
+    for (int r = 0; r < R; ++r) mbar_init(&s_full[r]);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  // zeros where nothing is ever copied: halo lines outside the block (the last
+  // NB x 64 of a plane), and the wave before the first (ring plane R - 1, fresh
+  // plane 1)
+  for (int x = threadIdx.x; x < R * NB * 64; x += blockDim.x)
+    ring[x / (NB * 64) * plane + NB * lines + x % (NB * 64)] = make_uint4(0, 0, 0, 0);
+  for (int x = threadIdx.x; x < plane; x += blockDim.x) ring[(R - 1) * plane + x] = make_uint4(0, 0, 0, 0);
+  for (int x = threadIdx.x; x < 2 * fplane; x += blockDim.x) fresh[x] = make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // before the bulk copies that reuse plane R - 1
+  __syncthreads();
+  const SweepTile W = tiles[s_slot];
+  const BlockDev<S>& B = blocks[W.block];
+  const int ni = B.ni, jw = W.jw, kh = W.kh, nl = jw * kh;
+  const int nsteps = ni + jw + kh - 2;
+  char* const nb = B.tl_nb;
+  T* const edge = reinterpret_cast<T*>(B.tl_edge);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (warp < kTileThreads / 32) {
+    // ------------------------- compute threads -------------------------
+    const int l = threadIdx.x;
+    const bool line = l < nl;
+    const int tk = l / jw, tj = l - tk * jw;
+    const T g1 = T(B.prm.gamma) - T(1);
+    const int nvis = B.prm.nvis;
+    // the j and k neighbours' lines, in the tile or among the halo lines of
+    // that side: fresh slot, first ring piece in a plane, piece stride
+    constexpr int HL = DIR > 0 ? 0 : 32, HU = DIR > 0 ? 32 : 0;
+    struct Near {
+      int slot, at, ps;
+    };
+    auto near = [&](bool in, int ln, int halo) {
+      return in ? Near{ln, ln, nl} : Near{lines + halo, NB * lines + halo, 64};
+    };
+    const Near jl = near(tj > 0, l - 1, HL + tk), jh = near(tj < jw - 1, l + 1, HU + tk);
+    const Near kl = near(tk > 0, l - jw, HL + kh + tj), kh_ = near(tk < kh - 1, l + jw, HU + kh + tj);
+    int i = line ? (DIR > 0 ? 0 : nsteps - 1) - tj - tk : -(1 << 24);  // this thread's point at step t
+    char* p = nb + ((W.base + (long long)(DIR > 0 ? 0 : nsteps - 1) * nl) * NB + l) * 16;
+    const int ps = DIR * nl * NB * 16;
+    T* out_j = nullptr;  // the records of the downstream tiles this line feeds, at point i
+    T* out_k = nullptr;
+    if (line) {
+      constexpr int o = DIR > 0 ? 1 : 0;
+      if (tj == (DIR > 0 ? jw - 1 : 0) && W.w[o] > 0) out_j = edge + (W.edge_j[o] + tk) * L::rec;
+      if (tk == (DIR > 0 ? kh - 1 : 0) && W.h[o] > 0) out_k = edge + (W.edge_k[o] + tj) * L::rec;
+    }
+    const unsigned full0 = (unsigned)__cvta_generic_to_shared(s_full);
+    const uint4 *pb = ring + (R - 1) * plane, *po = ring, *pa = ring + plane;  // waves t-1, t, t+1
+    const uint4* pown = own;
+    int ra = 1;           // ring index of wave t+1
+    unsigned parity = 0;  // of its barrier
+    mbar_wait(full0, 0, err);
+    __syncthreads();
+    for (int t = 0; t < nsteps; ++t) {
+      mbar_wait(full0 + 8 * ra, parity, err);
+      if ((unsigned)i < (unsigned)ni) {
+        const uint4* const fr = fresh + ((t + 1) & 1) * fplane;  // wave t-1's
+        TilePoint<T, MODE> cur;
+        cur.load(pown, nl, l, po);
+        T acc[5] = {T(0), T(0), T(0), T(0), T(0)}, v[5];
+        // lower neighbours first (i, j, k), then upper (i, j, k): the reference's order
+        if (LOWER) {
+          constexpr bool F = DIR > 0;
+          const uint4* const q = F ? pb : pa;
+          cur.template term<F>(0, false, q + l, nl, fr, sl, l, g1, nvis, acc);
+          cur.template term<F>(1, false, q + jl.at, jl.ps, fr, sl, jl.slot, g1, nvis, acc);
+          cur.template term<F>(2, false, q + kl.at, kl.ps, fr, sl, kl.slot, g1, nvis, acc);
+        }
+        if (UPPER) {
+          constexpr bool F = DIR < 0;
+          const uint4* const q = F ? pb : pa;
+          cur.template term<F>(0, true, q + l, nl, fr, sl, l, g1, nvis, acc);
+          cur.template term<F>(1, true, q + jh.at, jh.ps, fr, sl, jh.slot, g1, nvis, acc);
+          cur.template term<F>(2, true, q + kh_.at, kh_.ps, fr, sl, kh_.slot, g1, nvis, acc);
+        }
+        cur.result(acc, v);
+        TilePoint<T, MODE>::fresh_store(fresh + (t & 1) * fplane, sl, l, v);
+        if (out_j) edge_store(out_j + (long long)i * (kh * L::rec), v);
+        if (out_k) edge_store(out_k + (long long)i * (jw * L::rec), v);
+        TilePoint<T, MODE>::store(p, nl * 16, v);
+      }
+      i += DIR;
+      p += ps;
+      pb = po;
+      po = pa;
+      pa += plane;
+      if (++ra == R) {
+        ra = 0;
+        pa = ring;
+        parity ^= 1;
+      }
+      pown = pown + oplane == own + (R - 1) * oplane ? own : pown + oplane;
+      __syncthreads();
+    }
+  } else {
+    // ------------------- behind / ahead halo lines ----------------------
+    const bool behind = warp == kTileThreads / 32;
+    const int side = (behind == (DIR > 0)) ? 0 : 1;  // lower or upper neighbours
+    const bool isj = lane < kh;
+    const int q = isj ? lane : lane - kh;
+    const bool on = (behind || MODE == SW_GS) && (isj ? W.w[side] > 0 : (q < jw && W.h[side] > 0));
+    const int tj = isj ? (side ? jw : -1) : q, tk = isj ? q : (side ? kh : -1);
+    const int halo = (behind ? 0 : 32) + lane;
+    // the neighbour tile's own coordinates of this line
+    const int ow = isj ? W.w[side] : jw, oh = isj ? kh : W.h[side];
+    const int oj = isj ? (side ? 0 : ow - 1) : q, ok = isj ? q : (side ? 0 : oh - 1);
+    const int onl = ow * oh;
+    int i = on ? (DIR > 0 ? 0 : nsteps - 1) - tj - tk : -(1 << 24);  // its point on step 0
+    const char* src =
+        nb + (((isj ? W.base_j[side] : W.base_k[side]) + (long long)(i + oj + ok) * onl) * NB + ok * ow + oj) * 16;
+    const int ss = DIR * onl * NB * 16;
+    auto valid = [&](int x) { return (unsigned)x < (unsigned)ni; };
+    auto fetch = [&](int r, int s) {  // the line's point s steps from now into ring index r
+      if (valid(i + s * DIR)) {
+        const char* g = src + s * ss;
+        uint4* dst = ring + r * plane + NB * lines + halo;
+#pragma unroll
+        for (int c = 0; c < NB; ++c) cp_async16(dst + c * 64, g + c * onl * 16);
+      }
+    };
+    if (!behind) {
+      // a wave's bulk copies: lane 0 the neighbour state, lane 1 the own operands
+      const bool own_run = lane == 1;
+      const int per = own_run ? L::own : NB;
+      const char* const run = (own_run ? B.tl_own : nb) + (W.base + (long long)(DIR > 0 ? 0 : nsteps - 1) * nl) * per * 16;
+      uint4* const into = own_run ? own : ring;
+      const int into_plane = own_run ? oplane : plane, into_ring = own_run ? R - 1 : R;
+      const long long ws = (long long)DIR * nl * per * 16;
+      const unsigned bytes = (unsigned)nl * 16;
+      auto send = [&](int w) {  // wave w of the sweep, 0 .. nsteps (the zeros past the last)
+        unsigned long long* const m = &s_full[w % R];
+        if (lane == 0) mbar_expect(m, bytes * (NB + OWN));
+        __syncwarp();
+        if (lane < 2) bulk_copy(into + w % into_ring * into_plane, run + w * ws, bytes * (own_run ? OWN : NB), m);
+      };
+#pragma unroll
+      for (int s = 0; s < FN; ++s) {
+        send(s);
+        fetch(s, s);
+        cp_async_commit();
+      }
+      cp_async_wait<FN - 2>();
+      __syncthreads();
+      int r = FN;  // ring index of wave t + FN
+      for (int t = 0; t < nsteps; ++t) {
+        if (t + FN <= nsteps) send(t + FN);
+        fetch(r, FN);
+        cp_async_commit();
+        i += DIR;
+        src += ss;
+        if (++r == R) r = 0;
+        cp_async_wait<FN - 2>();
+        __syncthreads();
+      }
+    } else {
+      // Records are asked for in pairs, two and three steps before they are due,
+      // so that no step waits for an L2 load.  (In pairs: a warp's wait for a
+      // load is a wait for every later load too, so asking at every step makes
+      // every step as long as a load.)
+      const int per = (isj ? kh : jw) * L::rec;
+      const int slot = lines + halo;
+      T* const rec = edge + ((isj ? W.edge_j[side] : W.edge_k[side]) + q) * L::rec;
+      bool dead = false;
+      U b[2][2][5];
+      auto ask = [&](int x, U(&r)[2][5]) {  // reads the records of points x and x + DIR without waiting for them to fill
+        if (valid(x)) edge_load(rec + (long long)x * per, r[0]);
+        if (valid(x + DIR)) edge_load(rec + (long long)(x + DIR) * per, r[1]);
+      };
+      // fresh increments of step s's wave (the lane's point x) into fresh plane s & 1
+      auto deliver = [&](int s, int x, U(&r)[5]) {
+        bool full = !valid(x) || edge_full(r);
+        long long it = 0;
+        while (!dead && __any_sync(0xffffffffu, !full)) {
+          bool stop = ++it > spin_limit;
+          if ((it & 31) == 0 && *(volatile int*)err) stop = true;
+          if (__any_sync(0xffffffffu, stop)) {
+            if (lane == 0) atomicExch(err, 1);
+            dead = true;
+            break;
+          }
+          if (it > 8) __nanosleep(32);
+          if (!full) {
+            edge_load(rec + (long long)x * per, r);
+            full = edge_full(r);
+          }
+        }
+        if (valid(x)) {
+          T v[5];
+#pragma unroll
+          for (int m = 0; m < 5; ++m) memcpy(&v[m], &r[m], sizeof(T));
+          TilePoint<T, MODE>::fresh_store(fresh + (s & 1) * fplane, sl, slot, v);
+          edge_clear(rec + (long long)x * per);
+        }
+      };
+      fetch(R - 1, -1);
+#pragma unroll
+      for (int s = 0; s < FN; ++s) {
+        fetch(s, s);
+        cp_async_commit();
+      }
+      ask(i - DIR, b[0]);  // steps -1 and 0
+      ask(i + DIR, b[1]);  // steps 1 and 2
+      cp_async_wait<FN - 2>();
+      deliver(-1, i - DIR, b[0][0]);
+      __syncthreads();
+      int r = FN;
+      for (int t0 = 0; t0 < nsteps; t0 += 4) {
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+          const int t = t0 + d;
+          if (t < nsteps) {
+            fetch(r, FN);
+            cp_async_commit();
+            deliver(t, i, b[((d + 1) / 2) & 1][(d + 1) & 1]);
+            if (d & 1) ask(i + 2 * DIR, b[(d / 2) & 1]);  // steps t + 2 and t + 3
+            i += DIR;
+            src += ss;
+            if (++r == R) r = 0;
+            cp_async_wait<FN - 2>();
+            __syncthreads();
+          }
+        }
+      }
+    }
+  }
+  if (threadIdx.x == 0) {
+    const unsigned int n = atomicAdd(&ctl->done, 1u);
+    if (n + 1 == (unsigned)ntiles) {  // every CTA has its ticket: ready for the next launch
+      ctl->ticket = 0;
+      ctl->done = 0;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// natural order -> tile layout
+// ---------------------------------------------------------------------------
+// Static operands (metrics, magnitudes), refreshed whenever the metrics are set.
+template <typename S>
+__global__ void k_tile_static(const BlockDev<S>* __restrict__ blocks, int b) {
+  const BlockDev<S>& B = blocks[b];
+  const long long np = B.npad;
+  for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < B.ncomp; n += (long long)gridDim.x * blockDim.x) {
+    const int n32 = (int)n, r32 = n32 / B.ni;
+    const int ii = n32 - r32 * B.ni, jj = r32 % B.nj, kk = r32 / B.nj;
+    const long long idx = lin(B, NG + ii, NG + jj, NG + kk);
+    const TileSlot at = tile_slot(B, ii, jj, kk);
+    S k[9], gm[3], inv[3];
+    for (int m = 0; m < 9; ++m) k[m] = (S)B.metrics[m * np + idx];
+    for (int d = 0; d < 3; ++d) {  // unit normals of compute_flux_splitting (StateUpdater.cpp:231-249)
+      gm[d] = sqrt_s(k[3 * d] * k[3 * d] + k[3 * d + 1] * k[3 * d + 1] + k[3 * d + 2] * k[3 * d + 2]);
+      inv[d] = S(1) / (gm[d] < S(1.0e-30) ? S(1.0e-30) : gm[d]);
+    }
+    using L = TileLayout<S>;
+    if constexpr (sizeof(S) == 4) {
+      float4* const p = at.run<float4>(B.tl_own, L::own);
+      for (int d = 0; d < 3; ++d) p[d * at.nl] = make_float4(k[3 * d], k[3 * d + 1], k[3 * d + 2], gm[d]);
+    } else {
+      double2* const p = at.run<double2>(B.tl_own, L::own);
+      for (int d = 0; d < 3; ++d) {
+        p[2 * d * at.nl] = make_double2(k[3 * d], k[3 * d + 1]);
+        p[(2 * d + 1) * at.nl] = make_double2(k[3 * d + 2], gm[d]);
+      }
+      p[6 * at.nl] = make_double2(inv[0], inv[1]);
+      p[7 * at.nl] = make_double2(inv[2], 0.0);
+    }
+  }
+}
+
+// Per step: masked RHS, diagonal coefficient and the state a neighbour's term
+// needs (k_lusgs_prep's values), read coalesced in natural order and written
+// in 16-byte pieces.
+template <typename S, typename T>
+__global__ void __launch_bounds__(256, PointwiseMinBlocks<T>::n) k_tile_prep(const BlockDev<S>* __restrict__ blocks,
+                                                                             const Chunk* __restrict__ chunks) {
+  const Chunk ch = chunks[blockIdx.x];
+  const BlockDev<S>& B = blocks[ch.block];
+  if ((int)threadIdx.x >= ch.count) return;
+  const ParamsDev& P = B.prm;
+  const long long np = B.npad;
+  const int n32 = (int)ch.start + threadIdx.x, r32 = n32 / B.ni;
+  const int ii = n32 - r32 * B.ni, jj = r32 % B.nj, kk = r32 / B.nj;
+  const long long idx = lin(B, NG + ii, NG + jj, NG + kk);
+  const TileSlot at = tile_slot(B, ii, jj, kk);
+  const bool masked = B.bcmask[idx] != 0;
+  T rhs[5];
+  for (int m = 0; m < 5; ++m) rhs[m] = masked ? T(0) : (T)B.dq[m * np + idx];
+  const S* pr = FluxSrc<S>::prim(B);
+  const T rho = (T)pr[idx], u = (T)pr[np + idx], v = (T)pr[2 * np + idx], w = (T)pr[3 * np + idx],
+          p = (T)pr[4 * np + idx];
+  PrepPoint<T> q;
+  {
+    const S* met = FluxSrc<S>::metrics(B);
+    T km[9];
+    for (int m = 0; m < 9; ++m) km[m] = (T)met[m * np + idx];
+    q.form(P, rho, u, v, w, p, km, (T)B.mu[idx], (T)FluxSrc<S>::vol(B)[idx], (T)B.dt[idx]);
+  }
+  using L = TileLayout<T>;
+  const int nl = at.nl;
+  if constexpr (sizeof(T) == 4) {
+    float4* const y = at.run<float4>(B.tl_own, L::own) + L::met * nl;
+    y[0] = make_float4(q.coed, rhs[0], rhs[1], rhs[2]);
+    y[nl] = make_float4(rhs[3], rhs[4], 0.f, 0.f);
+    float4* const z = at.run<float4>(B.tl_nb, L::nb);
+    z[0] = make_float4(u, v, w, q.H);
+    z[nl] = make_float4(q.c, q.vcoef, q.af, 0.f);
+  } else {
+    double2* const y = at.run<double2>(B.tl_own, L::own) + L::met * nl;
+    y[0] = make_double2(q.coed, rhs[0]);
+    y[nl] = make_double2(rhs[1], rhs[2]);
+    y[2 * nl] = make_double2(rhs[3], rhs[4]);
+    double2* const z = at.run<double2>(B.tl_nb, L::nb);
+    z[0] = make_double2(u, v);
+    z[nl] = make_double2(w, q.H);
+    z[2 * nl] = make_double2(q.c2, q.af);
+    z[3 * nl] = make_double2(q.c, q.vcoef);
+    z[4 * nl] = make_double2(quotient_rcp(2.0 * q.c2), quotient_rcp(2.0 * q.c));
   }
 }
 

@@ -64,6 +64,8 @@ struct DeviceLists {
   int lanes[3] = {1, 1, 1};
   int lanes_cap = 32;                            // line tiles: at most this many grid lines per CTA (set at creation)
   int lmax[3] = {0, 0, 0};
+  LineChunk* inv_chunks[3] = {nullptr, nullptr, nullptr};  // inviscid kernels' chunks of lines
+  int n_inv_chunks[3] = {0, 0, 0};
   int line_units[3] = {0, 0, 0};                 // line tiles' face slots (lanes x (longest line + 1)) of shared memory
   Chunk* sweep_chunks[2] = {nullptr, nullptr};  // forward / backward hyperplane launches
   std::vector<int> sweep_off[2];                 // host: chunk range of each launch

@@ -96,6 +96,11 @@ struct LineTile {
   int pad;
 };
 
+// Points [c0, c1) of `count` lines from line `first` (inviscid.cuh).
+struct LineChunk {
+  int block, first, count, c0, c1;
+};
+
 // One physical BC region, memory coordinates (ghost offset applied).
 struct RegionDev {
   int block;

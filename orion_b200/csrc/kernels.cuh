@@ -28,6 +28,23 @@ template <> struct FluxSrc<float> {
 };
 
 
+// Asynchronous copies of 16 bytes or of one value into shared memory.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  const unsigned int s = (unsigned int)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void cp_async_value(double* smem, const double* gmem) {
+  const unsigned int s = (unsigned int)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_value(float* smem, const float* gmem) {
+  const unsigned int s = (unsigned int)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
 template <typename S>
 __device__ __forceinline__ long long lin(const BlockDev<S>& B, int i, int j, int k) {
   return (long long)i + (long long)B.nx * ((long long)j + (long long)B.ny * (long long)k);
@@ -684,15 +701,14 @@ __device__ __forceinline__ void tile_item(int it, int nlanes, int nfaces, int& l
 }
 
 // CTAs per SM the line kernels are compiled for (register cap 65536/(256*n)),
-// per compute precision, measured on C3: FP32 five (viscous; 3.91 ms against
-// 4.03 at six and 4.09 at four) and five (inviscid; four and six were slower),
-// FP64 three (viscous) and three (inviscid, with its boundary rounds in their
-// own kernel; two CTAs when they were inline).
+// per compute precision, measured on C3: viscous FP32 five (3.91 ms against
+// 4.03 at six and 4.09 at four), FP64 three; inviscid FP32 four, FP64 three
+// (inviscid.cuh).
 #ifndef ORION_VISC_MINB_F32
 #define ORION_VISC_MINB_F32 5
 #endif
 #ifndef ORION_INV_MINB_F32
-#define ORION_INV_MINB_F32 5
+#define ORION_INV_MINB_F32 4
 #endif
 #ifndef ORION_VISC_MINB_F64
 #define ORION_VISC_MINB_F64 3
@@ -747,327 +763,6 @@ __global__ void __launch_bounds__(256, LineMinBlocks<T>::visc) k_viscous(const B
     }
   }
 }
-
-// ===========================================================================
-// Inviscid RHS along one direction D (compute_block_inviscid + compute_flux_line,
-// src/solver/InviscidFluxComputer.cpp:136-192, 238-522, 543-647).
-// Face fluxes from WCNS-E-5 states (fixed stencils where the ghost-3 density
-// flag is set) and the Roe flux, then the flux difference; the boundary
-// re-calculation rounds (:377-521) are evaluated per output point by the
-// threads of points 0..2 and L-3..L-1 of flagged line ends.
-// ===========================================================================
-template <typename S, typename T>
-struct InvLine {
-  const S* prim;  // FluxSrc<S>::prim
-  long long o, st, np;
-  int L;
-  __device__ __forceinline__ T q(int p, int m) const { return (T)prim[m * np + o + (long long)p * st]; }
-};
-
-template <typename S, typename T>
-__device__ __forceinline__ T metric_half(const BlockDev<S>& B, int mc, long long o, long long st, int f, int L) {
-  // interp_metrics_half (InviscidFluxComputer.cpp:136-192), ni > 2
-  const S* a = FluxSrc<S>::metrics(B) + mc * B.npad;
-  auto Q = [&](int p) -> T { return (T)a[o + (long long)p * st]; };
-  if (f == 0) return (T(35) * Q(3) + T(-35) * Q(4) + T(21) * Q(5) + T(-5) * Q(6)) / T(16);
-  if (f == 1) return (T(5) * Q(3) + T(15) * Q(4) + T(-5) * Q(5) + T(1) * Q(6)) / T(16);
-  if (f == L) return (T(35) * Q(L + 2) + T(-35) * Q(L + 1) + T(21) * Q(L) + T(-5) * Q(L - 1)) / T(16);
-  if (f == L - 1) return (T(5) * Q(L + 2) + T(15) * Q(L + 1) + T(-5) * Q(L) + T(1) * Q(L - 1)) / T(16);
-  return (T(9) * (Q(f + 2) + Q(f + 3)) + T(-1) * (Q(f + 4) + Q(f + 1))) / T(16);
-}
-
-// Initial left/right states at face f (main WCNS loop + fixed boundary stencils).
-template <typename S, typename T>
-__device__ __forceinline__ void initial_states(const InvLine<S, T>& ln, int f, bool fl, bool fr, T ql[5], T qr[5]) {
-  const int L = ln.L;
-  const int ist = fl ? 2 : 0, ied = fr ? L - 2 : L;
-  for (int m = 0; m < 5; ++m) {
-    T l = T(0), r = T(0);
-    if (f >= ist && f <= ied) {
-      const T a0 = ln.q(f, m), a1 = ln.q(f + 1, m), a2 = ln.q(f + 2, m), a3 = ln.q(f + 3, m), a4 = ln.q(f + 4, m),
-              a5 = ln.q(f + 5, m);
-      l = wcns_left<T>(a0, a1, a2, a3, a4);
-      r = wcns_right<T>(a1, a2, a3, a4, a5);
-    }
-    if (ist > 1 && f <= 2) {
-      const T q1 = ln.q(3, m), q2 = ln.q(4, m), q3 = ln.q(5, m), q4 = ln.q(6, m);
-      if (f == 0) {
-        l = (T(35.) * q1 - T(35.) * q2 + T(21.) * q3 - T(5.) * q4) / T(16.);
-        r = l;
-      } else if (f == 1) {
-        l = (T(5.) * q1 + T(15.) * q2 - T(5.) * q3 + q4) / T(16.);
-        r = l;
-      } else {
-        l = (-q1 + T(9.) * q2 + T(9.) * q3 - q4) / T(16.);
-      }
-    }
-    if (ied < L && f >= L - 2) {
-      const T qn = ln.q(L + 2, m), qn1 = ln.q(L + 1, m), qn2 = ln.q(L, m), qn3 = ln.q(L - 1, m);
-      if (f == L) {
-        r = (T(35.) * qn - T(35.) * qn1 + T(21.) * qn2 - T(5.) * qn3) / T(16.);
-        l = r;
-      } else if (f == L - 1) {
-        r = (T(5.) * qn + T(15.) * qn1 - T(5.) * qn2 + qn3) / T(16.);
-        l = r;
-      } else {
-        r = (-qn + T(9.) * qn1 + T(9.) * qn2 - qn3) / T(16.);
-      }
-    }
-    ql[m] = l;
-    qr[m] = r;
-  }
-}
-
-template <int D, typename S, typename T>
-__device__ __forceinline__ void face_metric(const BlockDev<S>& B, long long o, long long st, int f, int L, T& kx,
-                                            T& ky, T& kz) {
-  kx = metric_half<S, T>(B, 3 * D + 0, o, st, f, L);
-  ky = metric_half<S, T>(B, 3 * D + 1, o, st, f, L);
-  kz = metric_half<S, T>(B, 3 * D + 2, o, st, f, L);
-}
-
-// Positivity fallback + Roe flux at face f (calc_flux_loop, InviscidFluxComputer.cpp:342-364).
-template <typename S, typename T>
-__device__ __forceinline__ void fallback_roe(const InvLine<S, T>& ln, int f, T ql[5], T qr[5], T kx, T ky, T kz,
-                                             T gamma, T out[5]) {
-  const int L = ln.L;
-  if (ql[0] <= T(1e-6) || ql[4] <= T(1e-6)) {
-    const int p = (f - 1 > 0 ? f - 1 : 0) + 2;
-    for (int m = 0; m < 5; ++m) ql[m] = ln.q(p, m);
-  }
-  if (qr[0] <= T(1e-6) || qr[4] <= T(1e-6)) {
-    const int p = (L - 1 < f ? L - 1 : f) + 3;
-    for (int m = 0; m < 5; ++m) qr[m] = ln.q(p, m);
-  }
-  roe_flux<T>(ql, qr, kx, ky, kz, T(0), T(0.1), gamma, out);
-}
-
-// Left-end re-calculation rounds (InviscidFluxComputer.cpp:377-448): the value
-// of fc[t] for t = 0, 1, 2 when the ghost-3 density flag is set.
-// Boundary re-calculation rounds of a flagged line end
-// (InviscidFluxComputer.cpp:377-521).  Each output point needs one round of
-// 4-5 Roe fluxes; every flux is folded into the output as soon as it is
-// computed, in the order and with the coefficients of the reference's formula,
-// so no per-face array is kept.
-template <int D, typename S, typename T>
-struct Cascade {
-  const BlockDev<S>& B;
-  const InvLine<S, T>& ln;
-  T gamma;
-  T acc[5];
-  __device__ __forceinline__ void flux(int f, const T l[5], const T r[5], T coef, bool first) {
-    T ql[5], qr[5], out[5];
-    for (int m = 0; m < 5; ++m) { ql[m] = l[m]; qr[m] = r[m]; }
-    T kx, ky, kz;
-    face_metric<D, S, T>(B, ln.o, ln.st, f, ln.L, kx, ky, kz);
-    fallback_roe<S, T>(ln, f, ql, qr, kx, ky, kz, gamma, out);
-    // acc = coef*F (first term) or acc + coef*F; a coefficient of +1 or -1 is an
-    // exact add or subtract of F as in the reference's expression
-    for (int m = 0; m < 5; ++m) {
-      if (first) acc[m] = coef * out[m];
-      else if (coef == T(1)) acc[m] = acc[m] + out[m];
-      else if (coef == T(-1)) acc[m] = acc[m] - out[m];
-      else acc[m] = acc[m] + coef * out[m];
-    }
-  }
-};
-
-template <int D, typename S, typename T>
-__device__ void cascade_left(const BlockDev<S>& B, const InvLine<S, T>& ln, int t, T gamma, T fc[5]) {
-  Cascade<D, S, T> cs{B, ln, gamma, {}};
-  T Q3[5], Q4[5], Q5[5], Q6[5];
-  for (int m = 0; m < 5; ++m) { Q3[m] = ln.q(3, m); Q4[m] = ln.q(4, m); Q5[m] = ln.q(5, m); Q6[m] = ln.q(6, m); }
-  T s[5], s2[5];
-  if (t == 0) {
-    // fc[0] = (-23 F0 + 21 F1 + 3 F2 - F3) / 24 over round-1 states
-    for (int m = 0; m < 5; ++m) s[m] = (T(3.) * Q3[m] - T(1.) * Q4[m]) / T(2.0);
-    cs.flux(0, s, s, T(-23.), true);
-    for (int m = 0; m < 5; ++m) s[m] = (T(19.) * Q3[m] + T(25.) * Q4[m] - T(2.) * Q5[m]) / T(42.0);
-    cs.flux(1, s, s, T(21.), false);
-    for (int m = 0; m < 5; ++m) s[m] = (T(4.) * Q3[m] + T(3.) * Q4[m] + T(9.) * Q5[m] + T(2.) * Q6[m]) / T(18.0);
-    cs.flux(2, s, s, T(3.), false);
-    for (int m = 0; m < 5; ++m) s[m] = (T(-2.) * Q3[m] + T(3.) * Q4[m] + T(3.) * Q5[m] + T(2.) * Q6[m]) / T(6.0);
-    cs.flux(3, s, s, T(-1), false);
-  } else if (t == 1) {
-    // fc[1] = (-22 F1 + 17 F2 + 9 F3 - 5 F4 + F5) / 24 over round-2 states
-    for (int m = 0; m < 5; ++m) s[m] = (T(3.) * Q3[m] + T(6.) * Q4[m] - Q5[m]) / T(8.0);
-    cs.flux(1, s, s, T(-22.), true);
-    for (int m = 0; m < 5; ++m) {
-      s[m] = (T(-30.) * Q3[m] + T(145.) * Q4[m] + T(29.) * Q5[m] - T(8.) * Q6[m]) / T(136.0);
-      s2[m] = (T(2.) * Q3[m] + T(49.) * Q4[m] + T(125.) * Q5[m] - T(40.) * Q6[m]) / T(136.0);
-    }
-    cs.flux(2, s, s2, T(17.), false);
-    for (int m = 0; m < 5; ++m) s[m] = (-Q4[m] + T(6.) * Q5[m] + T(3.) * Q6[m]) / T(8.0);
-    cs.flux(3, s, s, T(9.), false);
-    for (int m = 0; m < 5; ++m) s[m] = (Q4[m] + T(2.) * Q5[m] + T(5.) * Q6[m]) / T(8.0);
-    cs.flux(4, s, s, T(-5.), false);
-    for (int m = 0; m < 5; ++m) s[m] = (Q4[m] + Q5[m] + T(6.) * Q6[m]) / T(8.0);
-    cs.flux(5, s, s, T(1), false);
-  } else {
-    // fc[2] = (F1 - 27 F2 + 27 F3 - F4) / 24 over round-3 states; face 1 keeps the
-    // round-2 left state and the restored fixed right state, faces 2..4 the
-    // restored WCNS right states
-    for (int m = 0; m < 5; ++m) {
-      s[m] = (T(3.) * Q3[m] + T(6.) * Q4[m] - Q5[m]) / T(8.0);
-      s2[m] = (T(5.) * Q3[m] + T(15.) * Q4[m] - T(5.) * Q5[m] + Q6[m]) / T(16.);
-    }
-    cs.flux(1, s, s2, T(1), true);
-    const T coef[3] = {T(-27.), T(27.), T(-1)};
-    for (int f = 2; f <= 4; ++f) {
-      for (int m = 0; m < 5; ++m) {
-        if (f == 2) s[m] = (T(-29.) * Q3[m] + T(170.) * Q4[m] + T(63.) * Q5[m] + T(12.) * Q6[m]) / T(216.0);
-        else if (f == 3) s[m] = (-Q4[m] + T(6.) * Q5[m] + T(3.) * Q6[m]) / T(8.0);
-        else s[m] = (Q4[m] + T(2.) * Q5[m] + T(5.) * Q6[m]) / T(8.0);
-        s2[m] = wcns_right<T>(ln.q(f + 1, m), ln.q(f + 2, m), ln.q(f + 3, m), ln.q(f + 4, m), ln.q(f + 5, m));
-      }
-      cs.flux(f, s, s2, coef[f - 2], false);
-    }
-  }
-  for (int m = 0; m < 5; ++m) fc[m] = cs.acc[m] / T(24.0);
-}
-
-template <int D, typename S, typename T>
-__device__ void cascade_right(const BlockDev<S>& B, const InvLine<S, T>& ln, int t, T gamma, T fc[5]) {
-  const int N = ln.L;
-  Cascade<D, S, T> cs{B, ln, gamma, {}};
-  T Qn[5], Qn1[5], Qn2[5], Qn3[5];
-  for (int m = 0; m < 5; ++m) {
-    Qn[m] = ln.q(N + 2, m); Qn1[m] = ln.q(N + 1, m); Qn2[m] = ln.q(N, m); Qn3[m] = ln.q(N - 1, m);
-  }
-  T s[5], s2[5];
-  if (t == N - 1) {
-    // fc[N-1] = -(-23 F[N] + 21 F[N-1] + 3 F[N-2] - F[N-3]) / 24
-    for (int m = 0; m < 5; ++m) s[m] = (T(3.) * Qn[m] - T(1.) * Qn1[m]) / T(2.0);
-    cs.flux(N, s, s, T(-23.), true);
-    for (int m = 0; m < 5; ++m) s[m] = (T(19.) * Qn[m] + T(25.) * Qn1[m] - T(2.) * Qn2[m]) / T(42.0);
-    cs.flux(N - 1, s, s, T(21.), false);
-    for (int m = 0; m < 5; ++m) s[m] = (T(4.) * Qn[m] + T(3.) * Qn1[m] + T(9.) * Qn2[m] + T(2.) * Qn3[m]) / T(18.0);
-    cs.flux(N - 2, s, s, T(3.), false);
-    for (int m = 0; m < 5; ++m) s[m] = (T(-2.) * Qn[m] + T(3.) * Qn1[m] + T(3.) * Qn2[m] + T(2.) * Qn3[m]) / T(6.0);
-    cs.flux(N - 3, s, s, T(-1), false);
-  } else if (t == N - 2) {
-    // fc[N-2] = -(-22 F[N-1] + 17 F[N-2] + 9 F[N-3] - 5 F[N-4] + F[N-5]) / 24
-    for (int m = 0; m < 5; ++m) s[m] = (T(3.) * Qn[m] + T(6.) * Qn1[m] - Qn2[m]) / T(8.0);
-    cs.flux(N - 1, s, s, T(-22.), true);
-    for (int m = 0; m < 5; ++m) {
-      s2[m] = (T(-30.) * Qn[m] + T(145.) * Qn1[m] + T(29.) * Qn2[m] - T(8.) * Qn3[m]) / T(136.0);  // right
-      s[m] = (T(2.) * Qn[m] + T(49.) * Qn1[m] + T(125.) * Qn2[m] - T(40.) * Qn3[m]) / T(136.0);    // left
-    }
-    cs.flux(N - 2, s, s2, T(17.), false);
-    for (int m = 0; m < 5; ++m) s[m] = (-Qn1[m] + T(6.) * Qn2[m] + T(3.) * Qn3[m]) / T(8.0);
-    cs.flux(N - 3, s, s, T(9.), false);
-    for (int m = 0; m < 5; ++m) s[m] = (Qn1[m] + T(2.) * Qn2[m] + T(5.) * Qn3[m]) / T(8.0);
-    cs.flux(N - 4, s, s, T(-5.), false);
-    for (int m = 0; m < 5; ++m) s[m] = (Qn1[m] + Qn2[m] + T(6.) * Qn3[m]) / T(8.0);
-    cs.flux(N - 5, s, s, T(1), false);
-  } else {
-    // fc[N-3] = -(F[N-1] - 27 F[N-2] + 27 F[N-3] - F[N-4]) / 24
-    for (int m = 0; m < 5; ++m) {
-      s2[m] = (T(3.) * Qn[m] + T(6.) * Qn1[m] - Qn2[m]) / T(8.0);
-      s[m] = (T(5.) * Qn[m] + T(15.) * Qn1[m] - T(5.) * Qn2[m] + Qn3[m]) / T(16.);
-    }
-    cs.flux(N - 1, s, s2, T(1), true);
-    const T coef[3] = {T(-27.), T(27.), T(-1)};
-    for (int f = N - 2; f >= N - 4; --f) {
-      for (int m = 0; m < 5; ++m) {
-        if (f == N - 2) s2[m] = (T(-29.) * Qn[m] + T(170.) * Qn1[m] + T(63.) * Qn2[m] + T(12.) * Qn3[m]) / T(216.0);
-        else if (f == N - 3) s2[m] = (-Qn1[m] + T(6.) * Qn2[m] + T(3.) * Qn3[m]) / T(8.0);
-        else s2[m] = (Qn1[m] + T(2.) * Qn2[m] + T(5.) * Qn3[m]) / T(8.0);
-        s[m] = wcns_left<T>(ln.q(f, m), ln.q(f + 1, m), ln.q(f + 2, m), ln.q(f + 3, m), ln.q(f + 4, m));
-      }
-      cs.flux(f, s, s2, coef[N - 2 - f], false);
-    }
-  }
-  for (int m = 0; m < 5; ++m) fc[m] = -cs.acc[m] / T(24.0);
-}
-
-// Boundary re-calculation of flagged line ends (InviscidFluxComputer.cpp:377-521)
-// for one tile: the six outputs of each line's two ends by consecutive threads.
-// k_inviscid's regular loop skips these points, so each point's dq gets
-// direction D's terms once and in direction order.
-template <int D, typename S, typename T>
-__device__ __forceinline__ void inv_boundary_rounds(const BlockDev<S>& B, const LineTile& tl, int L, long long st,
-                                                    T gamma) {
-  const int nbnd = tl.count * 6;
-  for (int it = threadIdx.x; it < nbnd; it += blockDim.x) {
-    const int lane = it / 6, slot = it - lane * 6;
-    const long long o = line_origin(B, D, tl.first + lane);
-    const bool left = slot < 3;
-    const bool flag = left ? (B.prim[o] < 1.0e-20) : (B.prim[o + (long long)(L + 5) * st] < 1.0e-20);
-    if (!flag) continue;
-    const int t = left ? slot : L - 6 + slot;
-    InvLine<S, T> ln{FluxSrc<S>::prim(B), o, st, B.npad, L};
-    T fc[5];
-    if (left) cascade_left<D, S, T>(B, ln, t, gamma, fc);
-    else cascade_right<D, S, T>(B, ln, t, gamma, fc);
-    const long long idx = o + (long long)(t + NG) * st;
-    for (int m = 0; m < 5; ++m) {
-      S* q = B.dq + m * B.npad + idx;
-      *q = (S)((T)*q + fc[m]);
-    }
-  }
-}
-
-// The boundary rounds run in their own launch after k_inviscid<D>, over the
-// same tiles, with CTAs sized to a tile's six outputs per line: inlined, their
-// Roe fluxes need about 128 (FP32) or 250 (FP64) registers, against 48 and 80
-// for the face loop.  On C3 the split took the inviscid stage from 3.61 to
-// 3.25 ms mixed and from 12.2 to 11.9 ms plain (the FP64 face loop at three
-// CTAs per SM).
-template <int D, typename S, typename T>
-__global__ void __launch_bounds__(256) k_inv_cascade(const BlockDev<S>* __restrict__ blocks,
-                                                     const LineTile* __restrict__ tiles) {
-  const LineTile tl = tiles[blockIdx.x];
-  const BlockDev<S> B = blocks[tl.block];
-  inv_boundary_rounds<D, S, T>(B, tl, dim_along(B, D), stride_along(B, D), T(B.prm.gamma));
-}
-
-template <int D, typename S, typename T>
-__global__ void __launch_bounds__(256, LineMinBlocks<T>::inv) k_inviscid(const BlockDev<S>* __restrict__ blocks, const LineTile* __restrict__ tiles) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* fsh = reinterpret_cast<T*>(smem_raw);
-  const LineTile tl = tiles[blockIdx.x];
-  const BlockDev<S> B = blocks[tl.block];
-  const ParamsDev& P = B.prm;
-  const int L = dim_along(B, D);
-  const int nf = L + 1;
-  const long long st = stride_along(B, D);
-  const T gamma = T(P.gamma);
-  const int nitems = tl.count * nf;
-  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    int lane, f;
-    tile_item<D>(it, tl.count, nf, lane, f);
-    const long long o = line_origin(B, D, tl.first + lane);
-    InvLine<S, T> ln{FluxSrc<S>::prim(B), o, st, B.npad, L};
-    const bool fl = B.prim[o] < 1.0e-20;
-    const bool fr = B.prim[o + (long long)(L + 5) * st] < 1.0e-20;
-    T ql[5], qr[5], kx, ky, kz, fo[5];
-    initial_states<S, T>(ln, f, fl, fr, ql, qr);
-    face_metric<D, S, T>(B, o, st, f, L, kx, ky, kz);
-    fallback_roe<S, T>(ln, f, ql, qr, kx, ky, kz, gamma, fo);
-    T* dst = fsh + ((size_t)lane * nf + f) * 5;
-    for (int m = 0; m < 5; ++m) dst[m] = fo[m];
-  }
-  __syncthreads();
-  // regular points: flux difference of the face fluxes
-  const int npts = tl.count * L;
-  for (int it = threadIdx.x; it < npts; it += blockDim.x) {
-    int lane, t;
-    tile_item<D>(it, tl.count, L, lane, t);
-    const long long o = line_origin(B, D, tl.first + lane);
-    const bool fl = B.prim[o] < 1.0e-20;
-    const bool fr = B.prim[o + (long long)(L + 5) * st] < 1.0e-20;
-    if ((fl && t <= 2) || (fr && t >= L - 3)) continue;  // re-calculated below
-    const long long idx = o + (long long)(t + NG) * st;
-    const T* fb = fsh + (size_t)lane * nf * 5;
-    for (int m = 0; m < 5; ++m) {
-      S* q = B.dq + m * B.npad + idx;
-      *q = (S)((T)*q + flux_diff<T>(fb + m, 5, t, L));
-    }
-  }
-
-}
-
 
 // ===========================================================================
 // Interface residual averaging (HaloExchanger::average_interface_residuals,

@@ -19,16 +19,42 @@ template <> __device__ __forceinline__ double tsqrt<double>(double x) { return s
 template <> __device__ __forceinline__ float tsqrt<float>(float x) { return sqrtf(x); }
 template <typename T> __device__ __forceinline__ T tmax(T a, T b) { return (a < b) ? b : a; }  // std::max
 
+// a / b, correctly rounded, from r = RN(1/b): two Newton corrections of the
+// quotient with an exact remainder (Markstein, IBM J. Res. Dev. 34, 1990: with
+// r correctly rounded and q within one ulp, RN(q + r (a - b q)) = RN(a / b)).
+// The first correction brings q = RN(a r) within one ulp, the second is the
+// theorem's step.  Exact while a remainder stays normal: quotient_rcp gives 0,
+// and quotient 0, for a denominator beyond 1e+-290.
+__device__ __forceinline__ double quotient(double a, double b, double r) {
+  double q = a * r;
+  q = __fma_rn(__fma_rn(-b, q, a), r, q);
+  return __fma_rn(__fma_rn(-b, q, a), r, q);
+}
+__device__ __forceinline__ double quotient_rcp(double b) {
+  return (b > 1.0e-290 && b < 1.0e290) ? __drcp_rn(b) : 0.0;
+}
+
 // ---------------------------------------------------------------------------
 // Roe flux with Harten entropy fix: flux_Roe + calc_physical_flux
 // (src/solver/InviscidFluxComputer.cpp:14-131).  q = (rho,u,v,w,p).
 // ---------------------------------------------------------------------------
+// Quotients by one denominator: FP64 rounded as the division (quotient), FP32
+// the product with the reciprocal.
+template <typename T> struct Over {
+  T b, r;
+};
+__device__ __forceinline__ Over<double> over(double b) { return Over<double>{b, __drcp_rn(b)}; }
+__device__ __forceinline__ Over<float> over(float b) { return Over<float>{b, __fdividef(1.f, b)}; }
+__device__ __forceinline__ double div(double a, const Over<double>& o) { return quotient(a, o.b, o.r); }
+__device__ __forceinline__ float div(float a, const Over<float>& o) { return a * o.r; }
+
 template <typename T>
-__device__ __forceinline__ void physical_flux(const T q[5], T gamma, T nx, T ny, T nz, T nt, T f[5]) {
+__device__ __forceinline__ void physical_flux(const T q[5], const Over<T>& rg1, const Over<T>& rrho, T nx, T ny, T nz,
+                                              T nt, T f[5]) {
   const T rho = q[0], u = q[1], v = q[2], w = q[3], p = q[4];
   const T V = u * nx + v * ny + w * nz + nt;
-  const T E = p / (gamma - T(1)) + T(0.5) * rho * (u * u + v * v + w * w);
-  const T H = (E + p) / rho;
+  const T E = div(p, rg1) + T(0.5) * rho * (u * u + v * v + w * w);
+  const T H = div(E + p, rrho);
   f[0] = rho * V;
   f[1] = rho * u * V + p * nx;
   f[2] = rho * v * V + p * ny;
@@ -40,16 +66,17 @@ template <typename T>
 __device__ __forceinline__ void roe_flux(const T ql[5], const T qr[5], T nx, T ny, T nz, T nt, T efix, T gamma,
                                          T f[5]) {
   T fl[5], fr[5];
-  physical_flux(ql, gamma, nx, ny, nz, nt, fl);
-  physical_flux(qr, gamma, nx, ny, nz, nt, fr);
-  const T drho = qr[0] - ql[0], du = qr[1] - ql[1], dv = qr[2] - ql[2], dw = qr[3] - ql[3], dp = qr[4] - ql[4];
   const T gamma1 = gamma - T(1);
   const T gamma2 = gamma / gamma1;
-  const T hl = gamma2 * ql[4] / ql[0] + T(0.5) * (ql[1] * ql[1] + ql[2] * ql[2] + ql[3] * ql[3]);
-  const T hr = gamma2 * qr[4] / qr[0] + T(0.5) * (qr[1] * qr[1] + qr[2] * qr[2] + qr[3] * qr[3]);
+  const Over<T> rg1 = over(gamma1), rl = over(ql[0]), rr = over(qr[0]);
+  physical_flux(ql, rg1, rl, nx, ny, nz, nt, fl);
+  physical_flux(qr, rg1, rr, nx, ny, nz, nt, fr);
+  const T drho = qr[0] - ql[0], du = qr[1] - ql[1], dv = qr[2] - ql[2], dw = qr[3] - ql[3], dp = qr[4] - ql[4];
+  const T hl = div(gamma2 * ql[4], rl) + T(0.5) * (ql[1] * ql[1] + ql[2] * ql[2] + ql[3] * ql[3]);
+  const T hr = div(gamma2 * qr[4], rr) + T(0.5) * (qr[1] * qr[1] + qr[2] * qr[2] + qr[3] * qr[3]);
   const T sqrt_rL = tsqrt(ql[0]);
   const T sqrt_rR = tsqrt(qr[0]);
-  const T inv_den = T(1) / (sqrt_rL + sqrt_rR);
+  const T inv_den = over(sqrt_rL + sqrt_rR).r;
   const T rho_roe = sqrt_rL * sqrt_rR;
   const T u_roe = (sqrt_rL * ql[1] + sqrt_rR * qr[1]) * inv_den;
   const T v_roe = (sqrt_rL * ql[2] + sqrt_rR * qr[2]) * inv_den;
@@ -62,7 +89,7 @@ __device__ __forceinline__ void roe_flux(const T ql[5], const T qr[5], T nx, T n
   const T U_contra = u_roe * nx + v_roe * ny + w_roe * nz + nt;
   T grad_mag = tsqrt(nx * nx + ny * ny + nz * nz);
   grad_mag = tmax(grad_mag, T(1.0e-30));
-  const T inv_mag = T(1) / grad_mag;
+  const T inv_mag = over(grad_mag).r;
   const T nx_n = nx * inv_mag, ny_n = ny * inv_mag, nz_n = nz * inv_mag;
   const T c_mag = c * grad_mag;
   T l1 = tabs(U_contra - c_mag);
@@ -74,8 +101,8 @@ __device__ __forceinline__ void roe_flux(const T ql[5], const T qr[5], T nx, T n
   if (l4 < delta) l4 = tsqrt(l4 * l4 + delta2);
   if (l5 < delta) l5 = tsqrt(l5 * l5 + delta2);
   const T rodcta = rho_roe * (du * nx_n + dv * ny_n + dw * nz_n);
-  const T dp_c2 = dp / c2;
-  const T rodctac = rodcta / c;
+  const T dp_c2 = div(dp, over(c2));
+  const T rodctac = div(rodcta, over(c));
   const T a1 = l4 * (drho - dp_c2);
   const T a2 = l5 * (dp_c2 + rodctac) * T(0.5);
   const T a3 = l1 * (dp_c2 - rodctac) * T(0.5);
@@ -88,59 +115,12 @@ __device__ __forceinline__ void roe_flux(const T ql[5], const T qr[5], T nx, T n
   const T df1 = u_roe * a4 + nx_n * a5 + a6;
   const T df2 = v_roe * a4 + ny_n * a5 + a7;
   const T df3 = w_roe * a4 + nz_n * a5 + a8;
-  const T df4 = h_roe * a4 + U_contra * inv_mag * a5 + u_roe * a6 + v_roe * a7 + w_roe * a8 - c2 * a1 / gamma1;
+  const T df4 = h_roe * a4 + U_contra * inv_mag * a5 + u_roe * a6 + v_roe * a7 + w_roe * a8 - div(c2 * a1, rg1);
   f[0] = T(0.5) * (fl[0] + fr[0] - df0);
   f[1] = T(0.5) * (fl[1] + fr[1] - df1);
   f[2] = T(0.5) * (fl[2] + fr[2] - df2);
   f[3] = T(0.5) * (fl[3] + fr[3] - df3);
   f[4] = T(0.5) * (fl[4] + fr[4] - df4);
-}
-
-// ---------------------------------------------------------------------------
-// WCNS-E-5 left/right states at one face for one variable
-// (src/solver/InviscidFluxComputer.cpp:259-315).  s[0..5] are the six line
-// points q_line[i..i+5] around face i.
-// ---------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ T wcns_w(T g, T s, T C) {
-  const T EPS = T(1.0e-6);
-  const T IS = g * g + s * s;
-  return C / ((EPS + IS) * (EPS + IS));
-}
-
-template <typename T>
-__device__ __forceinline__ T wcns_left(T q_m2, T q_m1, T q_0, T q_p1, T q_p2) {
-  const T CL1 = T(1.0 / 16.0), CL2 = T(10.0 / 16.0), CL3 = T(5.0 / 16.0);
-  const T s1 = q_m2 - T(2) * q_m1 + q_0;
-  const T s2 = q_m1 - T(2) * q_0 + q_p1;
-  const T s3 = q_0 - T(2) * q_p1 + q_p2;
-  const T g1 = T(0.5) * (q_m2 - T(4) * q_m1 + T(3) * q_0);
-  const T g2 = T(0.5) * (q_p1 - q_m1);
-  const T g3 = T(0.5) * (T(-3) * q_0 + T(4) * q_p1 - q_p2);
-  const T wl1 = wcns_w(g1, s1, CL1);
-  const T wl2 = wcns_w(g2, s2, CL2);
-  const T wl3 = wcns_w(g3, s3, CL3);
-  const T sum = wl1 + wl2 + wl3;
-  return q_0 + T(0.125) * ((wl1 / sum) * (s1 + T(4) * g1) + (wl2 / sum) * (s2 + T(4) * g2) +
-                           (wl3 / sum) * (s3 + T(4) * g3));
-}
-
-template <typename T>
-__device__ __forceinline__ T wcns_right(T q_m1, T q_0, T q_p1, T q_p2, T q_p3) {
-  // sr1 = s2, sr2 = s3 of the left stencil; the right state is centred on q_p1.
-  const T CL1 = T(1.0 / 16.0), CL2 = T(10.0 / 16.0), CL3 = T(5.0 / 16.0);
-  const T sr1 = q_m1 - T(2) * q_0 + q_p1;
-  const T sr2 = q_0 - T(2) * q_p1 + q_p2;
-  const T sr3 = q_p1 - T(2) * q_p2 + q_p3;
-  const T gr1 = T(0.5) * (q_m1 - T(4) * q_0 + T(3) * q_p1);
-  const T gr2 = T(0.5) * (q_p2 - q_0);
-  const T gr3 = T(0.5) * (T(-3) * q_p1 + T(4) * q_p2 - q_p3);
-  const T wr1 = wcns_w(gr1, sr1, CL3);
-  const T wr2 = wcns_w(gr2, sr2, CL2);
-  const T wr3 = wcns_w(gr3, sr3, CL1);
-  const T sum = wr1 + wr2 + wr3;
-  return q_p1 + T(0.125) * ((wr1 / sum) * (sr1 - T(4) * gr1) + (wr2 / sum) * (sr2 - T(4) * gr2) +
-                            (wr3 / sum) * (sr3 - T(4) * gr3));
 }
 
 // 6th-order / boundary flux differences (FLUX_DXYZ,

@@ -16,6 +16,7 @@
 #include "output_dev.cuh"
 #include "shard_dev.cuh"
 #include "sweep_tiles.cuh"
+#include "inviscid.cuh"
 
 using namespace orion;
 
@@ -312,6 +313,32 @@ int build_line_tiles(orion_case_t c) {
   return 0;
 }
 
+// Inviscid kernels: InvShape's lines per CTA, each line in as few, even chunks
+// as its buffers hold.
+template <int D, typename T>
+int build_inv_chunks(orion_case_t c) {
+  using Z = InvShape<D, T>;
+  std::vector<LineChunk> v;
+  for (int b = 0; b < c->nblocks; ++b) {
+    const auto& h = c->hb[b];
+    const int len = D == 0 ? h.idim : (D == 1 ? h.jdim : h.kdim);
+    const int nlines = D == 0 ? h.jdim * h.kdim : (D == 1 ? h.idim * h.kdim : h.idim * h.jdim);
+    const int n = (len + Z::CM - 1) / Z::CM;
+    for (int s = 0; s < nlines; s += Z::NL)
+      for (int x = 0; x < n; ++x)
+        v.push_back(LineChunk{b, s, std::min(Z::NL, nlines - s), (int)((long long)x * len / n),
+                              (int)((long long)(x + 1) * len / n)});
+  }
+  c->L.n_inv_chunks[D] = (int)v.size();
+  return dev_upload(c, &c->L.inv_chunks[D], v, true);
+}
+template <typename T>
+int build_inv_chunks(orion_case_t c) {
+  int rc = build_inv_chunks<0, T>(c);
+  if (!rc) rc = build_inv_chunks<1, T>(c);
+  return rc ? rc : build_inv_chunks<2, T>(c);
+}
+
 // Tile wavefront sweeps: every block's tiles (tile_plan.hpp), per direction in
 // ticket order.  A tile's first point is `start` waves behind its block's
 // first, and the tiles it waits for start strictly earlier, so ordering by
@@ -401,6 +428,7 @@ int build_lists(orion_case_t c, const std::vector<long long>& prim_off, const Ex
   // line-kernel tiles: 16 grid lines per CTA in FP32, 32 in FP64 (autotuned defaults)
   L.lanes_cap = c->prec == ORION_PREC_FP64 ? 32 : 16;
   if ((rc = build_line_tiles(c))) return rc;
+  if ((rc = c->prec == ORION_PREC_FP64 ? build_inv_chunks<double>(c) : build_inv_chunks<float>(c))) return rc;
 
   // wavefront launches: launch t of the forward sweeps covers hyperplane t of
   // every block, launch t of the backward sweeps hyperplane nplanes-1-t.
@@ -1781,6 +1809,7 @@ int build_group(orion_group_t g, orion_case_t px) {
   std::vector<GroupMember> gm(nm);
   std::vector<Chunk> pad, itr;
   std::vector<LineTile> tl[3];
+  std::vector<LineChunk> ic[3];
   std::vector<RegionDev> regs;
   std::vector<std::vector<int>> phases;
   std::vector<int> pk_block, ap_block, ap_off{0}, ap_slot;
@@ -1814,6 +1843,9 @@ int build_group(orion_group_t g, orion_case_t px) {
       std::vector<LineTile> t;
       if ((rc = download(c, t, M.tiles[d], M.n_tiles[d]))) return rc;
       for (auto x : t) { x.block += bo; tl[d].push_back(x); }
+      std::vector<LineChunk> q;
+      if ((rc = download(c, q, M.inv_chunks[d], M.n_inv_chunks[d]))) return rc;
+      for (auto x : q) { x.block += bo; ic[d].push_back(x); }
       L.lanes[d] = std::max(L.lanes[d], M.lanes[d]);
       L.lmax[d] = std::max(L.lmax[d], M.lmax[d]);
       L.line_units[d] = std::max(L.line_units[d], M.line_units[d]);
@@ -1894,6 +1926,8 @@ int build_group(orion_group_t g, orion_case_t px) {
   for (int d = 0; d < 3; ++d) {
     if ((rc = dev_upload(px, &L.tiles[d], tl[d]))) return rc;
     L.n_tiles[d] = (int)tl[d].size();
+    if ((rc = dev_upload(px, &L.inv_chunks[d], ic[d]))) return rc;
+    L.n_inv_chunks[d] = (int)ic[d].size();
   }
   GroupRun& G = g->run;
   {

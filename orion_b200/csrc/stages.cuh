@@ -6,6 +6,7 @@
 
 #include "case.hpp"
 #include "kernels.cuh"
+#include "inviscid.cuh"
 #include "sweep_tiles.cuh"
 
 namespace orion {
@@ -37,9 +38,9 @@ struct Stages {
     CUDA_TRY(cudaFuncSetAttribute(k_viscous<0, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
     CUDA_TRY(cudaFuncSetAttribute(k_viscous<1, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
     CUDA_TRY(cudaFuncSetAttribute(k_viscous<2, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-    CUDA_TRY(cudaFuncSetAttribute(k_inviscid<0, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-    CUDA_TRY(cudaFuncSetAttribute(k_inviscid<1, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-    CUDA_TRY(cudaFuncSetAttribute(k_inviscid<2, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    CUDA_TRY(cudaFuncSetAttribute(k_inviscid<0, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)InvShape<0, T>::smem));
+    CUDA_TRY(cudaFuncSetAttribute(k_inviscid<1, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)InvShape<1, T>::smem));
+    CUDA_TRY(cudaFuncSetAttribute(k_inviscid<2, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)InvShape<2, T>::smem));
     return 0;
   }
 
@@ -117,14 +118,7 @@ struct Stages {
   template <int D>
   static void inv_dir(orion_case_t c) {
     auto& L = c->L;
-    const size_t smem = (size_t)L.line_units[D] * 5 * sizeof(T);
-    k_inviscid<D, S, T><<<L.n_tiles[D], kThreads, smem, c->stream>>>(blocks(c), L.tiles[D]);
-    {
-      // six outputs per line of the tile, whole warps: a CTA of 256 threads
-      // would leave most of its registers idle (about 128 per thread)
-      const int nt = std::min(kThreads, (6 * std::max(L.lanes[D], 1) + 31) / 32 * 32);
-      k_inv_cascade<D, S, T><<<L.n_tiles[D], nt, 0, c->stream>>>(blocks(c), L.tiles[D]);
-    }
+    k_inviscid<D, S, T><<<L.n_inv_chunks[D], InvShape<D, T>::NT, InvShape<D, T>::smem, c->stream>>>(blocks(c), L.inv_chunks[D]);
   }
 
   static int inviscid(orion_case_t c) {

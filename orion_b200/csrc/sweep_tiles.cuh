@@ -163,14 +163,6 @@ __device__ __forceinline__ bool edge_full(const U b[5]) {
   return b[0] != e && b[1] != e && b[2] != e && b[3] != e && b[4] != e;
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned int s = (unsigned int)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
 // mbarrier of one ring wave: one arrival (the copying warp's, with the wave's
 // byte count), completed by the bulk copies.
 __device__ __forceinline__ void mbar_init(unsigned long long* m) {
@@ -295,21 +287,6 @@ struct TilePoint<float, MODE> {
     reinterpret_cast<float*>(p + cs)[3] = v[4];
   }
 };
-
-// a / b, correctly rounded, from r = RN(1/b): two Newton corrections of the
-// quotient with an exact remainder (Markstein, IBM J. Res. Dev. 34, 1990: with
-// r correctly rounded and q within one ulp, RN(q + r (a - b q)) = RN(a / b)).
-// The first correction brings q = RN(a r) within one ulp, the second is the
-// theorem's step.  Exact while a remainder stays normal: quotient_rcp gives 0,
-// and quotient 0, for a denominator beyond 1e+-290.
-__device__ __forceinline__ double quotient(double a, double b, double r) {
-  double q = a * r;
-  q = __fma_rn(__fma_rn(-b, q, a), r, q);
-  return __fma_rn(__fma_rn(-b, q, a), r, q);
-}
-__device__ __forceinline__ double quotient_rcp(double b) {
-  return (b > 1.0e-290 && b < 1.0e290) ? __drcp_rn(b) : 0.0;
-}
 
 // FP64 (plain path): the reference's operations in the reference's order; the
 // two divisions of the pair's coefficients share the reciprocals prepared once

@@ -112,8 +112,9 @@ typedef struct orion_case_s* orion_case_t;
 typedef struct orion_group_s* orion_group_t;
 
 /* A step schedule: sweep form, cluster size (CLUSTER form: 8 or 16; 0 = the
- * largest co-resident) and the grid lines per CTA of the viscous and inviscid
- * line kernels (1-32).  ms_per_step is filled by orion_case_autotune. */
+ * largest co-resident) and lanes (1-32), kept and given back but without
+ * effect: the line kernels choose their own lines per CTA.  ms_per_step is
+ * filled by orion_case_autotune. */
 typedef struct {
   int sweep_form;
   int cluster_size;
@@ -215,10 +216,9 @@ int orion_last_residual(orion_case_t c, orion_residual_t* out);
  * sweep form either (the same operations in the same order). */
 int orion_case_set_schedule(orion_case_t c, const orion_schedule_t* s);
 int orion_case_get_schedule(orion_case_t c, orion_schedule_t* s);
-/* Autotuner: times candidate schedules on this case (line lanes 8/16/32 with
- * the current sweep form, then every sweep form the device supports with the
- * best lanes), steps_per_trial timed steps each after one warm-up step, and
- * applies the fastest.  The state (prim, the step counter) is saved before and
+/* Autotuner: times candidate schedules on this case (the current one, then
+ * every other sweep form the device supports), steps_per_trial timed steps each
+ * after one warm-up step, and applies the fastest.  The state (prim, the step counter) is saved before and
  * restored after every trial, so tuning leaves the solution where it was; the
  * next whole step recomputes every derived field.  Fills trials[0..*ntrials)
  * (cap entries at most) and *best.  Waits; no steps may be pending. */

@@ -42,7 +42,7 @@ constexpr int kHistCap = 4096;      // residual history ring
 #define ORION_SWEEP_THREADS 128
 #endif
 constexpr int kSweepThreads = ORION_SWEEP_THREADS;
-constexpr size_t kLineSmemBudget = 96 * 1024;
+constexpr size_t kLineBudget = 96 * 1024;  // five face values of the longest grid line a case may have
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -59,14 +59,9 @@ struct DeviceLists {
   int n_pad_chunks = 0;
   Chunk* int_chunks = nullptr;
   int n_int_chunks = 0;
-  LineTile* tiles[3] = {nullptr, nullptr, nullptr};
-  int n_tiles[3] = {0, 0, 0};
-  int lanes[3] = {1, 1, 1};
-  int lanes_cap = 32;                            // line tiles: at most this many grid lines per CTA (set at creation)
-  int lmax[3] = {0, 0, 0};
-  LineChunk* inv_chunks[3] = {nullptr, nullptr, nullptr};  // inviscid kernels' chunks of lines
-  int n_inv_chunks[3] = {0, 0, 0};
-  int line_units[3] = {0, 0, 0};                 // line tiles' face slots (lanes x (longest line + 1)) of shared memory
+  LineChunk* line_chunks[3] = {nullptr, nullptr, nullptr};  // work of the viscous and inviscid kernels
+  int n_line_chunks[3] = {0, 0, 0};
+  int lanes_cap = 32;                            // the schedule's lanes, kept for its readers
   Chunk* sweep_chunks[2] = {nullptr, nullptr};  // forward / backward hyperplane launches
   std::vector<int> sweep_off[2];                 // host: chunk range of each launch
   int* sweep_off_dev[2] = {nullptr, nullptr};    // device copies of sweep_off

@@ -88,15 +88,8 @@ struct Chunk {
   long long start;
 };
 
-// A tile of whole grid lines of one block along one direction.
-struct LineTile {
-  int block;
-  int first;  // first line id (lines enumerate the two transverse interior coordinates)
-  int count;  // lines in the tile
-  int pad;
-};
-
-// Points [c0, c1) of `count` lines from line `first` (inviscid.cuh).
+// Points [c0, c1) of `count` grid lines of one block along one direction from
+// line `first` (lines enumerate the two transverse interior coordinates).
 struct LineChunk {
   int block, first, count, c0, c1;
 };

@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(256, LineMinBlocks<T>::inv) k_inviscid(const B
         T acc = T(kRounds[e0].coef) * b[0];
         for (int e = 1; e < n; ++e) acc = acc + T(kRounds[e0 + e].coef) * b[e * 5 * NL];
         if (rh && !rl) acc = -acc;
-        dq[m * np] = (S)((T)old[o][m] + acc / T(24.0));
+        dq[m * np] = (S)((T)old[o][m] + div24(acc));
       }
       continue;
     }

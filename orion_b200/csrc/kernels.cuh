@@ -579,8 +579,8 @@ __global__ void k_node_derivs(const BlockDev<S>* __restrict__ blocks, const Chun
       const long long st = stride_along(B, d);
       const long long o = idx - (long long)(tt[d] + NG) * st;  // along-line coordinate 0
       const int L = dim_along(B, d);
-      const bool fl = B.prim[o] < 0.0;
-      const bool fr = B.prim[o + (long long)(L + 5) * st] < 0.0;
+      const bool fl = tt[d] <= 1 && B.prim[o] < 0.0;  // the one-sided formulas' points only
+      const bool fr = tt[d] >= L - 2 && B.prim[o + (long long)(L + 5) * st] < 0.0;
       const int comp[4] = {1, 2, 3, 5};
       for (int m = 0; m < 4; ++m) {
         const T v = node_deriv<T>(FluxSrc<S>::prim(B) + comp[m] * np, o, st, tt[d], L, fl, fr);
@@ -590,128 +590,18 @@ __global__ void k_node_derivs(const BlockDev<S>* __restrict__ blocks, const Chun
   }
 }
 
-// ===========================================================================
-// Viscous RHS along one direction D (compute_viscous_flux_block,
-// src/solver/FluxComputer.cpp:466-722, with interp_line_to_half :129-178,
-// compute_half_deriv_line :72-124, transform_derivs_to_phys :183-205,
-// compute_viscous_flux_1d :210-252, compute_flux_diff_1d :257-296).
-// One CTA per tile of whole lines: face fluxes to shared memory, then the
-// 6th-order difference and dq -= dfv / Re.
-// ===========================================================================
-template <typename T, typename A>
-__device__ __forceinline__ T interp_half(const A* __restrict__ a, long long o, long long st, int f, int L,
-                                         bool fl, bool fr) {
-  // interp_line_to_half at face f of a line of L points; a + o is memory coordinate 0.
-  auto Q = [&](int p) -> T { return (T)a[o + (long long)p * st]; };
-  if (fl && f == 0) return (T(35) * Q(3) + T(-35) * Q(4) + T(21) * Q(5) + T(-5) * Q(6)) / T(16);
-  if (fl && f == 1) return (T(5) * Q(3) + T(15) * Q(4) + T(-5) * Q(5) + T(1) * Q(6)) / T(16);
-  if (fr && f == L) return (T(35) * Q(L + 2) + T(-35) * Q(L + 1) + T(21) * Q(L) + T(-5) * Q(L - 1)) / T(16);
-  if (fr && f == L - 1) return (T(5) * Q(L + 2) + T(15) * Q(L + 1) + T(-5) * Q(L) + T(1) * Q(L - 1)) / T(16);
-  return (T(9) * (Q(f + 2) + Q(f + 3)) + T(-1) * (Q(f + 4) + Q(f + 1))) / T(16);
-}
-
-template <typename T, typename S>
-__device__ __forceinline__ T interp_half_s(const S* __restrict__ a, long long o, long long st, int f) {
-  auto Q = [&](int p) -> T { return (T)a[o + (long long)p * st]; };
-  return (T(9) * (Q(f + 2) + Q(f + 3)) + T(-1) * (Q(f + 4) + Q(f + 1))) / T(16);
-}
-
-template <typename T, typename A>
-__device__ __forceinline__ T half_deriv(const A* __restrict__ a, long long o, long long st, int f, int L, bool fl,
-                                        bool fr) {
-  auto Q = [&](int p) -> T { return (T)a[o + (long long)p * st]; };
-  if (fl && f == 0) return (T(-71) * Q(3) + T(141) * Q(4) + T(-93) * Q(5) + T(23) * Q(6)) / T(24);
-  if (fl && f == 1) return (T(-22) * Q(3) + T(17) * Q(4) + T(9) * Q(5) + T(-5) * Q(6) + T(1) * Q(7)) / T(24);
-  if (fr && f == L) return -(T(-71) * Q(L + 2) + T(141) * Q(L + 1) + T(-93) * Q(L) + T(23) * Q(L - 1)) / T(24);
-  if (fr && f == L - 1)
-    return -(T(-22) * Q(L + 2) + T(17) * Q(L + 1) + T(9) * Q(L) + T(-5) * Q(L - 1) + T(1) * Q(L - 2)) / T(24);
-  return (T(27) * (Q(f + 3) - Q(f + 2)) + T(-1) * (Q(f + 4) - Q(f + 1))) / T(24);
-}
-
-// cross derivative interpolated to face f with the source index clamped to the interior
-template <typename T, typename S>
-__device__ __forceinline__ T cross_half(const S* __restrict__ a, long long o, long long st, int f, int L) {
-  auto Q = [&](int p) -> T {
-    const int pc = p < NG ? NG : (p > L + NG - 1 ? L + NG - 1 : p);
-    return (T)a[o + (long long)pc * st];
-  };
-  return (T(9) * (Q(f + 2) + Q(f + 3)) + T(-1) * (Q(f + 4) + Q(f + 1))) / T(16);
-}
-
-template <int D, typename S, typename T>
-__device__ __forceinline__ void viscous_face(const BlockDev<S>& B, const ParamsDev& P, long long o, int f, int L,
-                                             bool fl, bool fr, T cp_prl, T fv[4]) {
-  const long long np = B.npad;
-  const long long st = stride_along(B, D);
-  const auto* prim = FluxSrc<S>::prim(B);
-  T uvwt[4];
-  const int comp[4] = {1, 2, 3, 5};
-  for (int m = 0; m < 4; ++m) uvwt[m] = interp_half<T>(prim + comp[m] * np, o, st, f, L, fl, fr);
-  const T vs = interp_half_s<T, S>(B.mu, o, st, f);
-  const T kcp = vs * cp_prl;
-  const T volh = interp_half_s<T, S>(FluxSrc<S>::vol(B), o, st, f);
-  T kxyz[9];
-  const auto* met = FluxSrc<S>::metrics(B);
-  for (int m = 0; m < 9; ++m) kxyz[m] = interp_half_s<T, S>(met + m * np, o, st, f);
-  T d[12];
-  // derivative along the line (half point), cross derivatives interpolated
-  for (int m = 0; m < 4; ++m) d[m + 4 * D] = half_deriv<T>(prim + comp[m] * np, o, st, f, L, fl, fr);
-#pragma unroll
-  for (int dd = 0; dd < 3; ++dd) {
-    if (dd == D) continue;
-    for (int m = 0; m < 4; ++m) d[m + 4 * dd] = cross_half<T, S>(B.duvwt + (m + 4 * dd) * np, o, st, f, L);
-  }
-  // transform_derivs_to_phys
-  const T vol_inv = T(1) / volh;
-  T g[12];
-  for (int m = 0; m < 3; ++m) {
-    const T k1 = kxyz[m], k2 = kxyz[m + 3], k3 = kxyz[m + 6];
-    for (int v = 0; v < 4; ++v) g[v * 3 + m] = (k1 * d[v] + k2 * d[v + 4] + k3 * d[v + 8]) * vol_inv;
-  }
-  // compute_viscous_flux_1d
-  const T CC = T(2.0 / 3.0);
-  const T vscc = vs * CC;
-  const T dudx = g[0], dudy = g[1], dudz = g[2];
-  const T dvdx = g[3], dvdy = g[4], dvdz = g[5];
-  const T dwdx = g[6], dwdy = g[7], dwdz = g[8];
-  const T txx = vscc * (T(2) * dudx - dvdy - dwdz);
-  const T tyy = vscc * (T(2) * dvdy - dwdz - dudx);
-  const T tzz = vscc * (T(2) * dwdz - dudx - dvdy);
-  const T txy = vs * (dudy + dvdx);
-  const T txz = vs * (dudz + dwdx);
-  const T tyz = vs * (dvdz + dwdy);
-  const T nx = kxyz[3 * D + 0], ny = kxyz[3 * D + 1], nz = kxyz[3 * D + 2];
-  fv[0] = txx * nx + txy * ny + txz * nz;
-  fv[1] = txy * nx + tyy * ny + tyz * nz;
-  fv[2] = txz * nx + tyz * ny + tzz * nz;
-  const T work = uvwt[0] * fv[0] + uvwt[1] * fv[1] + uvwt[2] * fv[2];
-  const T heat = kcp * (g[9] * nx + g[10] * ny + g[11] * nz);
-  fv[3] = work + heat;
-}
-
-template <int D>
-__device__ __forceinline__ void tile_item(int it, int nlanes, int nfaces, int& lane, int& pos) {
-  if (D == 0) {
-    lane = it / nfaces;
-    pos = it - lane * nfaces;
-  } else {
-    pos = it / nlanes;
-    lane = it - pos * nlanes;
-  }
-}
-
 // CTAs per SM the line kernels are compiled for (register cap 65536/(256*n)),
-// per compute precision, measured on C3: viscous FP32 five (3.91 ms against
-// 4.03 at six and 4.09 at four), FP64 three; inviscid FP32 four, FP64 three
-// (inviscid.cuh).
+// per compute precision, measured on 385x257x129 in 64 blocks, the three
+// directions: viscous FP32 four (2.49 ms; five 2.59), FP64 two (4.50 ms without
+// spills; three 5.70); inviscid FP32 four, FP64 three (inviscid.cuh).
 #ifndef ORION_VISC_MINB_F32
-#define ORION_VISC_MINB_F32 5
+#define ORION_VISC_MINB_F32 4
 #endif
 #ifndef ORION_INV_MINB_F32
 #define ORION_INV_MINB_F32 4
 #endif
 #ifndef ORION_VISC_MINB_F64
-#define ORION_VISC_MINB_F64 3
+#define ORION_VISC_MINB_F64 2
 #endif
 #ifndef ORION_INV_MINB_F64
 #define ORION_INV_MINB_F64 3
@@ -719,50 +609,6 @@ __device__ __forceinline__ void tile_item(int it, int nlanes, int nfaces, int& l
 template <typename T> struct LineMinBlocks;
 template <> struct LineMinBlocks<float> { static constexpr int visc = ORION_VISC_MINB_F32, inv = ORION_INV_MINB_F32; };
 template <> struct LineMinBlocks<double> { static constexpr int visc = ORION_VISC_MINB_F64, inv = ORION_INV_MINB_F64; };
-
-template <int D, typename S, typename T>
-__global__ void __launch_bounds__(256, LineMinBlocks<T>::visc) k_viscous(const BlockDev<S>* __restrict__ blocks, const LineTile* __restrict__ tiles) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* fsh = reinterpret_cast<T*>(smem_raw);
-  const LineTile tl = tiles[blockIdx.x];
-  const BlockDev<S> B = blocks[tl.block];
-  const ParamsDev& P = B.prm;
-  const int L = dim_along(B, D);
-  const int nf = L + 1;
-  const long long st = stride_along(B, D);
-  const T cp = T(1) / ((T(P.gamma) - T(1)) * T(P.moo) * T(P.moo));
-  const T cp_prl = cp / T(P.prl);
-  const T re_inv = (fabs(P.reynolds) > 1.0e-30) ? T(1) / T(P.reynolds) : T(0);
-  const int nitems = tl.count * nf;
-  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    int lane, f;
-    tile_item<D>(it, tl.count, nf, lane, f);
-    const long long o = line_origin(B, D, tl.first + lane);
-    const bool fl = B.prim[o] < 0.0;
-    const bool fr = B.prim[o + (long long)(L + 5) * st] < 0.0;
-    T fv[4];
-    viscous_face<D, S, T>(B, P, o, f, L, fl, fr, cp_prl, fv);
-    T* dst = fsh + ((size_t)lane * nf + f) * 4;
-    dst[0] = fv[0];
-    dst[1] = fv[1];
-    dst[2] = fv[2];
-    dst[3] = fv[3];
-  }
-  __syncthreads();
-  const int npts = tl.count * L;
-  for (int it = threadIdx.x; it < npts; it += blockDim.x) {
-    int lane, t;
-    tile_item<D>(it, tl.count, L, lane, t);
-    const long long o = line_origin(B, D, tl.first + lane);
-    const long long idx = o + (long long)(t + NG) * st;
-    const T* fb = fsh + (size_t)lane * nf * 4;
-    for (int m = 0; m < 4; ++m) {
-      const T dfv = flux_diff<T>(fb + m, 4, t, L);
-      S* q = B.dq + (m + 1) * B.npad + idx;
-      *q = (S)((T)*q - re_inv * dfv);
-    }
-  }
-}
 
 // ===========================================================================
 // Interface residual averaging (HaloExchanger::average_interface_residuals,

@@ -123,28 +123,28 @@ __device__ __forceinline__ void roe_flux(const T ql[5], const T qr[5], T nx, T n
   f[4] = T(0.5) * (fl[4] + fr[4] - df4);
 }
 
+// a / 24 and a / 1920, FP64 rounded as the divisions.
+__device__ __forceinline__ double div24(double a) { return quotient(a, 24.0, 1.0 / 24.0); }
+__device__ __forceinline__ float div24(float a) { return a * (1.f / 24.f); }
+__device__ __forceinline__ double div1920(double a) { return quotient(a, 1920.0, 1.0 / 1920.0); }
+__device__ __forceinline__ float div1920(float a) { return a * (1.f / 1920.f); }
+
 // 6th-order / boundary flux differences (FLUX_DXYZ,
 // src/solver/InviscidFluxComputer.cpp:197-233 and src/solver/FluxComputer.cpp:257-296,
-// identical formulas).  f points at face values with stride `st`; point t in [0,ni).
-// F(k) is face k's flux (faces 0..ni).
+// identical formulas) at point t in [0,ni); f(k) is face k's flux (faces 0..ni).
 template <typename T, typename F>
 __device__ __forceinline__ T flux_diff_at(F f, int t, int ni) {
   if (t >= 2 && t < ni - 2) {
     const T term1 = T(2250) * (f(t + 1) - f(t));
     const T term2 = T(-125) * (f(t + 2) - f(t - 1));
     const T term3 = T(9) * (f(t + 3) - f(t - 2));
-    return (term1 + term2 + term3) / T(1920);
+    return div1920(term1 + term2 + term3);
   }
-  if (t == 0) return (T(-23) * f(0) + T(21) * f(1) + T(3) * f(2) - f(3)) / T(24);
-  if (t == 1) return (f(0) - T(27) * f(1) + T(27) * f(2) - f(3)) / T(24);
-  if (t == ni - 1) return -(T(-23) * f(ni) + T(21) * f(ni - 1) + T(3) * f(ni - 2) - f(ni - 3)) / T(24);
+  if (t == 0) return div24(T(-23) * f(0) + T(21) * f(1) + T(3) * f(2) - f(3));
+  if (t == 1) return div24(f(0) - T(27) * f(1) + T(27) * f(2) - f(3));
+  if (t == ni - 1) return -div24(T(-23) * f(ni) + T(21) * f(ni - 1) + T(3) * f(ni - 2) - f(ni - 3));
   // t == ni - 2
-  return -(f(ni) - T(27) * f(ni - 1) + T(27) * f(ni - 2) - f(ni - 3)) / T(24);
-}
-
-template <typename T>
-__device__ __forceinline__ T flux_diff(const T* f, int st, int t, int ni) {
-  return flux_diff_at<T>([&](int k) -> T { return f[k * st]; }, t, ni);
+  return -div24(f(ni) - T(27) * f(ni - 1) + T(27) * f(ni - 2) - f(ni - 3));
 }
 
 // ---------------------------------------------------------------------------

@@ -285,38 +285,10 @@ namespace {
 // --------------------------------------------------------------------------
 // work-list builders
 // --------------------------------------------------------------------------
-// Line tiles per direction: up to L.lanes_cap grid lines per CTA, fewer where
-// the face fluxes of the longest line would not fit the shared-memory budget.
-int build_line_tiles(orion_case_t c) {
-  auto& L = c->L;
-  const int nb = c->nblocks;
-  const size_t tsz = (c->prec == ORION_PREC_FP64) ? 8 : 4;
-  int rc;
-  for (int d = 0; d < 3; ++d) {
-    int lmax = 0;
-    for (auto& h : c->hb) lmax = std::max(lmax, d == 0 ? h.idim : (d == 1 ? h.jdim : h.kdim));
-    L.lmax[d] = lmax;
-    int lanes = (int)std::min<size_t>((size_t)L.lanes_cap, kLineSmemBudget / ((size_t)(lmax + 1) * 5 * tsz));
-    if (lanes < 1) return fail(ORION_E_UNSUPPORTED, "grid line too long for the line kernels");
-    if (d > 0 && lanes >= 8) lanes = lanes / 8 * 8;
-    L.lanes[d] = lanes;
-    L.line_units[d] = lanes * (lmax + 1);
-    std::vector<LineTile> tiles;
-    for (int b = 0; b < nb; ++b) {
-      const auto& h = c->hb[b];
-      const int nlines = d == 0 ? h.jdim * h.kdim : (d == 1 ? h.idim * h.kdim : h.idim * h.jdim);
-      for (int s = 0; s < nlines; s += lanes) tiles.push_back(LineTile{b, s, std::min(lanes, nlines - s), 0});
-    }
-    if ((rc = dev_upload(c, &L.tiles[d], tiles, true))) return rc;
-    L.n_tiles[d] = (int)tiles.size();
-  }
-  return 0;
-}
-
-// Inviscid kernels: InvShape's lines per CTA, each line in as few, even chunks
-// as its buffers hold.
+// Viscous and inviscid kernels: InvShape's lines per CTA, each line in as few,
+// even chunks as the kernels' buffers hold.
 template <int D, typename T>
-int build_inv_chunks(orion_case_t c) {
+int build_line_chunks(orion_case_t c) {
   using Z = InvShape<D, T>;
   std::vector<LineChunk> v;
   for (int b = 0; b < c->nblocks; ++b) {
@@ -329,14 +301,14 @@ int build_inv_chunks(orion_case_t c) {
         v.push_back(LineChunk{b, s, std::min(Z::NL, nlines - s), (int)((long long)x * len / n),
                               (int)((long long)(x + 1) * len / n)});
   }
-  c->L.n_inv_chunks[D] = (int)v.size();
-  return dev_upload(c, &c->L.inv_chunks[D], v, true);
+  c->L.n_line_chunks[D] = (int)v.size();
+  return dev_upload(c, &c->L.line_chunks[D], v, true);
 }
 template <typename T>
-int build_inv_chunks(orion_case_t c) {
-  int rc = build_inv_chunks<0, T>(c);
-  if (!rc) rc = build_inv_chunks<1, T>(c);
-  return rc ? rc : build_inv_chunks<2, T>(c);
+int build_line_chunks(orion_case_t c) {
+  int rc = build_line_chunks<0, T>(c);
+  if (!rc) rc = build_line_chunks<1, T>(c);
+  return rc ? rc : build_line_chunks<2, T>(c);
 }
 
 // Tile wavefront sweeps: every block's tiles (tile_plan.hpp), per direction in
@@ -425,10 +397,11 @@ int build_lists(orion_case_t c, const std::vector<long long>& prim_off, const Ex
   L.n_int_chunks = (int)itr.size();
   if ((rc = dev_upload(c, &L.pad_base, c->shard.pad_base))) return rc;
 
-  // line-kernel tiles: 16 grid lines per CTA in FP32, 32 in FP64 (autotuned defaults)
   L.lanes_cap = c->prec == ORION_PREC_FP64 ? 32 : 16;
-  if ((rc = build_line_tiles(c))) return rc;
-  if ((rc = c->prec == ORION_PREC_FP64 ? build_inv_chunks<double>(c) : build_inv_chunks<float>(c))) return rc;
+  for (auto& h : c->hb)
+    if ((size_t)(std::max({h.idim, h.jdim, h.kdim}) + 1) * 5 * (c->prec == ORION_PREC_FP64 ? 8 : 4) > kLineBudget)
+      return fail(ORION_E_UNSUPPORTED, "grid line too long for the line kernels");
+  if ((rc = c->prec == ORION_PREC_FP64 ? build_line_chunks<double>(c) : build_line_chunks<float>(c))) return rc;
 
   // wavefront launches: launch t of the forward sweeps covers hyperplane t of
   // every block, launch t of the backward sweeps hyperplane nplanes-1-t.
@@ -1026,10 +999,7 @@ static int apply_schedule(orion_case_t c, const orion_schedule_t& s) {
     c->graph = nullptr;
   }
   int rc = 0;
-  if (s.lanes != c->L.lanes_cap) {
-    c->L.lanes_cap = s.lanes;
-    if ((rc = build_line_tiles(c))) return rc;
-  }
+  c->L.lanes_cap = s.lanes;
   rc = ops_for(c->prec).schedule(c, s.sweep_form, s.cluster_size);
   if (!rc && !c->group) rc = use_sweep_arrays(c, c->L.tiles_on);
   CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -1120,21 +1090,15 @@ int orion_case_autotune(orion_case_t c, int steps_per_trial, orion_schedule_t* t
   orion_schedule_t start;
   current_schedule(c, &start);
   best->ms_per_step = 0.f;
-  // phase 1: grid lines per CTA of the line kernels, with the current sweep form
-  for (int lanes : {8, 16, 32}) {
-    if (rc) break;
-    orion_schedule_t s = start;
-    s.lanes = lanes;
-    rc = trial(s);
-  }
-  // phase 2: every sweep form, with the best lanes
+  // the current schedule, then every other sweep form (the lanes change no kernel)
+  if (!rc) rc = trial(start);
   const orion_schedule_t forms[5] = {{ORION_SWEEP_TILES, 0, 0, 0.f}, {ORION_SWEEP_CLUSTER, 16, 0, 0.f},
                                      {ORION_SWEEP_CLUSTER, 8, 0, 0.f}, {ORION_SWEEP_GRID, 0, 0, 0.f},
                                      {ORION_SWEEP_PLANES, 0, 0, 0.f}};
   for (const auto& f : forms) {
     if (rc) break;
     if (f.sweep_form == start.sweep_form && (f.sweep_form != ORION_SWEEP_CLUSTER || f.cluster_size == start.cluster_size))
-      continue;  // timed in phase 1
+      continue;  // timed already
     orion_schedule_t s = f;
     s.lanes = best->lanes;
     const int r = trial(s);
@@ -1808,7 +1772,6 @@ int build_group(orion_group_t g, orion_case_t px) {
 
   std::vector<GroupMember> gm(nm);
   std::vector<Chunk> pad, itr;
-  std::vector<LineTile> tl[3];
   std::vector<LineChunk> ic[3];
   std::vector<RegionDev> regs;
   std::vector<std::vector<int>> phases;
@@ -1838,17 +1801,11 @@ int build_group(orion_group_t g, orion_case_t px) {
     gm[m].hist = M.hist;
     gm[m].counter = M.counter;
     gm[m].total = M.res_total;
-    // line tiles
+    // line kernels' chunks
     for (int d = 0; d < 3; ++d) {
-      std::vector<LineTile> t;
-      if ((rc = download(c, t, M.tiles[d], M.n_tiles[d]))) return rc;
-      for (auto x : t) { x.block += bo; tl[d].push_back(x); }
       std::vector<LineChunk> q;
-      if ((rc = download(c, q, M.inv_chunks[d], M.n_inv_chunks[d]))) return rc;
+      if ((rc = download(c, q, M.line_chunks[d], M.n_line_chunks[d]))) return rc;
       for (auto x : q) { x.block += bo; ic[d].push_back(x); }
-      L.lanes[d] = std::max(L.lanes[d], M.lanes[d]);
-      L.lmax[d] = std::max(L.lmax[d], M.lmax[d]);
-      L.line_units[d] = std::max(L.line_units[d], M.line_units[d]);
     }
     // halo copy: the member's own list, read in place
     gm[m].arena = static_cast<double*>(c->arena);
@@ -1924,10 +1881,8 @@ int build_group(orion_group_t g, orion_case_t px) {
   if ((rc = dev_upload(px, &L.int_chunks, itr))) return rc;
   L.n_int_chunks = (int)itr.size();
   for (int d = 0; d < 3; ++d) {
-    if ((rc = dev_upload(px, &L.tiles[d], tl[d]))) return rc;
-    L.n_tiles[d] = (int)tl[d].size();
-    if ((rc = dev_upload(px, &L.inv_chunks[d], ic[d]))) return rc;
-    L.n_inv_chunks[d] = (int)ic[d].size();
+    if ((rc = dev_upload(px, &L.line_chunks[d], ic[d]))) return rc;
+    L.n_line_chunks[d] = (int)ic[d].size();
   }
   GroupRun& G = g->run;
   {

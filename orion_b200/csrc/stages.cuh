@@ -7,6 +7,7 @@
 #include "case.hpp"
 #include "kernels.cuh"
 #include "inviscid.cuh"
+#include "viscous.cuh"
 #include "sweep_tiles.cuh"
 
 namespace orion {
@@ -18,8 +19,8 @@ template <typename S, typename T>
 struct Stages {
   static const BlockDev<S>* blocks(orion_case_t c) { return static_cast<const BlockDev<S>*>(c->d_blocks); }
 
-  // Line kernels take up to kLineSmemBudget of dynamic shared memory; the
-  // attribute is set once per process, before any stream capture.
+  // Dynamic shared memory above the default is set once per process, before
+  // any stream capture.
   static int set_attributes() {
     static std::once_flag once;
     static int rc = 0;
@@ -28,16 +29,15 @@ struct Stages {
   }
 
   static int set_line_attributes() {
-    const int b = (int)kLineSmemBudget;
     // the ring of a tile of kTileLines lines and its halo at most
     const int tb = (int)tile_smem_bytes<T>(kTileMaxLines);
     CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_LUSGS_FWD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb));
     CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_LUSGS_BWD, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb));
     CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_GS, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb));
     CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_GS, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb));
-    CUDA_TRY(cudaFuncSetAttribute(k_viscous<0, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-    CUDA_TRY(cudaFuncSetAttribute(k_viscous<1, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-    CUDA_TRY(cudaFuncSetAttribute(k_viscous<2, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    CUDA_TRY(cudaFuncSetAttribute(k_viscous<0, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscShape<0, T>::smem));
+    CUDA_TRY(cudaFuncSetAttribute(k_viscous<1, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscShape<1, T>::smem));
+    CUDA_TRY(cudaFuncSetAttribute(k_viscous<2, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscShape<2, T>::smem));
     CUDA_TRY(cudaFuncSetAttribute(k_inviscid<0, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)InvShape<0, T>::smem));
     CUDA_TRY(cudaFuncSetAttribute(k_inviscid<1, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)InvShape<1, T>::smem));
     CUDA_TRY(cudaFuncSetAttribute(k_inviscid<2, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)InvShape<2, T>::smem));
@@ -101,8 +101,9 @@ struct Stages {
   template <int D>
   static void visc_dir(orion_case_t c) {
     auto& L = c->L;
-    const size_t smem = (size_t)L.line_units[D] * 4 * sizeof(T);
-    k_viscous<D, S, T><<<L.n_tiles[D], kThreads, smem, c->stream>>>(blocks(c), L.tiles[D]);
+    using Z = ViscShape<D, T>;
+    static_assert(Z::NL == InvShape<D, T>::NL && Z::CM == InvShape<D, T>::CM, "one chunk list for both");
+    k_viscous<D, S, T><<<L.n_line_chunks[D], Z::NT, Z::smem, c->stream>>>(blocks(c), L.line_chunks[D]);
   }
 
   static int viscous(orion_case_t c) {
@@ -118,7 +119,7 @@ struct Stages {
   template <int D>
   static void inv_dir(orion_case_t c) {
     auto& L = c->L;
-    k_inviscid<D, S, T><<<L.n_inv_chunks[D], InvShape<D, T>::NT, InvShape<D, T>::smem, c->stream>>>(blocks(c), L.inv_chunks[D]);
+    k_inviscid<D, S, T><<<L.n_line_chunks[D], InvShape<D, T>::NT, InvShape<D, T>::smem, c->stream>>>(blocks(c), L.line_chunks[D]);
   }
 
   static int inviscid(orion_case_t c) {

@@ -83,6 +83,7 @@ struct DeviceLists {
   int n_sweep_tiles[2] = {0, 0};
   void* tile_ctl = nullptr;                      // TileCtl
   int tile_lines = 0;                            // lines of the largest tile
+  bool tile_small = false;                       // every tile has at most kTileLinesSmall
   int max_planes = 0;
   long long* halo_src = nullptr;
   long long* halo_dst = nullptr;

@@ -57,7 +57,7 @@ int dev_alloc(orion_case_t c, T** dptr, size_t n) {
 }
 
 // Bytes of one block's fields for storage size ssz.
-size_t block_bytes(const HostBlock& b, size_t ssz) {
+size_t block_bytes(const HostBlock& b, size_t ssz, int tile_lines) {
   const size_t np = (size_t)b.npad;
   size_t s = 0;
   auto add = [&](size_t bytes) { s = align_up(s, 256) + bytes; };
@@ -81,7 +81,7 @@ size_t block_bytes(const HostBlock& b, size_t ssz) {
   add((npl * b.kdim + 1) * 4);  // koff
   add(nc * 4);                  // sk_nat
   add(6 * nc * 4);              // sk_nb
-  const TilePlan p = make_tile_plan(b.idim, b.jdim, b.kdim, ssz);
+  const TilePlan p = make_tile_plan(b.idim, b.jdim, b.kdim, ssz, tile_lines);
   add(16 * (size_t)(b.jdim + b.kdim));  // t_j, t_k
   add(8 * p.base.size());               // t_base
   // one area for the form in use: sk_metrics 9, sk_vol, sk_prim 5, sk_mu, sk_coed, sk_rhs 5, sk_dq 5, sk_nrm 9,
@@ -91,7 +91,7 @@ size_t block_bytes(const HostBlock& b, size_t ssz) {
 }
 
 template <typename S>
-void carve_block(char* base, const HostBlock& b, BlockDev<S>& d) {
+void carve_block(char* base, const HostBlock& b, int tile_lines, BlockDev<S>& d) {
   const size_t np = (size_t)b.npad;
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -123,7 +123,7 @@ void carve_block(char* base, const HostBlock& b, BlockDev<S>& d) {
   d.koff = reinterpret_cast<int*>(take(((size_t)npl * b.kdim + 1) * 4));
   d.sk_nat = reinterpret_cast<int*>(take(nc * 4));
   d.sk_nb = reinterpret_cast<int*>(take(6 * nc * 4));
-  const TilePlan p = make_tile_plan(b.idim, b.jdim, b.kdim, sizeof(S));
+  const TilePlan p = make_tile_plan(b.idim, b.jdim, b.kdim, sizeof(S), tile_lines);
   const TileBytes tb = tile_bytes(sizeof(S));
   d.t_j = reinterpret_cast<int4*>(take(16 * (size_t)(b.jdim + b.kdim)));
   d.t_k = d.t_j + b.jdim;
@@ -322,7 +322,7 @@ int build_sweep_tiles(orion_case_t c) {
   L.tile_lines = 0;
   for (int b = 0; b < c->nblocks; ++b) {
     const auto& h = c->hb[b];
-    const TilePlan p = make_tile_plan(h.idim, h.jdim, h.kdim, ssz);
+    const TilePlan p = make_tile_plan(h.idim, h.jdim, h.kdim, ssz, tile_max_lines(ssz, L.tile_small));
     const int nJ = p.nJ(), nK = p.nK();
     for (int K = 0; K < nK; ++K)
       for (int J = 0; J < nJ; ++J) {
@@ -424,7 +424,7 @@ int build_lists(orion_case_t c, const std::vector<long long>& prim_off, const Ex
       void* dnb = b64 ? (void*)b64->sk_nb : (void*)b32->sk_nb;
       CUDA_TRY(cudaMemcpyAsync(dnb, nbv.data(), nbv.size() * 4, cudaMemcpyHostToDevice, c->stream));
       // natural order -> tile slots
-      const TilePlan p = make_tile_plan(h.idim, h.jdim, h.kdim, b64 ? 8 : 4);
+      const TilePlan p = make_tile_plan(h.idim, h.jdim, h.kdim, b64 ? 8 : 4, tile_max_lines(b64 ? 8 : 4, L.tile_small));
       std::vector<int4> tjk;
       for (int a = 0; a < p.nJ(); ++a)
         for (int x = 0; x < p.jw(a); ++x) tjk.push_back(make_int4(a, x, p.jw(a), 0));
@@ -805,11 +805,15 @@ static int create_case(int nglobal, const orion_block_desc_t* blocks, const int*
 
   // arena
   const size_t ssz = precision == ORION_PREC_FP64 ? 8 : 4;
+  long long lines = 0;
+  for (const auto& h : c->hb) lines += (long long)h.jdim * h.kdim;
+  c->L.tile_small = precision == ORION_PREC_FP64 && lines <= kTileSmallCase;
+  const int tile_lines = tile_max_lines(ssz, c->L.tile_small);
   std::vector<size_t> boff(nblocks);
   size_t total = 0;
   for (int b = 0; b < nblocks; ++b) {
     boff[b] = total;
-    total += block_bytes(c->hb[b], ssz);
+    total += block_bytes(c->hb[b], ssz, tile_lines);
   }
   if (cudaMallocAsync(&c->arena, total, c->stream) != cudaSuccess) {
     cudaGetLastError();
@@ -821,7 +825,7 @@ static int create_case(int nglobal, const orion_block_desc_t* blocks, const int*
   if (precision == ORION_PREC_FP64) {
     c->bd64.resize(nblocks);
     for (int b = 0; b < nblocks; ++b) {
-      carve_block(static_cast<char*>(c->arena) + boff[b], c->hb[b], c->bd64[b]);
+      carve_block(static_cast<char*>(c->arena) + boff[b], c->hb[b], tile_lines, c->bd64[b]);
       c->bd64[b].prm = c->P;  // every kernel reads its case's parameters from its block's descriptor
       c->bd64[b].int_base = gint[plan.local[b]];
       prim_off[b] = (c->bd64[b].prim - static_cast<double*>(c->arena));
@@ -832,7 +836,7 @@ static int create_case(int nglobal, const orion_block_desc_t* blocks, const int*
   } else {
     c->bd32.resize(nblocks);
     for (int b = 0; b < nblocks; ++b) {
-      carve_block(static_cast<char*>(c->arena) + boff[b], c->hb[b], c->bd32[b]);
+      carve_block(static_cast<char*>(c->arena) + boff[b], c->hb[b], tile_lines, c->bd32[b]);
       c->bd32[b].prm = c->P;  // every kernel reads its case's parameters from its block's descriptor
       c->bd32[b].int_base = gint[plan.local[b]];
       prim_off[b] = (c->bd32[b].prim - static_cast<double*>(c->arena));
@@ -889,6 +893,9 @@ size_t orion_footprint_estimate(int nblocks, const orion_block_desc_t* blocks, i
   if (nblocks <= 0 || !blocks) return 0;
   const size_t ssz = precision == ORION_PREC_FP64 ? 8 : 4;
   size_t s = 0;
+  long long lines = 0;
+  for (int b = 0; b < nblocks; ++b) lines += (long long)blocks[b].jdim * blocks[b].kdim;
+  const int tile_lines = tile_max_lines(ssz, lines <= kTileSmallCase);
   for (int b = 0; b < nblocks; ++b) {
     HostBlock h;
     h.idim = blocks[b].idim;
@@ -898,7 +905,7 @@ size_t orion_footprint_estimate(int nblocks, const orion_block_desc_t* blocks, i
     h.ny = h.jdim + 2 * NG;
     h.nz = h.kdim + 2 * NG;
     h.npad = (long long)h.nx * h.ny * h.nz;
-    s += block_bytes(h, ssz);
+    s += block_bytes(h, ssz, tile_lines);
   }
   return s + (s / 64);  // work lists and buffers are a small fraction
 }
@@ -1150,7 +1157,7 @@ int orion_case_sweep_schedule(orion_case_t c, int out[5]) {
   out[0] = L.tiles_on ? 3 : (L.cl_size > 0 ? 2 : (L.persist_grid > 0 ? 1 : 0));
   out[1] = L.tiles_on ? L.n_sweep_tiles[0] : (L.cl_size > 0 ? L.cl_count : L.persist_grid);
   out[2] = L.cl_size;
-  out[3] = L.tiles_on ? kTileThreads : L.sweep_nt;
+  out[3] = L.tiles_on ? tile_max_lines(c->prec == ORION_PREC_FP64 ? 8 : 4, L.tile_small) : L.sweep_nt;
   out[4] = L.max_planes;
   return 0;
 }
@@ -1874,6 +1881,7 @@ int build_group(orion_group_t g, orion_case_t px) {
     }
     max_planes = std::max(max_planes, M.max_planes);
     L.tile_lines = std::max(L.tile_lines, M.tile_lines);
+    L.tile_small = (m == 0 || L.tile_small) && M.tile_small;
   }
   // upload
   if ((rc = dev_upload(px, &L.pad_chunks, pad))) return rc;

@@ -28,13 +28,24 @@ struct Stages {
     return rc;
   }
 
+  // compute threads of the tile sweeps: one a line
+  static constexpr int tile_threads(bool small) { return (tile_max_lines(sizeof(T), small) + 31) / 32 * 32; }
+
+  template <bool SMALL>
+  static int tile_attributes() {
+    constexpr int TT = tile_threads(SMALL);
+    const int b = (int)tile_smem_bytes<T>(tile_max_lines(sizeof(T), SMALL));
+    CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_LUSGS_FWD, 1, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_LUSGS_BWD, -1, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_GS, 1, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_GS, -1, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+    return 0;
+  }
+
   static int set_line_attributes() {
-    // the ring of a tile of kTileLines lines and its halo at most
-    const int tb = (int)tile_smem_bytes<T>(kTileMaxLines);
-    CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_LUSGS_FWD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb));
-    CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_LUSGS_BWD, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb));
-    CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_GS, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb));
-    CUDA_TRY(cudaFuncSetAttribute(k_sweep_tiles<S, T, SW_GS, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb));
+    int rc = tile_attributes<true>();
+    if (!rc) rc = tile_attributes<false>();
+    if (rc) return rc;
     CUDA_TRY(cudaFuncSetAttribute(k_viscous<0, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscShape<0, T>::smem));
     CUDA_TRY(cudaFuncSetAttribute(k_viscous<1, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscShape<1, T>::smem));
     CUDA_TRY(cudaFuncSetAttribute(k_viscous<2, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscShape<2, T>::smem));
@@ -349,9 +360,13 @@ struct Stages {
     if (n <= 0) return 0;
     SweepCtl* sc = static_cast<SweepCtl*>(L.sweep_ctl);
     const size_t smem = tile_smem_bytes<T>(L.tile_lines);
-    k_sweep_tiles<S, T, MODE, DIR><<<n, kTileThreads + 64, smem, c->stream>>>(
-        blocks(c), static_cast<const SweepTile*>(L.sweep_tiles[d]), n, L.tile_lines,
-        static_cast<TileCtl*>(L.tile_ctl), &sc->error, L.spin_limit);
+    auto launch = [&](auto kernel, int tt) {
+      kernel<<<n, tt * (MODE == SW_GS && TileLayout<T>::split ? 2 : 1) + 64, smem, c->stream>>>(
+          blocks(c), static_cast<const SweepTile*>(L.sweep_tiles[d]), n, L.tile_lines,
+          static_cast<TileCtl*>(L.tile_ctl), &sc->error, L.spin_limit);
+    };
+    if (L.tile_small) launch(k_sweep_tiles<S, T, MODE, DIR, tile_threads(true)>, tile_threads(true));
+    else launch(k_sweep_tiles<S, T, MODE, DIR, tile_threads(false)>, tile_threads(false));
     return 0;
   }
 

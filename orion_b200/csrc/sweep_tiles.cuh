@@ -47,8 +47,6 @@
 
 namespace orion {
 
-constexpr int kTileThreads = (kTileMaxLines + 31) / 32 * 32;  // compute threads, one a line
-
 // 16-byte pieces per point of the tile layout (tl_own: met, dyn; tl_nb: nb), FP32 / FP64:
 //   met  {kx ky kz |k|} per direction                     / {kx ky}{kz |k|} per direction, {1/|k| x 2}{1/|k| -}
 //   dyn  {coed r0 r1 r2}{r3 r4 - -}                       / {coed r0}{r1 r2}{r3 r4}
@@ -58,9 +56,7 @@ constexpr int kTileThreads = (kTileMaxLines + 31) / 32 * 32;  // compute threads
 // t+1 (ahead) are in use and waves up to t + ring - 2 on their way; own
 // operands (met, dyn) of waves t to t + ring - 2.  FP32: six waves and two CTAs
 // an SM (193x97x65, 8 blocks: 1.93 ms a step, five waves 1.98; eight waves and
-// one CTA an SM the same, and 4% slower on 385x257x129).  FP64: one CTA an SM,
-// so that the six terms of a point overlap in registers (183 to 196; at two CTAs
-// and 168 registers a pass of 97x49x33 took 0.73 ms in place of 0.40).
+// one CTA an SM the same, and 4% slower on 385x257x129).
 #ifndef ORION_TILE_RING_F32
 #define ORION_TILE_RING_F32 6
 #endif
@@ -70,10 +66,19 @@ constexpr int kTileThreads = (kTileMaxLines + 31) / 32 * 32;  // compute threads
 template <typename T> struct TileLayout;
 template <> struct TileLayout<float> {
   static constexpr int met = 3, dyn = 2, nb = 3, own = met + dyn, rec = 8, minb = 2, ring = ORION_TILE_RING_F32;
+  static constexpr bool split = false;
 };
+// split: on the GS passes a second set of compute warps forms the terms of the
+// ahead neighbours one step early (they are known before the pass), so a step's
+// chain is three terms long in place of six and the FP64 pipe has twice the
+// warps.
 template <> struct TileLayout<double> {
   static constexpr int met = 8, dyn = 3, nb = 8, own = met + dyn, rec = 8, minb = 1, ring = ORION_TILE_RING_F64;
+  static constexpr bool split = true;
 };
+// Values a point's ahead terms are handed over in: the three terms one by one
+// where they are subtracted after the behind ones (forward), else their sum.
+constexpr int kTileAheadValues = 15;
 
 // One tile, in ticket order of one direction.
 struct SweepTile {
@@ -97,13 +102,14 @@ struct TileCtl {
 
 // Dynamic shared memory of tiles of `lines` lines at most: the ring (per wave
 // [piece][line], then [piece][32 behind and 32 ahead halo lines]), the fresh
-// increments of two waves ([piece][line, halo line]) and the own operands
-// ([piece][line]).
+// increments of two waves ([piece][line, halo line]), the own operands
+// ([piece][line]) and the ahead terms of two waves ([value][line]).
 template <typename T>
 constexpr size_t tile_smem_bytes(int lines) {
   using L = TileLayout<T>;
   return (size_t)(L::ring * L::nb + 2 * ((5 * sizeof(T) + 15) / 16)) * 16 * (size_t)(lines + 64) +
-         (size_t)(L::ring - 1) * L::own * 16 * (size_t)lines;
+         (size_t)(L::ring - 1) * L::own * 16 * (size_t)lines +
+         (L::split ? (size_t)2 * kTileAheadValues * sizeof(T) * (size_t)lines : 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -385,22 +391,26 @@ struct TilePoint<double, MODE> {
 };
 
 // MODE: SW_LUSGS_FWD (lower neighbours), SW_LUSGS_BWD (upper), SW_GS with DIR
-// +1 / -1 (all six).  Warps: kTileThreads compute threads, one warp for the
-// behind halo lines, and one that starts the bulk copies and, on the GS passes,
-// brings the ahead halo lines.
+// +1 / -1 (all six).  Warps: TT compute threads, one a line (split GS passes: TT
+// more for the ahead terms), one warp for the behind halo lines, and one that
+// starts the bulk copies and, on the GS passes, brings the ahead halo lines.
 //
 // Step t handles wave t (forward) or W-1-t.  At its start wave t + FN is sent
 // for; the compute threads wait for wave t+1, update wave t from ring waves
 // t-1 and t+1 and the fresh increments of t-1; the behind warp delivers its
 // lines' fresh increments of wave t (read at t+1).
-template <typename S, typename T, int MODE, int DIR>
-__global__ void __launch_bounds__(kTileThreads + 64, TileLayout<T>::minb)
+template <typename S, typename T, int MODE, int DIR, int TT>
+__global__ void __launch_bounds__(TT * (MODE == SW_GS && TileLayout<T>::split ? 2 : 1) + 64, TileLayout<T>::minb)
     k_sweep_tiles(const BlockDev<S>* __restrict__ blocks, const SweepTile* __restrict__ tiles, int ntiles, int lines,
                   TileCtl* __restrict__ ctl, int* __restrict__ err, long long spin_limit) {
   static_assert(sizeof(S) == sizeof(T), "the tile sweeps keep operands in their storage precision");
   using L = TileLayout<T>;
   using U = typename EdgeBits<T>::type;
   constexpr int R = L::ring, NB = L::nb, FN = R - 2;
+  constexpr bool SPLIT = MODE == SW_GS && L::split;
+  constexpr int NC = TT / 32 * (SPLIT ? 2 : 1);    // compute warps
+  constexpr int LAND = SPLIT ? FN - 3 : FN - 2;    // copies that may be on their way: waves to t + 2 (split: t + 3) are in
+  static_assert(LAND >= 0, "the split passes look one wave further");
   // own pieces copied (the last of the run stay: the backward LU-SGS pass reads no RHS)
   constexpr int OWN = L::met + (MODE == SW_LUSGS_BWD ? 1 : L::dyn);
   constexpr bool LOWER = MODE != SW_LUSGS_BWD, UPPER = MODE != SW_LUSGS_FWD;
@@ -412,6 +422,7 @@ __global__ void __launch_bounds__(kTileThreads + 64, TileLayout<T>::minb)
   const int plane = NB * sl, fplane = FP * sl, oplane = L::own * lines;
   uint4* const fresh = ring + R * plane;
   uint4* const own = fresh + 2 * fplane;
+  T* const ahead_terms = reinterpret_cast<T*>(own + (R - 1) * oplane);  // [2][kTileAheadValues][lines]
   if (threadIdx.x == 0) {
     s_slot = (int)atomicAdd(&ctl->ticket, 1u);
 #pragma unroll
@@ -435,9 +446,10 @@ __global__ void __launch_bounds__(kTileThreads + 64, TileLayout<T>::minb)
   T* const edge = reinterpret_cast<T*>(B.tl_edge);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  if (warp < kTileThreads / 32) {
+  if (warp < NC) {
     // ------------------------- compute threads -------------------------
-    const int l = threadIdx.x;
+    const bool helper = SPLIT && warp >= TT / 32;
+    const int l = (int)threadIdx.x - (helper ? TT : 0);
     const bool line = l < nl;
     const int tk = l / jw, tj = l - tk * jw;
     const T g1 = T(B.prm.gamma) - T(1);
@@ -468,38 +480,8 @@ __global__ void __launch_bounds__(kTileThreads + 64, TileLayout<T>::minb)
     const uint4* pown = own;
     int ra = 1;           // ring index of wave t+1
     unsigned parity = 0;  // of its barrier
-    mbar_wait(full0, 0, err);
-    __syncthreads();
-    for (int t = 0; t < nsteps; ++t) {
-      mbar_wait(full0 + 8 * ra, parity, err);
-      if ((unsigned)i < (unsigned)ni) {
-        const uint4* const fr = fresh + ((t + 1) & 1) * fplane;  // wave t-1's
-        TilePoint<T, MODE> cur;
-        cur.load(pown, nl, l, po);
-        T acc[5] = {T(0), T(0), T(0), T(0), T(0)}, v[5];
-        // lower neighbours first (i, j, k), then upper (i, j, k): the reference's order
-        if (LOWER) {
-          constexpr bool F = DIR > 0;
-          const uint4* const q = F ? pb : pa;
-          cur.template term<F>(0, false, q + l, nl, fr, sl, l, g1, nvis, acc);
-          cur.template term<F>(1, false, q + jl.at, jl.ps, fr, sl, jl.slot, g1, nvis, acc);
-          cur.template term<F>(2, false, q + kl.at, kl.ps, fr, sl, kl.slot, g1, nvis, acc);
-        }
-        if (UPPER) {
-          constexpr bool F = DIR < 0;
-          const uint4* const q = F ? pb : pa;
-          cur.template term<F>(0, true, q + l, nl, fr, sl, l, g1, nvis, acc);
-          cur.template term<F>(1, true, q + jh.at, jh.ps, fr, sl, jh.slot, g1, nvis, acc);
-          cur.template term<F>(2, true, q + kh_.at, kh_.ps, fr, sl, kh_.slot, g1, nvis, acc);
-        }
-        cur.result(acc, v);
-        TilePoint<T, MODE>::fresh_store(fresh + (t & 1) * fplane, sl, l, v);
-        if (out_j) edge_store(out_j + (long long)i * (kh * L::rec), v);
-        if (out_k) edge_store(out_k + (long long)i * (jw * L::rec), v);
-        TilePoint<T, MODE>::store(p, nl * 16, v);
-      }
+    auto next = [&]() {   // on to the next step
       i += DIR;
-      p += ps;
       pb = po;
       po = pa;
       pa += plane;
@@ -509,11 +491,88 @@ __global__ void __launch_bounds__(kTileThreads + 64, TileLayout<T>::minb)
         parity ^= 1;
       }
       pown = pown + oplane == own + (R - 1) * oplane ? own : pown + oplane;
-      __syncthreads();
+    };
+    mbar_wait(full0, 0, err);
+    __syncthreads();
+    if constexpr (SPLIT) {
+      if (helper) {
+        // step s: the terms of wave s's ahead neighbours (wave s + 1), read by
+        // the other warps at step s, formed while they are at step s - 1
+        for (int s = 0; s < nsteps; ++s) {
+          mbar_wait(full0 + 8 * ra, parity, err);
+          if ((unsigned)i < (unsigned)ni) {
+            TilePoint<T, MODE> cur;
+            cur.load(pown, nl, l, po);
+            T* const out = ahead_terms + (s & 1) * kTileAheadValues * lines + l;
+            T a[3][5] = {};
+            constexpr bool U = DIR > 0;  // the ahead neighbours are the upper ones
+            // upper terms are subtracted one by one after the lower ones: each is
+            // handed over as 0 - term; lower ones are summed first
+            T(&a1)[5] = a[U ? 1 : 0];
+            T(&a2)[5] = a[U ? 2 : 0];
+            const Near &nj = U ? jh : jl, &nk = U ? kh_ : kl;
+            cur.template term<false>(0, U, pa + l, nl, fresh, sl, l, g1, nvis, a[0]);
+            cur.template term<false>(1, U, pa + nj.at, nj.ps, fresh, sl, nj.slot, g1, nvis, a1);
+            cur.template term<false>(2, U, pa + nk.at, nk.ps, fresh, sl, nk.slot, g1, nvis, a2);
+#pragma unroll
+            for (int m = 0; m < (U ? 15 : 5); ++m) out[m * lines] = a[m / 5][m % 5];
+          }
+          next();
+          __syncthreads();
+        }
+      }
+    }
+    if (!helper) {
+      if (SPLIT) __syncthreads();  // wave 0's ahead terms
+      for (int t = 0; t < nsteps; ++t) {
+        mbar_wait(full0 + 8 * ra, parity, err);
+        if ((unsigned)i < (unsigned)ni) {
+          const uint4* const fr = fresh + ((t + 1) & 1) * fplane;  // wave t-1's
+          TilePoint<T, MODE> cur;
+          cur.load(pown, nl, l, po);
+          T acc[5] = {T(0), T(0), T(0), T(0), T(0)}, v[5];
+          const T* const given = ahead_terms + (t & 1) * kTileAheadValues * lines + l;
+          // lower neighbours first (i, j, k), then upper (i, j, k): the reference's order
+          if (LOWER) {
+            constexpr bool F = DIR > 0;
+            if constexpr (SPLIT && !F) {
+#pragma unroll
+              for (int m = 0; m < 5; ++m) acc[m] = given[m * lines];
+            } else {
+              const uint4* const q = F ? pb : pa;
+              cur.template term<F>(0, false, q + l, nl, fr, sl, l, g1, nvis, acc);
+              cur.template term<F>(1, false, q + jl.at, jl.ps, fr, sl, jl.slot, g1, nvis, acc);
+              cur.template term<F>(2, false, q + kl.at, kl.ps, fr, sl, kl.slot, g1, nvis, acc);
+            }
+          }
+          if (UPPER) {
+            constexpr bool F = DIR < 0;
+            if constexpr (SPLIT && !F) {
+#pragma unroll
+              for (int m = 0; m < 15; ++m) acc[m % 5] += given[m * lines];
+            } else {
+              const uint4* const q = F ? pb : pa;
+              cur.template term<F>(0, true, q + l, nl, fr, sl, l, g1, nvis, acc);
+              cur.template term<F>(1, true, q + jh.at, jh.ps, fr, sl, jh.slot, g1, nvis, acc);
+              cur.template term<F>(2, true, q + kh_.at, kh_.ps, fr, sl, kh_.slot, g1, nvis, acc);
+            }
+          }
+          cur.result(acc, v);
+          TilePoint<T, MODE>::fresh_store(fresh + (t & 1) * fplane, sl, l, v);
+          if (out_j) edge_store(out_j + (long long)i * (kh * L::rec), v);
+          if (out_k) edge_store(out_k + (long long)i * (jw * L::rec), v);
+          TilePoint<T, MODE>::store(p, nl * 16, v);
+        }
+        p += ps;
+        next();
+        __syncthreads();
+      }
+    } else {
+      __syncthreads();  // the last step
     }
   } else {
     // ------------------- behind / ahead halo lines ----------------------
-    const bool behind = warp == kTileThreads / 32;
+    const bool behind = warp == NC;
     const int side = (behind == (DIR > 0)) ? 0 : 1;  // lower or upper neighbours
     const bool isj = lane < kh;
     const int q = isj ? lane : lane - kh;
@@ -558,8 +617,9 @@ __global__ void __launch_bounds__(kTileThreads + 64, TileLayout<T>::minb)
         fetch(s, s);
         cp_async_commit();
       }
-      cp_async_wait<FN - 2>();
+      cp_async_wait<LAND>();
       __syncthreads();
+      if (SPLIT) __syncthreads();  // wave 0's ahead terms
       int r = FN;  // ring index of wave t + FN
       for (int t = 0; t < nsteps; ++t) {
         if (t + FN <= nsteps) send(t + FN);
@@ -568,7 +628,7 @@ __global__ void __launch_bounds__(kTileThreads + 64, TileLayout<T>::minb)
         i += DIR;
         src += ss;
         if (++r == R) r = 0;
-        cp_async_wait<FN - 2>();
+        cp_async_wait<LAND>();
         __syncthreads();
       }
     } else {
@@ -619,9 +679,10 @@ __global__ void __launch_bounds__(kTileThreads + 64, TileLayout<T>::minb)
       }
       ask(i - DIR, b[0]);  // steps -1 and 0
       ask(i + DIR, b[1]);  // steps 1 and 2
-      cp_async_wait<FN - 2>();
+      cp_async_wait<LAND>();
       deliver(-1, i - DIR, b[0][0]);
       __syncthreads();
+      if (SPLIT) __syncthreads();
       int r = FN;
       for (int t0 = 0; t0 < nsteps; t0 += 4) {
 #pragma unroll
@@ -635,7 +696,7 @@ __global__ void __launch_bounds__(kTileThreads + 64, TileLayout<T>::minb)
             i += DIR;
             src += ss;
             if (++r == R) r = 0;
-            cp_async_wait<FN - 2>();
+            cp_async_wait<LAND>();
             __syncthreads();
           }
         }

@@ -7,9 +7,16 @@
 
 namespace orion {
 
-// lines per tile: FP64 tiles of 112 keep five waves of ring and four of own
-// operands in 227 KB of shared memory, FP32 tiles run two to an SM
-constexpr int kTileMaxLines = 112;
+// Lines per tile at most.  FP32 tiles of 112 run two to an SM, FP64 tiles of 96
+// keep their waves in 227 KB of shared memory.  An FP64 case with few lines
+// takes tiles of 64: it has SMs to spare, and a wave of two warps is shorter
+// than one of three (they share the SM's load path).  Few: at most 148 x 64
+// grid lines along i in all blocks, one small tile an SM (97x49x33 by stages
+// 5.29 ms against 5.71, Euler 111x53x47 3.97 against 4.15; 193x97x65, 12,936
+// lines, 2.63 against 2.54; FP32 gained nothing).
+constexpr int kTileLinesSmall = 64;
+constexpr long long kTileSmallCase = 148 * kTileLinesSmall;
+constexpr int tile_max_lines(size_t ssz, bool small) { return ssz == 8 ? (small ? kTileLinesSmall : 96) : 112; }
 constexpr int kTileMaxEdge = 32;    // jw + kh (one halo warp)
 // Components of the hyperplane form's point arrays.  The two forms' arrays
 // share memory (only the form in use keeps its arrays), so a plan that needs
@@ -52,7 +59,7 @@ inline void tile_counts(int ni, int nj, int nk, int nJ, int nK, long long& slots
 // counted with the compute warps) x waves, weighted by the hops the wavefront
 // takes through the tiles.  Partitions whose arrays outgrow the hyperplane
 // form's are taken only when none fits.
-inline TilePlan make_tile_plan(int ni, int nj, int nk, size_t ssz) {
+inline TilePlan make_tile_plan(int ni, int nj, int nk, size_t ssz, int max_lines) {
   const size_t budget = (size_t)kPlaneComps * ssz * (size_t)ni * nj * nk;
   int bJ = nj, bK = nk;
   double best = -1.0;
@@ -65,7 +72,7 @@ inline TilePlan make_tile_plan(int ni, int nj, int nk, size_t ssz) {
     lastJ = nJ;
     const int jw = (nj + nJ - 1) / nJ;
     int lastK = 0;
-    for (int h = std::min(kTileMaxEdge - jw, kTileMaxLines / jw); h >= 1; --h) {
+    for (int h = std::min(kTileMaxEdge - jw, max_lines / jw); h >= 1; --h) {
       const int nK = (nk + h - 1) / h;
       if (nK == lastK) continue;
       lastK = nK;

@@ -19,8 +19,8 @@ static int fault(const char* what, int ni, int nj, int nk, size_t ssz) {
   return 1;
 }
 
-static int check(int ni, int nj, int nk, size_t ssz) {
-  const TilePlan p = make_tile_plan(ni, nj, nk, ssz);
+static int check(int ni, int nj, int nk, size_t ssz, int max_lines) {
+  const TilePlan p = make_tile_plan(ni, nj, nk, ssz, max_lines);
   const int nJ = p.nJ(), nK = p.nK();
   if (p.jb.front() != 0 || p.jb.back() != nj || p.kb.front() != 0 || p.kb.back() != nk) return fault("cover", ni, nj, nk, ssz);
   if (tile_array_bytes(p.slots, p.records, ssz) > (size_t)kPlaneComps * ssz * ni * nj * nk) return fault("memory", ni, nj, nk, ssz);
@@ -47,7 +47,7 @@ static int check(int ni, int nj, int nk, size_t ssz) {
     for (int a = 0; a < nJ; ++a) {
       const int jw = p.jw(a), kh = p.kh(b), nsteps = ni + jw + kh - 2;
       const size_t t = (size_t)b * nJ + a;
-      if (jw < 1 || kh < 1 || jw * kh > kTileMaxLines || jw + kh > kTileMaxEdge) return fault("tile size", ni, nj, nk, ssz);
+      if (jw < 1 || kh < 1 || jw * kh > max_lines || jw + kh > kTileMaxEdge) return fault("tile size", ni, nj, nk, ssz);
       if (p.base[t] < jw * kh || p.base[t] + (long long)(nsteps + 1) * jw * kh > p.slots) return fault("waves", ni, nj, nk, ssz);
       for (int dir = 1; dir >= -1; dir -= 2) {
         // own lines: point and slot by step
@@ -100,7 +100,8 @@ static int check(int ni, int nj, int nk, size_t ssz) {
 int main(int argc, char** argv) {
   for (int x = 1; x + 2 < argc; x += 3)
     for (size_t ssz : {4, 8})
-      if (check(std::atoi(argv[x]), std::atoi(argv[x + 1]), std::atoi(argv[x + 2]), ssz)) return 1;
+      for (bool small : {false, true})
+        if (check(std::atoi(argv[x]), std::atoi(argv[x + 1]), std::atoi(argv[x + 2]), ssz, tile_max_lines(ssz, small))) return 1;
   std::printf("ok\n");
   return 0;
 }

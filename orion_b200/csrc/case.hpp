@@ -81,6 +81,8 @@ struct DeviceLists {
   bool tiles_on = false;
   void* sweep_tiles[2] = {nullptr, nullptr};     // SweepTile lists, forward / backward
   int n_sweep_tiles[2] = {0, 0};
+  void* tile_rows = nullptr;                     // TileRow list of the preparation
+  int n_tile_rows = 0;
   void* tile_ctl = nullptr;                      // TileCtl
   int tile_lines = 0;                            // lines of the largest tile
   bool tile_small = false;                       // every tile has at most kTileLinesSmall

@@ -341,75 +341,15 @@ __global__ void k_bc_phase(const BlockDev<S>* __restrict__ blocks, const RegionD
 // (they are read nowhere else).  phydtime = min(1000, min dt*vol) via atomicMin
 // on the bit pattern of a positive double.
 // ===========================================================================
-template <typename S, bool DO_Q>
-__device__ __forceinline__ void state_point(const BlockDev<S>& B, const ParamsDev& P, long long idx, int i, int j,
-                                            int k, S& c_out, S& mu_out) {
-  // arithmetic in the storage precision S of c, mu, dt (FP64 on the plain path)
-  const long long np = B.npad;
-  const bool inI = (i >= NG && i < NG + B.ni), inJ = (j >= NG && j < NG + B.nj), inK = (k >= NG && k < NG + B.nk);
-  const int nin = (int)inI + (int)inJ + (int)inK;
-  double* prim = B.prim;
-  const S gamma = (S)P.gamma, moo = (S)P.moo, visc = (S)P.visc;
-  S T = (S)prim[5 * np + idx];
-  S cval = B.c[idx];
-  if (nin >= 2) {
-    // interior (nin == 3) or ghost face slab (nin == 2), update_thermodynamics_block
-    S rho = (S)__ldg(prim + idx);
-    const S p = (S)__ldg(prim + 4 * np + idx);
-    if (nin == 2) rho = tabs(rho);
-    const S a2 = gamma * p / rho;
-    cval = tsqrt(tabs(a2));
-    B.c[idx] = cval;
-    if (P.nvis == 1) {
-      T = (moo * moo) * a2;
-      prim[5 * np + idx] = (double)T;
-    }
-    if (DO_Q) {
-      // update_conservative_block (StateUpdater.cpp:94-149), FP64
-      const double r0 = __ldg(prim + idx), u = __ldg(prim + np + idx), v = __ldg(prim + 2 * np + idx),
-                   w = __ldg(prim + 3 * np + idx), pd = __ldg(prim + 4 * np + idx);
-      const bool use_abs = (nin == 2);
-      const double rc = (use_abs || r0 < 0.0) ? fabs(r0) : r0;
-      const double gm1_inv = 1.0 / (P.gamma - 1.0);
-      B.q[idx] = rc;
-      B.q[np + idx] = rc * u;
-      B.q[2 * np + idx] = rc * v;
-      B.q[3 * np + idx] = rc * w;
-      const double ke = 0.5 * rc * (u * u + v * v + w * w);
-      B.q[4 * np + idx] = pd * gm1_inv + ke;
-    }
-  }
-  S muv = B.mu[idx];
-  if (P.nvis == 1) {
-    // update_viscosity_block (StateUpdater.cpp:75-92): whole padded array
-    S tm = T;
-    if (tm < S(1e-6)) tm = S(1e-6);
-    muv = tm * tsqrt(tm) * (S(1) + visc) / (tm + visc);
-    B.mu[idx] = muv;
-  }
-  for (int m = 0; m < 5; ++m) B.dq[m * np + idx] = (S)0;
-  if (sizeof(S) == 4) {  // the flux kernels' FP32 copy of prim, after the BCs and T
-    for (int m = 0; m < 5; ++m) B.prim_f[m * np + idx] = (float)prim[m * np + idx];
-    B.prim_f[5 * np + idx] = (float)prim[5 * np + idx];
-  }
-  c_out = cval;
-  mu_out = muv;
-}
-
+// calculate_spectrum + calculate_local_dt_cell (TimeIntegrator.cpp:20-125) from
+// one point's values; km: its metrics.
 template <typename S>
-__device__ __forceinline__ S timestep_point(const BlockDev<S>& B, const ParamsDev& P, long long idx, S c, S mu) {
-  // calculate_spectrum + calculate_local_dt_cell (TimeIntegrator.cpp:20-125)
-  const long long np = B.npad;
-  const S u = (S)__ldg(B.prim + np + idx), v = (S)__ldg(B.prim + 2 * np + idx), w = (S)__ldg(B.prim + 3 * np + idx);
-  const S rho = (S)__ldg(B.prim + idx);
-  const S vol = (S)__ldg(FluxSrc<S>::vol(B) + idx);
+__device__ __forceinline__ S timestep_value(const ParamsDev& P, S rho, S u, S v, S w, S vol, S c, S mu, const S km[9]) {
   const S reynolds = (S)P.reynolds, csrv = (S)P.csrv;
   S sum_spec = S(0);
-  const auto* met = FluxSrc<S>::metrics(B);
+#pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const S mx = (S)__ldg(met + (3 * d + 0) * np + idx);
-    const S my = (S)__ldg(met + (3 * d + 1) * np + idx);
-    const S mz = (S)__ldg(met + (3 * d + 2) * np + idx);
+    const S mx = km[3 * d], my = km[3 * d + 1], mz = km[3 * d + 2];
     const S U_contra = tabs(u * mx + v * my + w * mz);
     const S grad_len = tsqrt(mx * mx + my * my + mz * mz);
     const S spec = U_contra + c * grad_len;
@@ -467,7 +407,7 @@ __device__ __forceinline__ void dtmin_final_body(const double* __restrict__ part
   }
 }
 
-// CTAs per SM (256 threads each) the state and sweep-preparation kernels are
+// CTAs per SM (256 threads each) the sweep-preparation kernels are
 // compiled for (register cap 65536 / (256 n)), per precision.  Measured on C3
 // against the compiler's own choice (80-109 registers): FP32 six, FP64 four
 // (a few spilled registers each) took the mixed step from 16.7 to 15.9 ms and
@@ -478,35 +418,90 @@ __device__ __forceinline__ void dtmin_final_body(const double* __restrict__ part
 #ifndef ORION_PTWISE_MINB_F64
 #define ORION_PTWISE_MINB_F64 4
 #endif
+#ifndef ORION_STATE_MINB
+#define ORION_STATE_MINB 4
+#endif
 template <typename T> struct PointwiseMinBlocks;
 template <> struct PointwiseMinBlocks<float> { static constexpr int n = ORION_PTWISE_MINB_F32; };
 template <> struct PointwiseMinBlocks<double> { static constexpr int n = ORION_PTWISE_MINB_F64; };
 
+// One point a thread, every value it needs asked for before the first is used:
+// what bounds it is the latency of its loads, and stores in between held the
+// later ones back (385x257x129 mixed 0.83 -> 0.57 ms, plain 1.06 -> 0.72; at four
+// CTAs an SM, three the same).  Arithmetic in the storage precision S of c, mu,
+// dt (FP64 on the plain path).
 template <typename S, bool DO_Q, bool DO_DT>
-__global__ void __launch_bounds__(256, PointwiseMinBlocks<S>::n) k_state(const BlockDev<S>* __restrict__ blocks, const Chunk* __restrict__ chunks,
+__global__ void __launch_bounds__(256, ORION_STATE_MINB) k_state(const BlockDev<S>* __restrict__ blocks, const Chunk* __restrict__ chunks,
                         double* __restrict__ dt_part) {
   const Chunk ch = chunks[blockIdx.x];
-  const BlockDev<S> B = blocks[ch.block];
+  const BlockDev<S>& B = blocks[ch.block];
   const ParamsDev& P = B.prm;
   double local_min = 1000.0;
-#pragma unroll 4
-  for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
-    const long long idx = ch.start + t;
-    const int i32 = (int)idx;  // padded index < 2^31
-    const int i = i32 % B.nx;
-    const int r = i32 / B.nx;
-    const int j = r % B.ny;
-    const int k = r / B.ny;
-    S c, mu;
-    state_point<S, DO_Q>(B, P, idx, i, j, k, c, mu);
-    if (DO_DT) {
-      const bool interior = (i >= NG && i < NG + B.ni && j >= NG && j < NG + B.nj && k >= NG && k < NG + B.nk);
-      if (interior) {
-        const S dtv = timestep_point(B, P, idx, c, mu);
-        B.dt[idx] = dtv;
-        const double dt_phys = (double)dtv * B.vol[idx];
-        if (dt_phys < local_min) local_min = dt_phys;
+  if ((int)threadIdx.x < ch.count) {
+    const long long np = B.npad;
+    const int nx = B.nx, ny = B.ny;
+    const int i32 = (int)ch.start + threadIdx.x;  // padded index < 2^31
+    const long long idx = i32;
+    const int r32 = i32 / nx, i = i32 - r32 * nx;
+    const int k = r32 / ny, j = r32 - k * ny;
+    const bool inI = (i >= NG && i < NG + B.ni), inJ = (j >= NG && j < NG + B.nj), inK = (k >= NG && k < NG + B.nk);
+    const int nin = (int)inI + (int)inJ + (int)inK;  // 3: interior, 2: ghost face slab
+    double* const prim = B.prim;
+    double pr[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) pr[m] = prim[m * np + idx];
+    S km[9], vol = S(0);
+    double vol64 = 0.0;
+    if (DO_DT && nin == 3) {
+      const S* const met = FluxSrc<S>::metrics(B);
+#pragma unroll
+      for (int m = 0; m < 9; ++m) km[m] = met[m * np + idx];
+      vol = FluxSrc<S>::vol(B)[idx];
+      vol64 = B.vol[idx];
+    }
+    const int nvis = P.nvis;
+    const S moo = (S)P.moo, visc = (S)P.visc;
+    S T = (S)pr[5], cval = S(0), muv = S(0);
+    if (nin >= 2) {  // update_thermodynamics_block
+      S rho = (S)pr[0];
+      if (nin == 2) rho = tabs(rho);
+      const S a2 = (S)P.gamma * (S)pr[4] / rho;
+      cval = tsqrt(tabs(a2));
+      if (nvis == 1) T = (moo * moo) * a2;
+    }
+    if (nvis == 1) {  // update_viscosity_block (StateUpdater.cpp:75-92): whole padded array
+      S tm = T;
+      if (tm < S(1e-6)) tm = S(1e-6);
+      muv = tm * tsqrt(tm) * (S(1) + visc) / (tm + visc);
+      B.mu[idx] = muv;
+    }
+    if (nin >= 2) {
+      B.c[idx] = cval;
+      if (nvis == 1) prim[5 * np + idx] = (double)T;
+      if (DO_Q) {  // update_conservative_block (StateUpdater.cpp:94-149), FP64
+        const bool use_abs = (nin == 2);
+        const double rc = (use_abs || pr[0] < 0.0) ? fabs(pr[0]) : pr[0];
+        const double gm1_inv = 1.0 / (P.gamma - 1.0);
+        B.q[idx] = rc;
+        B.q[np + idx] = rc * pr[1];
+        B.q[2 * np + idx] = rc * pr[2];
+        B.q[3 * np + idx] = rc * pr[3];
+        const double ke = 0.5 * rc * (pr[1] * pr[1] + pr[2] * pr[2] + pr[3] * pr[3]);
+        B.q[4 * np + idx] = pr[4] * gm1_inv + ke;
       }
+    }
+#pragma unroll
+    for (int m = 0; m < 5; ++m) B.dq[m * np + idx] = (S)0;
+    if constexpr (sizeof(S) == 4) {  // the flux kernels' FP32 copy of prim, after the BCs and T
+#pragma unroll
+      for (int m = 0; m < 5; ++m) B.prim_f[m * np + idx] = (float)pr[m];
+      B.prim_f[5 * np + idx] = (nin >= 2 && nvis == 1) ? (float)T : (float)pr[5];
+    }
+    if (DO_DT && nin == 3) {
+      const S dtv = timestep_value<S>(P, (S)pr[0], (S)pr[1], (S)pr[2], (S)pr[3], vol, cval, muv, km);
+      B.dt[idx] = dtv;
+      const double dt_phys = (double)dtv * vol64;
+      if (dt_phys < local_min) local_min = dt_phys;
     }
   }
   if (DO_DT) block_min_to(local_min, dt_part);
@@ -525,7 +520,11 @@ __global__ void k_timestep(const BlockDev<S>* __restrict__ blocks, const Chunk* 
     const int n32 = (int)n, r32 = n32 / B.ni;
     const int ii = n32 - r32 * B.ni, jj = r32 % B.nj, kk = r32 / B.nj;
     const long long idx = lin(B, NG + ii, NG + jj, NG + kk);
-    const S dtv = timestep_point(B, P, idx, B.c[idx], B.mu[idx]);
+    const long long np = B.npad;
+    S km[9];
+    for (int m = 0; m < 9; ++m) km[m] = (S)__ldg(FluxSrc<S>::metrics(B) + m * np + idx);
+    const S dtv = timestep_value<S>(P, (S)B.prim[idx], (S)B.prim[np + idx], (S)B.prim[2 * np + idx],
+                                    (S)B.prim[3 * np + idx], FluxSrc<S>::vol(B)[idx], B.c[idx], B.mu[idx], km);
     B.dt[idx] = dtv;
     const double dt_phys = (double)dtv * B.vol[idx];
     if (dt_phys < local_min) local_min = dt_phys;
@@ -539,53 +538,39 @@ __global__ void k_timestep(const BlockDev<S>* __restrict__ blocks, const Chunk* 
 // (compute_derivatives_cell + compute_node_deriv_line,
 // src/solver/FluxComputer.cpp:13-67, 301-376).
 // ===========================================================================
-template <typename T, typename A>
-__device__ __forceinline__ T node_deriv(const A* __restrict__ q, long long o, long long st, int t, int L,
-                                        bool fl, bool fr) {
-  // q + o is memory coordinate 0 of the line, st the along-line stride, t the interior index.
-  auto Q = [&](int p) -> T { return (T)q[o + (long long)p * st]; };
-  if (fl && t == 0) {
-    const T q1 = Q(3), q2 = Q(4), q3 = Q(5), q4 = Q(6);
-    return (T(-11) * q1 + T(18) * q2 - T(9) * q3 + T(2) * q4) / T(6);
-  }
-  if (fl && t == 1) {
-    const T q1 = Q(3), q2 = Q(4), q3 = Q(5), q4 = Q(6), q5 = Q(7);
-    return (T(-3) * q1 + T(-10) * q2 + T(18) * q3 + T(-6) * q4 + T(1) * q5) / T(12);
-  }
-  if (fr && t == L - 1) {
-    const T qn = Q(L + 2), qn_1 = Q(L + 1), qn_2 = Q(L), qn_3 = Q(L - 1);
-    return -(T(-11) * qn + T(18) * qn_1 - T(9) * qn_2 + T(2) * qn_3) / T(6);
-  }
-  if (fr && t == L - 2) {
-    const T qn = Q(L + 2), qn_1 = Q(L + 1), qn_2 = Q(L), qn_3 = Q(L - 1), qn_4 = Q(L - 2);
-    return -(T(-3) * qn + T(-10) * qn_1 + T(18) * qn_2 + T(-6) * qn_3 + T(1) * qn_4) / T(12);
-  }
-  const int p = t + NG;
-  return (T(8) * (Q(p + 1) - Q(p - 1)) + T(-1) * (Q(p + 2) - Q(p - 2))) / T(12);
-}
-
 template <typename S, typename T>
 __global__ void k_node_derivs(const BlockDev<S>* __restrict__ blocks, const Chunk* __restrict__ chunks) {
   const Chunk ch = chunks[blockIdx.x];
-  const BlockDev<S> B = blocks[ch.block];
+  const BlockDev<S>& B = blocks[ch.block];
+  if ((int)threadIdx.x >= ch.count) return;
   const long long np = B.npad;
-  for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
-    const long long n = ch.start + t;
-    const int n32 = (int)n, r32 = n32 / B.ni;
-    const int ii = n32 - r32 * B.ni, jj = r32 % B.nj, kk = r32 / B.nj;
-    const long long idx = lin(B, NG + ii, NG + jj, NG + kk);
-    const int tt[3] = {ii, jj, kk};
-    for (int d = 0; d < 3; ++d) {
-      const long long st = stride_along(B, d);
-      const long long o = idx - (long long)(tt[d] + NG) * st;  // along-line coordinate 0
-      const int L = dim_along(B, d);
-      const bool fl = tt[d] <= 1 && B.prim[o] < 0.0;  // the one-sided formulas' points only
-      const bool fr = tt[d] >= L - 2 && B.prim[o + (long long)(L + 5) * st] < 0.0;
-      const int comp[4] = {1, 2, 3, 5};
-      for (int m = 0; m < 4; ++m) {
-        const T v = node_deriv<T>(FluxSrc<S>::prim(B) + comp[m] * np, o, st, tt[d], L, fl, fr);
-        B.duvwt[(m + 4 * d) * np + idx] = (S)v;
+  const int n32 = (int)ch.start + threadIdx.x, r32 = n32 / B.ni;
+  const int kk = r32 / B.nj, jj = r32 - kk * B.nj, ii = n32 - r32 * B.ni;
+  const long long idx = lin(B, NG + ii, NG + jj, NG + kk);
+  const S* const prim = FluxSrc<S>::prim(B) + idx;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int t = d == 0 ? ii : (d == 1 ? jj : kk), L = dim_along(B, d);
+    const int st = (int)stride_along(B, d);  // padded indices are below 2^31
+    // one-sided at the two points of a flagged end (ghost-3 density below zero)
+    bool low = t <= 1, high = t >= L - 2;
+    if (low) low = B.prim[idx - (long long)(t + NG) * st] < 0.0;
+    if (high) high = B.prim[idx + (long long)(L + 2 - t) * st] < 0.0;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const S* const q = prim + (m < 3 ? m + 1 : 5) * np;
+      T v;
+      if (low || high) {
+        const int in = low ? st : -st, far = low ? t : L - 1 - t;  // points from the end
+        const S* const e = q - far * in;
+        const T q1 = (T)e[0], q2 = (T)e[in], q3 = (T)e[2 * in], q4 = (T)e[3 * in];
+        if (far == 0) v = div6(T(-11) * q1 + T(18) * q2 - T(9) * q3 + T(2) * q4);
+        else v = div12(T(-3) * q1 + T(-10) * q2 + T(18) * q3 + T(-6) * q4 + T(1) * (T)e[4 * in]);
+        if (!low) v = -v;
+      } else {
+        v = div12(T(8) * ((T)q[st] - (T)q[-st]) + T(-1) * ((T)q[2 * st] - (T)q[-2 * st]));
       }
+      B.duvwt[(m + 4 * d) * np + idx] = (S)v;
     }
   }
 }
@@ -1342,13 +1327,15 @@ __global__ void __launch_bounds__(NT, 1) k_sweeps_cluster(const BlockDev<S>* __r
 // partials (ResidualMonitor::compute).
 template <typename S>
 __device__ __forceinline__ void limited_update(const BlockDev<S>& B, const ParamsDev& P, long long idx,
-                                               const double dq[5]);
+                                               const double pr[5], const double dq[5]);
 __device__ __forceinline__ void res_combine(double& sum, double& mx, long long& key, double osum, double omx,
                                             long long okey);
 template <int NT>
 __device__ __forceinline__ void block_reduce_res(double& sum, double& mx, long long& key);
 
-// CTAs per SM the finish kernel is compiled for (register cap 65536 / (NT n)):
+// The finish kernel asks for every value before its first store (385x257x129
+// mixed 0.67 -> 0.50 ms, plain 0.81 -> 0.66).
+// CTAs per SM it is compiled for (register cap 65536 / (NT n)):
 // on C3 four (64 registers, a few spilled) took the update stage from 7.43 to
 // 7.04 ms mixed and 11.93 to 11.54 ms plain against no cap (105 registers).
 #ifndef ORION_FINISH_MINB
@@ -1404,11 +1391,20 @@ __global__ void __launch_bounds__(NT, ORION_FINISH_MINB) k_sweep_finish(const Bl
   const long long np = B.npad, nc = B.ncomp;
   double sum = 0.0, mx = -1.0;
   long long key = (long long)0x7fffffffffffffffLL;
-  for (int t = threadIdx.x; t < ch.count; t += NT) {
-    const long long n = ch.start + t;
+  if ((int)threadIdx.x < ch.count) {
+    const long long n = ch.start + threadIdx.x;
     const int n32 = (int)n, r32 = n32 / B.ni;
-    const int ii = n32 - r32 * B.ni, jj = r32 % B.nj, kk = r32 / B.nj;
+    const int kk = r32 / B.nj, jj = r32 - kk * B.nj, ii = n32 - r32 * B.ni;
     const long long idx = lin(B, NG + ii, NG + jj, NG + kk);
+    // every load before the first store
+    double pr[5], vol = 0.0, dt = 0.0;
+#pragma unroll
+    for (int m = 0; m < 5; ++m) pr[m] = B.prim[m * np + idx];
+    if (DO_RES) {
+      vol = B.vol[idx];
+      dt = (double)B.dt[idx];
+    }
+    const bool masked = B.bcmask[idx] != 0;
     S sw[5];
     if (TILES) {
       tile_increment(B, tile_slot(B, ii, jj, kk), sw);
@@ -1419,16 +1415,14 @@ __global__ void __launch_bounds__(NT, ORION_FINISH_MINB) k_sweep_finish(const Bl
       for (int m = 0; m < 5; ++m) sw[m] = __ldcs(B.sk_dq + m * nc + c);
     }
     double dq[5];
-    const bool masked = B.bcmask[idx] != 0;
+#pragma unroll
     for (int m = 0; m < 5; ++m) {
       const S v = masked ? (S)0 : sw[m];
       B.dq[m * np + idx] = v;
       dq[m] = (double)v;
     }
-    limited_update(B, P, idx, dq);
+    limited_update(B, P, idx, pr, dq);
     if (DO_RES) {
-      double vol = B.vol[idx];
-      double dt = (double)B.dt[idx];
       if (vol < 1e-30) vol = 1e-30;
       if (dt < 1e-30) dt = 1e-30;
       const double inv_factor = 1.0 / (dt * vol);
@@ -1450,18 +1444,17 @@ __global__ void __launch_bounds__(NT, ORION_FINISH_MINB) k_sweep_finish(const Bl
 }
 
 // ===========================================================================
-// Final update: set_boundary_dq_zero + update_limited (StateUpdater.cpp:447-542),
-// optionally fused with the residual (ResidualMonitor::compute,
-// src/solver/ResidualMonitor.cpp:11-137): per-CTA partial sums and maxima with
-// the lexicographic location key; a single CTA combines them in fixed order.
+// update_limited (StateUpdater.cpp:447-542) and the residual
+// (ResidualMonitor::compute, src/solver/ResidualMonitor.cpp:11-137): per-CTA
+// partial sums and maxima with the lexicographic location key; a single CTA
+// combines them in fixed order.
 // ===========================================================================
 template <typename S>
 __device__ __forceinline__ void limited_update(const BlockDev<S>& B, const ParamsDev& P, long long idx,
-                                               const double dq[5]) {
+                                               const double pr[5], const double dq[5]) {
   const long long np = B.npad;
   const double gm1 = P.gamma - 1.0;
-  const double r = B.prim[idx], u = B.prim[np + idx], v = B.prim[2 * np + idx], w = B.prim[3 * np + idx],
-               p = B.prim[4 * np + idx];
+  const double r = pr[0], u = pr[1], v = pr[2], w = pr[3], p = pr[4];
   const double E = p / gm1 + 0.5 * r * (u * u + v * v + w * w);
   double qn[5];
   qn[0] = r + dq[0];
@@ -1536,12 +1529,11 @@ __device__ __forceinline__ void block_reduce_res(double& sum, double& mx, long l
   }
 }
 
-template <typename S, bool DO_UPDATE, bool DO_RES, int NT>
+template <typename S, int NT>
 __global__ void __launch_bounds__(NT) k_update_res(const BlockDev<S>* __restrict__ blocks, const Chunk* __restrict__ chunks,
                                                     ResPartial* __restrict__ partials) {
   const Chunk ch = chunks[blockIdx.x];
   const BlockDev<S> B = blocks[ch.block];
-  const ParamsDev& P = B.prm;
   const long long np = B.npad;
   double sum = 0.0, mx = -1.0;
   long long key = (long long)0x7fffffffffffffffLL;
@@ -1551,36 +1543,24 @@ __global__ void __launch_bounds__(NT) k_update_res(const BlockDev<S>* __restrict
     const int ii = n32 - r32 * B.ni, jj = r32 % B.nj, kk = r32 / B.nj;
     const long long idx = lin(B, NG + ii, NG + jj, NG + kk);
     double dq[5];
-    if (DO_UPDATE && B.bcmask[idx]) {
-      for (int m = 0; m < 5; ++m) {
-        B.dq[m * np + idx] = (S)0;
-        dq[m] = 0.0;
-      }
-    } else {
-      for (int m = 0; m < 5; ++m) dq[m] = (double)B.dq[m * np + idx];
-    }
-    if (DO_UPDATE) limited_update(B, P, idx, dq);
-    if (DO_RES) {
-      double vol = B.vol[idx];
-      double dt = (double)B.dt[idx];
-      if (vol < 1e-30) vol = 1e-30;
-      if (dt < 1e-30) dt = 1e-30;
-      const double inv_factor = 1.0 / (dt * vol);
-      const long long kbase = (B.int_base + n) * 5;
-      for (int m = 0; m < 5; ++m) {
-        const double res = fabs(dq[m]) * inv_factor;
-        sum += res * res;
-        if (res > mx || (res == mx && kbase + m < key)) {
-          mx = res;
-          key = kbase + m;
-        }
+    for (int m = 0; m < 5; ++m) dq[m] = (double)B.dq[m * np + idx];
+    double vol = B.vol[idx];
+    double dt = (double)B.dt[idx];
+    if (vol < 1e-30) vol = 1e-30;
+    if (dt < 1e-30) dt = 1e-30;
+    const double inv_factor = 1.0 / (dt * vol);
+    const long long kbase = (B.int_base + n) * 5;
+    for (int m = 0; m < 5; ++m) {
+      const double res = fabs(dq[m]) * inv_factor;
+      sum += res * res;
+      if (res > mx || (res == mx && kbase + m < key)) {
+        mx = res;
+        key = kbase + m;
       }
     }
   }
-  if (DO_RES) {
-    block_reduce_res<NT>(sum, mx, key);
-    if (threadIdx.x == 0) partials[blockIdx.x] = ResPartial{sum, mx, key};
-  }
+  block_reduce_res<NT>(sum, mx, key);
+  if (threadIdx.x == 0) partials[blockIdx.x] = ResPartial{sum, mx, key};
 }
 
 template <typename S>

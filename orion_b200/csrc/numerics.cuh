@@ -123,7 +123,11 @@ __device__ __forceinline__ void roe_flux(const T ql[5], const T qr[5], T nx, T n
   f[4] = T(0.5) * (fl[4] + fr[4] - df4);
 }
 
-// a / 24 and a / 1920, FP64 rounded as the divisions.
+// a / 6, a / 12, a / 24 and a / 1920, FP64 rounded as the divisions.
+__device__ __forceinline__ double div6(double a) { return quotient(a, 6.0, 1.0 / 6.0); }
+__device__ __forceinline__ float div6(float a) { return a * (1.f / 6.f); }
+__device__ __forceinline__ double div12(double a) { return quotient(a, 12.0, 1.0 / 12.0); }
+__device__ __forceinline__ float div12(float a) { return a * (1.f / 12.f); }
 __device__ __forceinline__ double div24(double a) { return quotient(a, 24.0, 1.0 / 24.0); }
 __device__ __forceinline__ float div24(float a) { return a * (1.f / 24.f); }
 __device__ __forceinline__ double div1920(double a) { return quotient(a, 1920.0, 1.0 / 1920.0); }

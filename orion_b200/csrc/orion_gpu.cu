@@ -319,6 +319,7 @@ int build_sweep_tiles(orion_case_t c) {
   auto& L = c->L;
   const size_t ssz = c->prec == ORION_PREC_FP64 ? 8 : 4;
   std::vector<SweepTile> all;
+  std::vector<TileRow> rows;
   L.tile_lines = 0;
   for (int b = 0; b < c->nblocks; ++b) {
     const auto& h = c->hb[b];
@@ -356,6 +357,8 @@ int build_sweep_tiles(orion_case_t c) {
         }
         L.tile_lines = std::max(L.tile_lines, w.jw * w.kh);
         all.push_back(w);
+        for (int k = w.kb; k < w.kb + w.kh; ++k)
+          for (int i = 0; i < h.idim; i += kPrepI) rows.push_back(TileRow{b, i, w.jb, k});
       }
   }
   for (int dir = 0; dir < 2; ++dir) {
@@ -372,9 +375,12 @@ int build_sweep_tiles(orion_case_t c) {
     L.sweep_tiles[dir] = d;
     L.n_sweep_tiles[dir] = (int)all.size();
   }
+  TileRow* d_rows = nullptr;
   TileCtl* ctl = nullptr;
   int rc;
-  if ((rc = dev_alloc(c, &ctl, 1))) return rc;
+  if ((rc = dev_upload(c, &d_rows, rows, true)) || (rc = dev_alloc(c, &ctl, 1))) return rc;
+  L.tile_rows = d_rows;
+  L.n_tile_rows = (int)rows.size();
   L.tile_ctl = ctl;
   return 0;
 }
@@ -1786,6 +1792,7 @@ int build_group(orion_group_t g, orion_case_t px) {
   std::vector<long long> pk_idx, ap_idx;
   std::vector<std::vector<Chunk>> planes[2];
   std::vector<SweepTile> stiles[2];
+  std::vector<TileRow> trows;
   int max_planes = 0;
   for (int m = 0; m < nm; ++m) {
     orion_case_t c = mem[m];
@@ -1854,6 +1861,14 @@ int build_group(orion_group_t g, orion_case_t px) {
       for (int x : as) {
         if (x >= M.n_pack) return fail(ORION_E_UNSUPPORTED, "a shard cannot join a group");
         ap_slot.push_back(slot_base + x);
+      }
+    }
+    {
+      std::vector<TileRow> r;
+      if ((rc = download(c, r, static_cast<const TileRow*>(M.tile_rows), (size_t)M.n_tile_rows))) return rc;
+      for (auto x : r) {
+        x.block += bo;
+        trows.push_back(x);
       }
     }
     // sweeps: hyperplane t of every member, or the members' tiles after one another
@@ -1934,7 +1949,10 @@ int build_group(orion_group_t g, orion_case_t px) {
   L.sweep_nt = kSweepThreads;
   {
     TileCtl* ctl = nullptr;
-    if ((rc = dev_alloc(px, &ctl, 1))) return rc;
+    TileRow* rows = nullptr;
+    if ((rc = dev_upload(px, &rows, trows)) || (rc = dev_alloc(px, &ctl, 1))) return rc;
+    L.tile_rows = rows;
+    L.n_tile_rows = (int)trows.size();
     L.tile_ctl = ctl;
     int* sctl = nullptr;
     if ((rc = dev_alloc(px, &sctl, 4))) return rc;

@@ -373,7 +373,7 @@ struct Stages {
   static int update(orion_case_t c, bool fuse_residual) {
     auto& L = c->L;
     if (L.tiles_on) {
-      k_tile_prep<S, T><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks);
+      k_tile_prep<S, T><<<L.n_tile_rows, 256, 0, c->stream>>>(blocks(c), static_cast<const TileRow*>(L.tile_rows));
     } else {
       k_lusgs_prep<S, T><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks);
       k_sweep_pairs<S, T><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks);
@@ -454,7 +454,7 @@ struct Stages {
 
   static int residual(orion_case_t c) {
     auto& L = c->L;
-    k_update_res<S, false, true, kThreads><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks,
+    k_update_res<S, kThreads><<<L.n_int_chunks, kThreads, 0, c->stream>>>(blocks(c), L.int_chunks,
                                                                                         L.partials);
     residual_final(c);
     return 0;

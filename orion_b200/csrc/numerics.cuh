@@ -24,11 +24,15 @@ template <typename T> __device__ __forceinline__ T tmax(T a, T b) { return (a < 
 // r correctly rounded and q within one ulp, RN(q + r (a - b q)) = RN(a / b)).
 // The first correction brings q = RN(a r) within one ulp, the second is the
 // theorem's step.  Exact while a remainder stays normal: quotient_rcp gives 0,
-// and quotient 0, for a denominator beyond 1e+-290.
+// and quotient 0, for a denominator beyond 1e+-290.  Where the corrections meet
+// an infinity (an infinite or zero denominator, an infinite quotient) they end
+// in a NaN, and the product a r is what the division gives; the test is on the
+// high word, off the FP64 pipe.
 __device__ __forceinline__ double quotient(double a, double b, double r) {
-  double q = a * r;
-  q = __fma_rn(__fma_rn(-b, q, a), r, q);
-  return __fma_rn(__fma_rn(-b, q, a), r, q);
+  const double q0 = a * r;
+  const double q1 = __fma_rn(__fma_rn(-b, q0, a), r, q0);
+  const double q2 = __fma_rn(__fma_rn(-b, q1, a), r, q1);
+  return (__double2hiint(q2) & 0x7ff00000) == 0x7ff00000 ? q0 : q2;
 }
 __device__ __forceinline__ double quotient_rcp(double b) {
   return (b > 1.0e-290 && b < 1.0e290) ? __drcp_rn(b) : 0.0;

@@ -25,7 +25,7 @@
 // Across tiles a CTA needs the fresh increments of its behind-j and behind-k
 // neighbour tiles.  The producing thread stores each into an edge record as
 // soon as it has it; a warp of the consuming CTA polls the record itself,
-// word by word against a value no increment can have (kEdgeEmpty), and puts
+// word by word against a value no increment can have (all bits set), and puts
 // the record back to empty after reading.  So a hop between tiles costs one
 // L2 store and one L2 load: no fence, no progress counter, and no reset
 // between passes.  The ahead neighbours' old increments are plain loads: the

@@ -34,3 +34,26 @@ def test_mixed_rhs_follows_the_plain_one(dims, physical):
     assert np.isfinite(a).all() and np.isfinite(b).all()
     err = np.sqrt(((a - b) ** 2).sum() / (a ** 2).sum())
     assert err <= 1e-3, err
+
+
+@pytest.mark.parametrize("component", [1, 2, 3])
+def test_overflowing_smoothness_drops_its_stencils(component):
+    """A velocity of 1e80 at one point overflows the squared smoothness measure
+    of every stencil that holds it.  Those weights are c / inf = 0, so a state
+    one or two points away comes from the stencils without it and is finite:
+    only the two faces at the point are not, and dq only up to three points
+    from it along its three lines."""
+    n, s = 40, 20
+    case = cases.small_case("inf", dims=(n, n, n), noise_seed=6, nvis=0)
+    fs = solver.FlowFieldSet(case, precision=_lib.PREC_FP64)
+    solver.apply_physical_bc(None, fs)
+    prim = fs.download(0, "prim")
+    prim[component, 3 + s, 3 + s, 3 + s] = 1e80
+    fs.upload(0, "prim", prim)
+    solver.StateUpdater.update_flow_states(fs)
+    solver.InviscidFluxComputer.compute_inviscid_rhs(fs)
+    dq = fs.download(0, "dq")[:, 3:-3, 3:-3, 3:-3]
+    fs.close()
+    near = np.zeros((n, n, n), bool)
+    near[s - 3:s + 4, s, s] = near[s, s - 3:s + 4, s] = near[s, s, s - 3:s + 4] = True
+    assert np.isfinite(dq[:, ~near]).all()

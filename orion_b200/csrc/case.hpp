@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -194,6 +195,8 @@ struct orion_case_s {
   // group is built from them without reading the lists back
   std::unordered_map<const void*, std::vector<unsigned char>> list_mirror;
   IoPipe* io = nullptr;  // orion_io_*, made on first use
+  float* pack_stage = nullptr;  // orion_case_pack_output, made on first use
+  std::mutex pack_mu;           // of pack_stage
 };
 
 // A group of cases stepped together: one launch per stage over all of their

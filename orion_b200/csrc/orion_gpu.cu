@@ -632,6 +632,7 @@ void destroy_case(orion_case_t c) {
   io_release(c);
   // stream-ordered frees: no device-wide synchronisation while other cases run
   for (void* p : c->allocs) cudaFreeAsync(p, c->stream);
+  if (c->pack_stage) cudaFreeAsync(c->pack_stage, c->stream);
   if (c->arena) cudaFreeAsync(c->arena, c->stream);
   if (c->d_blocks) cudaFreeAsync(c->d_blocks, c->stream);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
@@ -1274,11 +1275,27 @@ int orion_case_pack_output(orion_case_t c, int block, float* host) {
   bool st;
   int rc = field_info(c, block, ORION_FIELD_PRIM, &dprim, &nc, &st);
   if (rc) return rc;
-  // Packed into the block's node derivatives, which every viscous stage forms
-  // anew before it reads them: an allocation per call mapped and unmapped memory
-  // (49 blocks of a group of 8 cases: 13 to 20 ms for 92 MB, of which the copies
-  // need 2).
-  float* const stage = c->prec == ORION_PREC_FP64 ? reinterpret_cast<float*>(c->bd64[block].duvwt) : c->bd32[block].duvwt;
+  // One staging buffer per case, for its largest block, kept from the first call
+  // on: an allocation per call mapped and unmapped memory (49 blocks of a group of
+  // 8 cases: 13 to 20 ms for 92 MB, of which the copies need 2).  A call holds it
+  // until its copy has arrived.  A capturing stream cannot be waited for, and would
+  // give memory of its graph only.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return fail(ORION_E_CUDA, "pack output: the case's stream is capturing");
+  }
+  std::lock_guard<std::mutex> lk(c->pack_mu);
+  if (!c->pack_stage) {
+    long long most = 0;
+    for (const auto& b : c->hb) most = std::max(most, (long long)b.idim * b.jdim * b.kdim);
+    if (cudaMallocAsync((void**)&c->pack_stage, sizeof(float) * 7 * most, c->stream) != cudaSuccess) {
+      cudaGetLastError();
+      c->pack_stage = nullptr;
+      return fail(ORION_E_NOMEM, "output staging buffer");
+    }
+  }
+  float* const stage = c->pack_stage;
   out::k_pack_output<<<148 * 4, kThreads, 0, c->stream>>>(static_cast<const double*>(dprim), h.npad, h.idim, h.jdim,
                                                           h.kdim, h.nx, h.ny, c->P.gamma, stage);
   cudaError_t e = cudaGetLastError();

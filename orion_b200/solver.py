@@ -214,7 +214,7 @@ class FlowFieldSet:
 
     def set_schedule(self, sweep: str, cluster_size: int = 0, lanes: int = 32):
         """Fixes the step schedule: sweep form (tiles | planes | grid | cluster), cluster size
-        (8, 16, 0 = largest co-resident) and grid lines per CTA of the line kernels."""
+        (8, 16, 0 = largest co-resident) and lanes (1-32), kept but without effect."""
         form = {v: k for k, v in _lib.SWEEP_NAMES.items()}[sweep]
         s = _lib.Schedule(form, cluster_size, lanes, 0.0)
         check(_lib.load().orion_case_set_schedule(self._h, C.byref(s)))

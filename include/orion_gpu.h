@@ -178,7 +178,9 @@ int orion_case_grid_metrics(orion_case_t c, int block, const double* x, const do
  * writes, src/postprocess/PostProcess.cpp:116-243): host receives 7 arrays of
  * idim*jdim*kdim floats, i fastest: density, pressure, temperature, Mach
  * (sqrt(|u|^2 / (gamma p / rho)) in FP64, 0 where gamma p / rho <= 1e-30),
- * u, v, w.  Packed on the device, then copied; waits. */
+ * u, v, w.  Packed on the device, then copied; waits.  The first call takes 28
+ * bytes a point of the case's largest block, kept until the case is destroyed;
+ * ORION_E_CUDA while the case's stream is capturing. */
 int orion_case_pack_output(orion_case_t c, int block, float* host);
 
 /* Grid metrics and Jacobian of one block on the host (compute_grid_metrics +

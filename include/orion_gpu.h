@@ -33,7 +33,9 @@ extern "C" {
 #define ORION_E_NOMEM (-3)     /* device allocation failed */
 #define ORION_E_UNSUPPORTED (-4)
 #define ORION_E_NUMERIC (-5)   /* non-finite residual */
-#define ORION_E_TIMEOUT (-6)   /* a bounded device wait gave up */
+#define ORION_E_TIMEOUT (-6)   /* a bounded device wait gave up: from the first call that waits for the sweeps concerned
+                                  (step, poll, sync, download, pack_output, residuals, phydtime, io_wait), once;
+                                  the state they left is of no use, new steps start from a new one */
 
 /* precision of a case */
 #define ORION_PREC_FP64 0      /* plain form: every stage in FP64 */

@@ -567,7 +567,6 @@ int build_lists(orion_case_t c, const std::vector<long long>& prim_off, const Ex
 
   if ((rc = dev_alloc(c, &L.partials, (size_t)L.n_int_chunks))) return rc;
   if ((rc = dev_alloc(c, &L.hist, (size_t)kHistCap))) return rc;
-  if ((rc = dev_alloc(c, &L.counter, 1))) return rc;
   if ((rc = dev_alloc(c, &L.dtmin, 1))) return rc;
   if ((rc = dev_alloc(c, &L.res_total, 1))) return rc;
   if ((rc = dev_alloc(c, &L.dt_part, (size_t)std::max(L.n_pad_chunks, L.n_int_chunks)))) return rc;
@@ -575,6 +574,7 @@ int build_lists(orion_case_t c, const std::vector<long long>& prim_off, const Ex
     int* ctl = nullptr;
     if ((rc = dev_alloc(c, &ctl, 4))) return rc;
     L.sweep_ctl = ctl;
+    L.counter = ctl + 2;
   }
   if ((rc = build_sweep_tiles(c))) return rc;
   return 0;
@@ -671,7 +671,15 @@ int field_info(orion_case_t c, int block, int field, void** dptr, int* ncomp, bo
 // member of a group that runs another form than its own, and a wait that gave up.
 static int use_sweep_arrays(orion_case_t c, bool tiles) {
   if (c->sweep_arrays == (tiles ? 1 : 0)) return 0;
-  return ops_for(c->prec).sweep_arrays(c, tiles);
+  const int rc = ops_for(c->prec).sweep_arrays(c, tiles);
+  if (rc) c->sweep_arrays = -1;
+  return rc;
+}
+
+// n updates were enqueued: after the launches, so that whoever sees the count
+// and then waits for the stream has waited for them.
+static void sweeps_enqueued(orion_case_t c, int n) {
+  if (c->L.tiles_on || c->L.persist_grid > 0) c->sweeps_sent += n;
 }
 
 static int capture_step(orion_case_t c, cudaGraph_t* g) {
@@ -1033,7 +1041,8 @@ int orion_case_get_schedule(orion_case_t c, orion_schedule_t* s) {
 }
 
 static int launch_steps(orion_case_t c, int nsteps);
-static int sweep_status(orion_case_t c);
+static int sweep_status(orion_case_t c, long long sent);
+static int wait_checked(orion_case_t c);
 static int enqueue_hist_copy(orion_case_t c, int nsteps, cudaStream_t st = nullptr);
 
 int orion_case_autotune(orion_case_t c, int steps_per_trial, orion_schedule_t* trials, int cap, int* ntrials,
@@ -1091,7 +1100,7 @@ int orion_case_autotune(orion_case_t c, int steps_per_trial, orion_schedule_t* t
     if ((r = launch_steps(c, steps_per_trial))) return r;
     CUDA_TRY(cudaEventRecord(e1, c->stream));
     CUDA_TRY(cudaEventSynchronize(e1));
-    if ((r = sweep_status(c))) return r;
+    if ((r = sweep_status(c, c->sweeps_sent))) return r;
     float ms = 0.f;
     CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
     if ((r = copy_state(false))) return r;
@@ -1140,8 +1149,7 @@ int orion_case_autotune(orion_case_t c, int steps_per_trial, orion_schedule_t* t
 
 int orion_case_sync(orion_case_t c) {
   if (!c) return fail(ORION_E_INVALID, "null case");
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
-  return 0;
+  return wait_checked(c);
 }
 
 int orion_case_stream(orion_case_t c, void** stream) {
@@ -1214,6 +1222,7 @@ int orion_case_download(orion_case_t c, int block, int field, double* host) {
   int rc = field_info(c, block, field, &d, &nc, &st);
   if (rc) return rc;
   if (!host) return fail(ORION_E_INVALID, "null host pointer");
+  if ((rc = wait_checked(c))) return rc;
   const size_t n = (size_t)c->hb[block].npad * nc;
   if (st && c->prec != ORION_PREC_FP64) {
     std::vector<float> tmp(n);
@@ -1286,6 +1295,7 @@ int orion_case_pack_output(orion_case_t c, int block, float* host) {
     return fail(ORION_E_CUDA, "pack output: the case's stream is capturing");
   }
   std::lock_guard<std::mutex> lk(c->pack_mu);
+  if ((rc = wait_checked(c))) return rc;
   if (!c->pack_stage) {
     long long most = 0;
     for (const auto& b : c->hb) most = std::max(most, (long long)b.idim * b.jdim * b.kdim);
@@ -1338,9 +1348,49 @@ int orion_compute_inviscid_rhs(orion_case_t c) {
 }
 int orion_update_solution(orion_case_t c) {
   return dispatch(c, [&](const StageOps& o) {
-    const int rc = use_sweep_arrays(c, c->L.tiles_on);
-    return rc ? rc : o.update(c, false);
+    int rc = use_sweep_arrays(c, c->L.tiles_on);
+    if (!rc) rc = o.update(c, false);
+    if (!rc) sweeps_enqueued(c, 1);
+    return rc;
   });
+}
+
+// An error word that was read (the stream is idle): a wait of the sweeps gave up.
+static int sweep_report(orion_case_t c, int word) {
+  if (!word) return 0;
+  c->sweep_arrays = -1;  // edge records may hold increments nobody read
+  CUDA_TRY(cudaMemsetAsync(c->L.sweep_ctl, 0, 2 * sizeof(int), c->stream));
+  CUDA_TRY(cudaStreamSynchronize(c->stream));
+  return fail(ORION_E_TIMEOUT, "a bounded wait of the implicit sweeps (grid barrier or tile progress) gave up waiting");
+}
+
+// Reads the sweeps' error word when updates up to `sent` (c->sweeps_sent, taken
+// before the stream was found idle) have run since it was last read.
+static int sweep_status(orion_case_t c, long long sent) {
+  if (c->sweeps_read >= sent) return 0;
+  int ctl[2] = {0, 0};
+  CUDA_TRY(cudaMemcpy(ctl, c->L.sweep_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
+  c->sweeps_read = sent;
+  return sweep_report(c, ctl[1]);
+}
+
+// The wait of every call that hands out what the steps left: a state or a
+// residual after sweeps that gave up is an error there, once.
+static int wait_checked(orion_case_t c) {
+  const long long sent = c->sweeps_sent;
+  CUDA_TRY(cudaStreamSynchronize(c->stream));
+  return sweep_status(c, sent);
+}
+
+// The same with the history counter, in one copy.
+static int wait_checked_counter(orion_case_t c, int* cnt) {
+  const long long sent = c->sweeps_sent;
+  CUDA_TRY(cudaStreamSynchronize(c->stream));
+  int ctl[3] = {0, 0, 0};
+  CUDA_TRY(cudaMemcpy(ctl, c->L.sweep_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
+  c->sweeps_read = sent;
+  *cnt = ctl[2];
+  return sweep_report(c, ctl[1]);
 }
 
 static int read_hist(orion_case_t c, long long first, int n, orion_residual_t* out) {
@@ -1362,9 +1412,8 @@ int orion_residual_compute(orion_case_t c, orion_residual_t* out) {
   if (!c || !out) return fail(ORION_E_INVALID, "null argument");
   if (c->shard.nranks > 1) return fail(ORION_E_INVALID, "a shard's residual is orion_shard_residual, reduced over the shards");
   int cnt = 0;
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
-  CUDA_TRY(cudaMemcpy(&cnt, c->L.counter, sizeof(int), cudaMemcpyDeviceToHost));
-  int rc = dispatch(c, [&](const StageOps& o) { return o.residual(c); });
+  int rc = wait_checked_counter(c, &cnt);
+  if (!rc) rc = dispatch(c, [&](const StageOps& o) { return o.residual(c); });
   if (rc) return rc;
   c->hist_count = cnt + 1;
   return read_hist(c, cnt, 1, out);
@@ -1373,7 +1422,8 @@ int orion_residual_compute(orion_case_t c, orion_residual_t* out) {
 int orion_phydtime(orion_case_t c, double* out) {
   if (!c || !out) return fail(ORION_E_INVALID, "null argument");
   unsigned long long bits = 0;
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
+  const int rc = wait_checked(c);
+  if (rc) return rc;
   CUDA_TRY(cudaMemcpy(&bits, c->L.dtmin, sizeof(bits), cudaMemcpyDeviceToHost));
   double v;
   std::memcpy(&v, &bits, sizeof(v));
@@ -1388,6 +1438,7 @@ static int launch_steps(orion_case_t c, int nsteps) {
   if (!rc && !c->L.group) rc = use_sweep_arrays(c, c->L.tiles_on);  // a group's: its members' (orion_group_submit)
   if (rc) return rc;
   for (int s = 0; s < nsteps; ++s) CUDA_TRY(cudaGraphLaunch(c->graph, c->stream));
+  sweeps_enqueued(c, nsteps);
   c->steps_done += nsteps;
   return 0;
 }
@@ -1400,22 +1451,8 @@ int orion_step_async(orion_case_t c, int nsteps) {
   return 0;
 }
 
-// Reads the sweep barrier's error flag (the stream is idle).
-static int sweep_status(orion_case_t c) {
-  if (!c->L.sweep_ctl) return 0;
-  int ctl[2] = {0, 0};
-  CUDA_TRY(cudaMemcpy(ctl, c->L.sweep_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
-  if (ctl[1]) {
-    c->sweep_arrays = -1;  // edge records may hold increments nobody read
-    CUDA_TRY(cudaMemsetAsync(c->L.sweep_ctl, 0, sizeof(ctl), c->stream));
-    CUDA_TRY(cudaStreamSynchronize(c->stream));
-    return fail(ORION_E_TIMEOUT, "a bounded wait of the implicit sweeps (grid barrier or tile progress) gave up waiting");
-  }
-  return 0;
-}
-
-static int group_status(orion_group_t g) {
-  const int rc = sweep_status(g->proxy);
+static int group_status(orion_group_t g, long long sent) {
+  const int rc = sweep_status(g->proxy, sent);
   if (rc == ORION_E_TIMEOUT)
     for (auto c : g->members) c->sweep_arrays = -1;
   return rc;
@@ -1431,8 +1468,7 @@ int orion_step(orion_case_t c, int nsteps, orion_residual_t* hist) {
     const int n = std::min(nsteps - done, kHistCap);
     int rc = launch_steps(c, n);
     if (rc) return rc;
-    CUDA_TRY(cudaStreamSynchronize(c->stream));
-    rc = sweep_status(c);
+    rc = wait_checked(c);
     if (rc) return rc;
     if (hist) {
       rc = read_hist(c, (long long)cnt + done, n, hist + done);
@@ -1487,6 +1523,7 @@ static int enqueue_hist_copy(orion_case_t c, int nsteps, cudaStream_t st) {
 int orion_case_poll(orion_case_t c, orion_residual_t* out, int cap, int* n) {
   if (!c || !n || (cap > 0 && !out)) return fail(ORION_E_INVALID, "null argument");
   *n = 0;
+  const long long sent = (c->group ? c->group->proxy : c)->sweeps_sent;
   if (c->io) {  // pipelined I/O copies the history on the output copy stream
     const cudaError_t qo = cudaStreamQuery(c->io->out);
     if (qo == cudaErrorNotReady) return 0;
@@ -1501,7 +1538,7 @@ int orion_case_poll(orion_case_t c, orion_residual_t* out, int cap, int* n) {
     cudaGetLastError();
     return fail(ORION_E_CUDA, std::string("case stream: ") + cudaGetErrorString(q));
   }
-  int rc = c->group ? group_status(c->group) : sweep_status(c);
+  int rc = c->group ? group_status(c->group, sent) : sweep_status(c, sent);
   if (rc) return rc;
   const int take = std::min(cap, c->pending_n);
   for (int s = 0; s < take; ++s) {
@@ -1642,8 +1679,8 @@ extern "C" {
 int orion_last_residual(orion_case_t c, orion_residual_t* out) {
   if (!c || !out) return fail(ORION_E_INVALID, "null argument");
   int cnt = 0;
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
-  CUDA_TRY(cudaMemcpy(&cnt, c->L.counter, sizeof(int), cudaMemcpyDeviceToHost));
+  const int rc = wait_checked_counter(c, &cnt);
+  if (rc) return rc;
   if (cnt <= 0) return fail(ORION_E_INVALID, "no step has run");
   return read_hist(c, cnt - 1, 1, out);
 }
@@ -1743,8 +1780,7 @@ int orion_io_wait(orion_case_t c) {
     CUDA_TRY(cudaStreamSynchronize(c->io->in));
     CUDA_TRY(cudaStreamSynchronize(c->io->out));
   }
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
-  return sweep_status(c);
+  return wait_checked(c);
 }
 
 }  // extern "C"
@@ -2078,8 +2114,9 @@ int orion_group_submit(orion_group_t g, int nsteps) {
 
 int orion_group_sync(orion_group_t g) {
   if (!g) return fail(ORION_E_INVALID, "null group");
+  const long long sent = g->proxy->sweeps_sent;
   CUDA_TRY(cudaStreamSynchronize(g->proxy->stream));
-  return group_status(g);
+  return group_status(g, sent);
 }
 
 int orion_group_step_launches(orion_group_t g, int* n) {
@@ -2170,8 +2207,8 @@ int orion_shard_average_end(orion_case_t c) {
 int orion_shard_residual(orion_case_t c, orion_shard_residual_t* out) {
   if (!c || !out) return fail(ORION_E_INVALID, "null argument");
   int rc = dispatch(c, [&](const StageOps& o) { return o.residual(c); });
+  if (!rc) rc = wait_checked(c);
   if (rc) return rc;
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
   ResPartial t{};
   unsigned long long bits = 0;
   CUDA_TRY(cudaMemcpy(&t, c->L.res_total, sizeof(t), cudaMemcpyDeviceToHost));

@@ -6,12 +6,13 @@ read when a case is made).  With a limit of one poll the first CTA to arrive
 gives up at once: the kernel records the error and every CTA returns, the host
 reports ORION_E_TIMEOUT, and the context stays usable for the next case.
 """
+import ctypes as C
 import os
 
 import numpy as np
 import pytest
 
-from orion_b200 import _lib, cases, solver
+from orion_b200 import _lib, cases, output, shard, solver
 from orion_b200._lib import OrionError
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +62,80 @@ def test_tile_wavefront_wait_timeout_is_reported_and_the_context_survives():
     assert np.array_equal(a.step(3), b.step(3))
     a.close()
     b.close()
+
+
+def _limited(case, precision=_lib.PREC_FP64, make=solver.FlowFieldSet):
+    """A case whose device waits give up after one poll."""
+    os.environ["ORION_SWEEP_SPIN_LIMIT"] = "1"
+    try:
+        return make(case, precision=precision)
+    finally:
+        del os.environ["ORION_SWEEP_SPIN_LIMIT"]
+
+
+def _restart(fs):
+    _lib.check(_lib.load().orion_case_init_flow(fs.handle, fs.case.noise_seed, fs.case.noise_amp))
+
+
+def _stages(fs):
+    halo = solver.HaloExchanger()
+    halo.exchange_bc(None, fs)
+    solver.apply_physical_bc(None, fs)
+    solver.StateUpdater.update_flow_states(fs)
+    solver.TimeIntegrator.calculate_time_step(fs)
+    solver.FluxComputer.compute_viscous_rhs(fs)
+    halo.average_interface_residuals(None, fs)
+    solver.InviscidFluxComputer.compute_inviscid_rhs(fs)
+    halo.average_interface_residuals(None, fs)
+    solver.StateUpdater.update_solution(fs)
+
+
+def _phydtime(fs):
+    v = C.c_double()
+    _lib.check(_lib.load().orion_phydtime(fs.handle, C.byref(v)))
+
+
+# what hands out a result: how the steps were enqueued, the call that waits
+WAITS = {
+    "stages-residual": (_stages, lambda fs: solver.ResidualMonitor.compute(fs)),
+    "stages-download": (_stages, lambda fs: fs.download(0, "prim")),
+    "async-sync": (lambda fs: fs.step_async(1), lambda fs: fs.sync()),
+    "async-download": (lambda fs: fs.step_async(1), lambda fs: fs.download(0, "dq")),
+    "async-pack": (lambda fs: fs.step_async(1), lambda fs: output.pack_block(fs, 0)),
+    "async-last": (lambda fs: fs.step_async(1), lambda fs: fs.last_residual()),
+    "async-phydtime": (lambda fs: fs.step_async(1), _phydtime),
+}
+
+
+@pytest.mark.parametrize("precision", [_lib.PREC_FP64, _lib.PREC_MIXED], ids=["plain", "mixed"])
+@pytest.mark.parametrize("how", list(WAITS))
+def test_every_call_that_hands_out_a_result_reports_the_timeout(how, precision):
+    """Sweeps that gave up leave a state and a residual of no use: the first
+    call that waits for them says so, whichever it is, and the case steps on
+    from a new state."""
+    send, wait = WAITS[how]
+    case = cases.small_case("timeout_waits", dims=(33, 70, 25), noise_seed=5)
+    fs = _limited(case, precision)
+    send(fs)
+    with pytest.raises(OrionError, match="-6"):
+        wait(fs)
+    wait(fs)  # reported once
+    fs.set_schedule("planes", 0, 16)
+    _restart(fs)
+    ref = solver.FlowFieldSet(case, precision=precision)
+    ref.set_schedule("planes", 0, 16)
+    assert np.array_equal(fs.step(2), ref.step(2))
+    fs.close()
+    ref.close()
+
+
+def test_a_shard_reports_the_timeout_with_its_residual():
+    case = cases.small_case("timeout_shard", dims=(33, 141, 25), split=(1, 2, 1), noise_seed=5)
+    shards = [_limited(case, make=lambda c, precision, r=r: shard.Shard(c, [0, 1], r, precision=precision))
+              for r in range(2)]
+    try:
+        with pytest.raises(OrionError, match="-6"):
+            shard.ShardGroup(shards, shard.LocalTransport()).run(1)
+    finally:
+        for s in shards:
+            s.close()

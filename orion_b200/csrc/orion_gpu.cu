@@ -2051,6 +2051,7 @@ int orion_group_create(int n, const orion_case_t* cases, orion_group_t* out) {
   for (auto c : g->members) {
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     tiles = tiles && c->L.tiles_on;
+    px->L.spin_limit = std::min(px->L.spin_limit, c->L.spin_limit);  // the members' bound
   }
   px->L.tiles_on = tiles;  // otherwise one launch per hyperplane
   g->proxy = px.get();

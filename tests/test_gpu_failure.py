@@ -139,3 +139,24 @@ def test_a_shard_reports_the_timeout_with_its_residual():
     finally:
         for s in shards:
             s.close()
+
+
+GROUP = [dict(name="tg0", dims=(33, 70, 25), noise_seed=5), dict(name="tg1", dims=(25, 33, 61), noise_seed=6),
+         dict(name="tg2", dims=(33, 75, 23), split=(2, 1, 1), noise_seed=7)]
+
+
+def _group(limited=0):
+    """A group whose member `limited` bounds its waits by one poll; so does the group."""
+    members = [(_limited if m == limited else solver.FlowFieldSet)(cases.small_case(**sp)) for m, sp in enumerate(GROUP)]
+    return members, solver.CaseGroup(members)
+
+
+@pytest.mark.parametrize("limited", [0, 2])
+def test_a_group_takes_its_members_wait_limit(limited):
+    members, g = _group(limited)
+    g.submit(1)
+    with pytest.raises(OrionError, match="-6"):
+        g.sync()
+    g.close()
+    for fs in members:
+        fs.close()

@@ -291,7 +291,12 @@ int orion_io_wait(orion_case_t c);
  * the group before destroying or re-grouping its cases.
  * orion_group_submit enqueues nsteps group steps (one CUDA graph per step)
  * and each member's history copy, and returns at once; poll each member with
- * orion_case_poll.  orion_group_sync waits for the group's stream. */
+ * orion_case_poll.  orion_group_sync waits for the group's stream.  When the
+ * group's sweeps gave up waiting (ORION_E_TIMEOUT; the group takes its members'
+ * lowest limit), orion_group_sync and the next waiting call on every member
+ * report it, once each, also after the group was destroyed; a poll that does
+ * drops the unpolled history.  Submitting to the group after orion_group_sync
+ * reported it starts anew. */
 int orion_group_create(int n, const orion_case_t* cases, orion_group_t* out);
 int orion_group_submit(orion_group_t g, int nsteps);
 int orion_group_sync(orion_group_t g);

@@ -185,6 +185,7 @@ struct orion_case_s {
   // updates enqueued whose sweeps wait on the device (tile and grid forms), and
   // how many of them the error word has been read after (sweep_status)
   std::atomic<long long> sweeps_sent{0}, sweeps_read{0};
+  std::atomic<bool> group_failed{false};  // its group's sweeps gave up and the case has not reported it yet
   orion::ShardLists shard;
   long long total_interior = 0;
   cudaGraphExec_t graph = nullptr;
@@ -213,6 +214,8 @@ struct orion_group_s {
   orion_case_s* proxy = nullptr;
   orion::GroupRun run;
   std::vector<int> block_off;  // each member's first block in the group's descriptors
+  std::atomic<bool> failed{false};  // its sweeps gave up and orion_group_sync has not reported it yet
+  std::atomic<bool> told{false};    // orion_group_sync has, and no steps were submitted since
 };
 
 namespace orion {

@@ -1041,7 +1041,11 @@ int orion_case_get_schedule(orion_case_t c, orion_schedule_t* s) {
 }
 
 static int launch_steps(orion_case_t c, int nsteps);
-static int sweep_status(orion_case_t c, long long sent);
+struct SweepMark {
+  long long own, group;
+};
+static SweepMark sweep_mark(orion_case_t c);
+static int sweep_status(orion_case_t c, SweepMark m);
 static int wait_checked(orion_case_t c);
 static int enqueue_hist_copy(orion_case_t c, int nsteps, cudaStream_t st = nullptr);
 
@@ -1100,7 +1104,7 @@ int orion_case_autotune(orion_case_t c, int steps_per_trial, orion_schedule_t* t
     if ((r = launch_steps(c, steps_per_trial))) return r;
     CUDA_TRY(cudaEventRecord(e1, c->stream));
     CUDA_TRY(cudaEventSynchronize(e1));
-    if ((r = sweep_status(c, c->sweeps_sent))) return r;
+    if ((r = sweep_status(c, sweep_mark(c)))) return r;
     float ms = 0.f;
     CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
     if ((r = copy_state(false))) return r;
@@ -1355,42 +1359,78 @@ int orion_update_solution(orion_case_t c) {
   });
 }
 
-// An error word that was read (the stream is idle): a wait of the sweeps gave up.
-static int sweep_report(orion_case_t c, int word) {
-  if (!word) return 0;
-  c->sweep_arrays = -1;  // edge records may hold increments nobody read
-  CUDA_TRY(cudaMemsetAsync(c->L.sweep_ctl, 0, 2 * sizeof(int), c->stream));
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
-  return fail(ORION_E_TIMEOUT, "a bounded wait of the implicit sweeps (grid barrier or tile progress) gave up waiting");
+// Updates enqueued so far on the case's stream, its own and its group's; taken
+// before a wait, it names the updates the wait was for.
+static SweepMark sweep_mark(orion_case_t c) {
+  return SweepMark{c->sweeps_sent, c->group ? c->group->proxy->sweeps_sent.load() : 0};
 }
 
-// Reads the sweeps' error word when updates up to `sent` (c->sweeps_sent, taken
-// before the stream was found idle) have run since it was last read.
-static int sweep_status(orion_case_t c, long long sent) {
+// An error word that was read (the stream is idle), put back; the edge records
+// may hold increments nobody read.
+static int sweep_clear(orion_case_t c, int word) {
+  if (!word) return 0;
+  c->sweep_arrays = -1;
+  CUDA_TRY(cudaMemsetAsync(c->L.sweep_ctl, 0, 2 * sizeof(int), c->stream));
+  CUDA_TRY(cudaStreamSynchronize(c->stream));
+  return 0;
+}
+
+// Reads the sweeps' error word when updates up to `sent` have run since it was
+// last read.
+static int sweep_word(orion_case_t c, long long sent, int* word) {
+  *word = 0;
   if (c->sweeps_read >= sent) return 0;
   int ctl[2] = {0, 0};
   CUDA_TRY(cudaMemcpy(ctl, c->L.sweep_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
   c->sweeps_read = sent;
-  return sweep_report(c, ctl[1]);
+  *word = ctl[1];
+  return sweep_clear(c, ctl[1]);
 }
 
-// The wait of every call that hands out what the steps left: a state or a
-// residual after sweeps that gave up is an error there, once.
+static int gave_up() {
+  return fail(ORION_E_TIMEOUT, "a bounded wait of the implicit sweeps (grid barrier or tile progress) gave up waiting");
+}
+
+// The group's error word: whoever reads it, the group and every member have it
+// to report.
+static int group_word(orion_group_t g, long long sent) {
+  int word;
+  const int rc = sweep_word(g->proxy, sent, &word);
+  if (!word) return rc;
+  g->failed = true;
+  for (auto c : g->members) {
+    c->sweep_arrays = -1;
+    c->group_failed = true;
+  }
+  return rc;
+}
+
+// Reports sweeps that gave up, once, as far as they were enqueued at the mark
+// (the stream was found idle since).
+static int sweep_status(orion_case_t c, SweepMark m) {
+  int word, rc = sweep_word(c, m.own, &word);
+  if (!rc && c->group) rc = group_word(c->group, m.group);
+  const bool grouped = c->group_failed.exchange(false);
+  return rc ? rc : (word || grouped ? gave_up() : 0);
+}
+
+// The wait of every call that hands out what the steps left.
 static int wait_checked(orion_case_t c) {
-  const long long sent = c->sweeps_sent;
+  const SweepMark m = sweep_mark(c);
   CUDA_TRY(cudaStreamSynchronize(c->stream));
-  return sweep_status(c, sent);
+  return sweep_status(c, m);
 }
 
 // The same with the history counter, in one copy.
 static int wait_checked_counter(orion_case_t c, int* cnt) {
-  const long long sent = c->sweeps_sent;
+  const SweepMark m = sweep_mark(c);
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   int ctl[3] = {0, 0, 0};
   CUDA_TRY(cudaMemcpy(ctl, c->L.sweep_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
-  c->sweeps_read = sent;
+  c->sweeps_read = m.own;
   *cnt = ctl[2];
-  return sweep_report(c, ctl[1]);
+  const int rc = sweep_clear(c, ctl[1]), other = sweep_status(c, m);
+  return rc ? rc : (ctl[1] ? gave_up() : other);
 }
 
 static int read_hist(orion_case_t c, long long first, int n, orion_residual_t* out) {
@@ -1449,13 +1489,6 @@ int orion_step_async(orion_case_t c, int nsteps) {
   if (rc) return rc;
   if (c->hist_count >= 0) c->hist_count += nsteps;
   return 0;
-}
-
-static int group_status(orion_group_t g, long long sent) {
-  const int rc = sweep_status(g->proxy, sent);
-  if (rc == ORION_E_TIMEOUT)
-    for (auto c : g->members) c->sweep_arrays = -1;
-  return rc;
 }
 
 int orion_step(orion_case_t c, int nsteps, orion_residual_t* hist) {
@@ -1523,7 +1556,7 @@ static int enqueue_hist_copy(orion_case_t c, int nsteps, cudaStream_t st) {
 int orion_case_poll(orion_case_t c, orion_residual_t* out, int cap, int* n) {
   if (!c || !n || (cap > 0 && !out)) return fail(ORION_E_INVALID, "null argument");
   *n = 0;
-  const long long sent = (c->group ? c->group->proxy : c)->sweeps_sent;
+  const SweepMark m = sweep_mark(c);
   if (c->io) {  // pipelined I/O copies the history on the output copy stream
     const cudaError_t qo = cudaStreamQuery(c->io->out);
     if (qo == cudaErrorNotReady) return 0;
@@ -1538,7 +1571,8 @@ int orion_case_poll(orion_case_t c, orion_residual_t* out, int cap, int* n) {
     cudaGetLastError();
     return fail(ORION_E_CUDA, std::string("case stream: ") + cudaGetErrorString(q));
   }
-  int rc = c->group ? group_status(c->group, sent) : sweep_status(c, sent);
+  const int rc = sweep_status(c, m);
+  if (rc == ORION_E_TIMEOUT) c->pending_n = 0;  // the history of sweeps that gave up is not given out
   if (rc) return rc;
   const int take = std::min(cap, c->pending_n);
   for (int s = 0; s < take; ++s) {
@@ -2079,6 +2113,7 @@ int orion_group_destroy(orion_group_t g) {
   if (!g) return 0;
   std::lock_guard<std::mutex> lk(g_struct_mu);
   cudaStreamSynchronize(g->proxy->stream);
+  group_word(g, g->proxy->sweeps_sent);  // the members report what nobody asked for
   for (size_t m = 0; m < g->members.size(); ++m) {
     g->members[m]->stream = g->saved_streams[m];
     g->members[m]->group = nullptr;
@@ -2090,6 +2125,14 @@ int orion_group_destroy(orion_group_t g) {
 
 int orion_group_submit(orion_group_t g, int nsteps) {
   if (!g || nsteps < 0) return fail(ORION_E_INVALID, "bad arguments");
+  // Steps after orion_group_sync told of sweeps that gave up start anew: what
+  // members still had to say of them would be taken for the new steps'.
+  if (g->told.exchange(false))
+    for (auto c : g->members)
+      if (c->group_failed.exchange(false)) c->pending_n = 0;
+  // likewise the group's own report once every member has made its
+  if (g->failed && std::none_of(g->members.begin(), g->members.end(), [](orion_case_t c) { return c->group_failed.load(); }))
+    g->failed = false;
   for (auto c : g->members) {
     if (c->pending_n + nsteps > kHistCap)
       return fail(ORION_E_INVALID, "more unpolled steps than the history ring holds (4096)");
@@ -2117,7 +2160,10 @@ int orion_group_sync(orion_group_t g) {
   if (!g) return fail(ORION_E_INVALID, "null group");
   const long long sent = g->proxy->sweeps_sent;
   CUDA_TRY(cudaStreamSynchronize(g->proxy->stream));
-  return group_status(g, sent);
+  const int rc = group_word(g, sent);
+  if (rc || !g->failed.exchange(false)) return rc;
+  g->told = true;
+  return gave_up();
 }
 
 int orion_group_step_launches(orion_group_t g, int* n) {

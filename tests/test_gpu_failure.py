@@ -160,3 +160,59 @@ def test_a_group_takes_its_members_wait_limit(limited):
     g.close()
     for fs in members:
         fs.close()
+
+
+def _poll(fs):
+    while True:
+        h = fs.poll()
+        if h is not None:
+            return h
+
+
+def _steps_like_a_new_case(fs):
+    """In the tile form: the edge records that the group's sweeps left are gone."""
+    _restart(fs)
+    ref = solver.FlowFieldSet(fs.case)
+    assert np.array_equal(fs.step(2), ref.step(2))
+    ref.close()
+
+
+@pytest.mark.parametrize("ask", ["poll", "sync", "download", "destroyed"])
+def test_every_member_of_a_group_reports_the_timeout(ask):
+    members, g = _group(limited=1)
+    g.submit(1)
+    if ask == "sync":
+        with pytest.raises(OrionError, match="-6"):
+            g.sync()
+        g.sync()  # reported once
+    if ask == "destroyed":
+        g.close()
+    for fs in members:
+        with pytest.raises(OrionError, match="-6"):
+            _poll(fs) if ask == "poll" else fs.download(0, "prim")
+    for fs in members:
+        if ask == "poll":
+            assert len(_poll(fs)) == 0  # nor is that history given out later
+        fs.sync()
+    g.close()
+    for m, fs in enumerate(members):
+        if m != 1:  # this one still gives up after one poll
+            _steps_like_a_new_case(fs)
+        fs.close()
+
+
+def test_a_group_that_told_its_timeout_starts_anew():
+    members, g = _group()
+    for _ in range(2):  # the second round's reports are its own
+        g.submit(1)
+        with pytest.raises(OrionError, match="-6"):
+            g.sync()
+    for fs in members:
+        with pytest.raises(OrionError, match="-6"):
+            _poll(fs)
+        assert len(_poll(fs)) == 0
+    g.submit(0)
+    g.sync()
+    g.close()
+    for fs in members:
+        fs.close()

@@ -19,21 +19,25 @@ template <> __device__ __forceinline__ double tsqrt<double>(double x) { return s
 template <> __device__ __forceinline__ float tsqrt<float>(float x) { return sqrtf(x); }
 template <typename T> __device__ __forceinline__ T tmax(T a, T b) { return (a < b) ? b : a; }  // std::max
 
-// a / b, correctly rounded, from r = RN(1/b): two Newton corrections of the
-// quotient with an exact remainder (Markstein, IBM J. Res. Dev. 34, 1990: with
-// r correctly rounded and q within one ulp, RN(q + r (a - b q)) = RN(a / b)).
+// a / b, correctly rounded, from r = RN(1/b), b > 0: two Newton corrections of
+// the quotient with an exact remainder (Markstein, IBM J. Res. Dev. 34, 1990:
+// with r correctly rounded and q within one ulp, RN(q + r (a - b q)) = RN(a / b)).
 // The first correction brings q = RN(a r) within one ulp, the second is the
-// theorem's step.  Exact while a remainder stays normal: quotient_rcp gives 0,
-// and quotient 0, for a denominator beyond 1e+-290.  Where the corrections meet
-// an infinity (an infinite or zero denominator, an infinite quotient) they end
-// in a NaN, and the product a r is what the division gives; the test is on the
-// high word, off the FP64 pipe.
+// theorem's step.  The remainder is formed as b q - a and subtracted, so that a
+// zero keeps its sign.  Exact while the remainder and 1/b are normal numbers
+// (|a| from 2^-959, b from 2^-1021 to 2^1021) and the quotient is one or zero;
+// below that the last bit may differ, and a b whose reciprocal overflows gives
+// an infinity.  Where the corrections meet an infinity (an infinite or zero
+// denominator, an infinite quotient) they end in a NaN, and the product a r is
+// what the division gives; the test is on the high word, off the FP64 pipe.
 __device__ __forceinline__ double quotient(double a, double b, double r) {
   const double q0 = a * r;
-  const double q1 = __fma_rn(__fma_rn(-b, q0, a), r, q0);
-  const double q2 = __fma_rn(__fma_rn(-b, q1, a), r, q1);
+  const double q1 = __fma_rn(-__fma_rn(b, q0, -a), r, q0);
+  const double q2 = __fma_rn(-__fma_rn(b, q1, -a), r, q1);
   return (__double2hiint(q2) & 0x7ff00000) == 0x7ff00000 ? q0 : q2;
 }
+// 0, and so quotient 0, for a denominator outside 1e-290 .. 1e290 (a sound speed
+// no flow has).
 __device__ __forceinline__ double quotient_rcp(double b) {
   return (b > 1.0e-290 && b < 1.0e290) ? __drcp_rn(b) : 0.0;
 }

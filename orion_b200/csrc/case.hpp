@@ -67,7 +67,7 @@ struct DeviceLists {
   Chunk* sweep_chunks[2] = {nullptr, nullptr};  // forward / backward hyperplane launches
   std::vector<int> sweep_off[2];                 // host: chunk range of each launch
   int* sweep_off_dev[2] = {nullptr, nullptr};    // device copies of sweep_off
-  void* sweep_ctl = nullptr;                     // SweepCtl: grid barrier, error word of the sweeps' waits
+  void* sweep_ctl = nullptr;                     // SweepCtl: grid barrier, error of the sweeps' waits
   int persist_grid = 0;                          // CTAs of the persistent sweep kernel (0: per-plane launches)
   int sweep_nt = 256;                            // threads per sweep CTA = hyperplane chunk size
   // cluster sweeps: mesh blocks grouped per thread-block cluster
@@ -107,7 +107,7 @@ struct DeviceLists {
   int n_ap = 0;
   ResPartial* partials = nullptr;
   ResidualOut* hist = nullptr;
-  int* counter = nullptr;     // of the history; directly behind sweep_ctl, one copy reads both
+  int* counter = nullptr;
   unsigned long long* dtmin = nullptr;
   double* dt_part = nullptr;  // per-CTA minima of dt_phys
   long long* pad_base = nullptr;
@@ -182,9 +182,7 @@ struct orion_case_s {
   orion::DeviceLists L;
   // whose arrays the sweeps' shared memory holds: 1 the tile form's, 0 the plane-major ones, -1 neither
   std::atomic<int> sweep_arrays{-1};
-  // updates enqueued whose sweeps wait on the device (tile and grid forms), and
-  // how many of them the error word has been read after (sweep_status)
-  std::atomic<long long> sweeps_sent{0}, sweeps_read{0};
+  int* gave_up = nullptr;  // pinned: set by a device wait of the sweeps that gave up (SweepCtl::host)
   std::atomic<bool> group_failed{false};  // its group's sweeps gave up and the case has not reported it yet
   orion::ShardLists shard;
   long long total_interior = 0;

@@ -849,8 +849,15 @@ enum SweepMode { SW_LUSGS_FWD = 0, SW_LUSGS_BWD = 1, SW_GS = 2 };
 // reports ORION_E_TIMEOUT) instead of spinning forever.
 struct SweepCtl {
   unsigned int counter;
-  int error;
+  int error;   // a wait gave up: what the other waits look at
+  int* host;   // the same in the host's memory, read there after the work has finished: no copy on any path
 };
+
+__device__ __forceinline__ void sweep_gave_up(SweepCtl* ctl) {
+  atomicExch(&ctl->error, 1);
+  *(volatile int*)ctl->host = 1;
+  __threadfence_system();
+}
 
 __device__ __forceinline__ bool grid_barrier(SweepCtl* ctl, unsigned int target, long long spin_limit) {
   __syncthreads();
@@ -865,7 +872,7 @@ __device__ __forceinline__ bool grid_barrier(SweepCtl* ctl, unsigned int target,
       if (v >= target) break;
       if (*(volatile int*)&ctl->error) { abort = 1; break; }
       if (++it > spin_limit) {
-        atomicExch(&ctl->error, 1);
+        sweep_gave_up(ctl);
         abort = 1;
         break;
       }

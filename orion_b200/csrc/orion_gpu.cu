@@ -282,6 +282,42 @@ int orion::build_cluster_lists(orion_case_t c, int nclusters) {
 
 namespace {
 
+// Words in pinned host memory that the sweeps' waits report to, one a case,
+// from pages kept for the life of the process: pinning or unpinning memory per
+// case may synchronise the device under other cases.
+std::mutex g_word_mu;
+std::vector<int*> g_free_words;
+
+int* acquire_word() {
+  constexpr size_t kPage = 4096, kLine = 64;
+  std::lock_guard<std::mutex> lk(g_word_mu);
+  if (g_free_words.empty()) {
+    char* page = nullptr;
+    if (cudaHostAlloc((void**)&page, kPage, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    for (size_t o = 0; o < kPage; o += kLine) g_free_words.push_back(reinterpret_cast<int*>(page + o));
+  }
+  int* w = g_free_words.back();
+  g_free_words.pop_back();
+  *w = 0;
+  return w;
+}
+
+void release_word(int* w) {
+  std::lock_guard<std::mutex> lk(g_word_mu);
+  g_free_words.push_back(w);
+}
+
+int make_sweep_ctl(orion_case_t c) {
+  if (!(c->gave_up = acquire_word())) return fail(ORION_E_NOMEM, "pinned error word");
+  SweepCtl* ctl = nullptr;
+  const int rc = dev_upload(c, &ctl, std::vector<SweepCtl>{SweepCtl{0, 0, c->gave_up}});
+  c->L.sweep_ctl = ctl;
+  return rc;
+}
+
 // --------------------------------------------------------------------------
 // work-list builders
 // --------------------------------------------------------------------------
@@ -567,15 +603,11 @@ int build_lists(orion_case_t c, const std::vector<long long>& prim_off, const Ex
 
   if ((rc = dev_alloc(c, &L.partials, (size_t)L.n_int_chunks))) return rc;
   if ((rc = dev_alloc(c, &L.hist, (size_t)kHistCap))) return rc;
+  if ((rc = dev_alloc(c, &L.counter, 1))) return rc;
   if ((rc = dev_alloc(c, &L.dtmin, 1))) return rc;
   if ((rc = dev_alloc(c, &L.res_total, 1))) return rc;
   if ((rc = dev_alloc(c, &L.dt_part, (size_t)std::max(L.n_pad_chunks, L.n_int_chunks)))) return rc;
-  {
-    int* ctl = nullptr;
-    if ((rc = dev_alloc(c, &ctl, 4))) return rc;
-    L.sweep_ctl = ctl;
-    L.counter = ctl + 2;
-  }
+  if ((rc = make_sweep_ctl(c))) return rc;
   if ((rc = build_sweep_tiles(c))) return rc;
   return 0;
 }
@@ -637,6 +669,7 @@ void destroy_case(orion_case_t c) {
   if (c->d_blocks) cudaFreeAsync(c->d_blocks, c->stream);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   if (c->hist_host) release_hist_ring(c->hist_host);
+  if (c->gave_up) release_word(c->gave_up);
   delete c;
 }
 
@@ -674,12 +707,6 @@ static int use_sweep_arrays(orion_case_t c, bool tiles) {
   const int rc = ops_for(c->prec).sweep_arrays(c, tiles);
   if (rc) c->sweep_arrays = -1;
   return rc;
-}
-
-// n updates were enqueued: after the launches, so that whoever sees the count
-// and then waits for the stream has waited for them.
-static void sweeps_enqueued(orion_case_t c, int n) {
-  if (c->L.tiles_on || c->L.persist_grid > 0) c->sweeps_sent += n;
 }
 
 static int capture_step(orion_case_t c, cudaGraph_t* g) {
@@ -1041,11 +1068,7 @@ int orion_case_get_schedule(orion_case_t c, orion_schedule_t* s) {
 }
 
 static int launch_steps(orion_case_t c, int nsteps);
-struct SweepMark {
-  long long own, group;
-};
-static SweepMark sweep_mark(orion_case_t c);
-static int sweep_status(orion_case_t c, SweepMark m);
+static int sweep_status(orion_case_t c);
 static int wait_checked(orion_case_t c);
 static int enqueue_hist_copy(orion_case_t c, int nsteps, cudaStream_t st = nullptr);
 
@@ -1104,7 +1127,7 @@ int orion_case_autotune(orion_case_t c, int steps_per_trial, orion_schedule_t* t
     if ((r = launch_steps(c, steps_per_trial))) return r;
     CUDA_TRY(cudaEventRecord(e1, c->stream));
     CUDA_TRY(cudaEventSynchronize(e1));
-    if ((r = sweep_status(c, sweep_mark(c)))) return r;
+    if ((r = sweep_status(c))) return r;
     float ms = 0.f;
     CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
     if ((r = copy_state(false))) return r;
@@ -1226,16 +1249,15 @@ int orion_case_download(orion_case_t c, int block, int field, double* host) {
   int rc = field_info(c, block, field, &d, &nc, &st);
   if (rc) return rc;
   if (!host) return fail(ORION_E_INVALID, "null host pointer");
-  if ((rc = wait_checked(c))) return rc;
   const size_t n = (size_t)c->hb[block].npad * nc;
   if (st && c->prec != ORION_PREC_FP64) {
     std::vector<float> tmp(n);
     CUDA_TRY(cudaMemcpyAsync(tmp.data(), d, n * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-    CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if ((rc = wait_checked(c))) return rc;
     for (size_t i = 0; i < n; ++i) host[i] = (double)tmp[i];
   } else {
     CUDA_TRY(cudaMemcpyAsync(host, d, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if ((rc = wait_checked(c))) return rc;
   }
   return 0;
 }
@@ -1299,7 +1321,6 @@ int orion_case_pack_output(orion_case_t c, int block, float* host) {
     return fail(ORION_E_CUDA, "pack output: the case's stream is capturing");
   }
   std::lock_guard<std::mutex> lk(c->pack_mu);
-  if ((rc = wait_checked(c))) return rc;
   if (!c->pack_stage) {
     long long most = 0;
     for (const auto& b : c->hb) most = std::max(most, (long long)b.idim * b.jdim * b.kdim);
@@ -1316,7 +1337,7 @@ int orion_case_pack_output(orion_case_t c, int block, float* host) {
   if (e == cudaSuccess) e = cudaMemcpyAsync(host, stage, sizeof(float) * 7 * n, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return fail(ORION_E_CUDA, std::string("pack output: ") + cudaGetErrorString(e));
-  return 0;
+  return sweep_status(c);
 }
 
 int orion_case_init_flow(orion_case_t c, uint64_t seed, double amp) {
@@ -1352,51 +1373,31 @@ int orion_compute_inviscid_rhs(orion_case_t c) {
 }
 int orion_update_solution(orion_case_t c) {
   return dispatch(c, [&](const StageOps& o) {
-    int rc = use_sweep_arrays(c, c->L.tiles_on);
-    if (!rc) rc = o.update(c, false);
-    if (!rc) sweeps_enqueued(c, 1);
-    return rc;
+    const int rc = use_sweep_arrays(c, c->L.tiles_on);
+    return rc ? rc : o.update(c, false);
   });
 }
 
-// Updates enqueued so far on the case's stream, its own and its group's; taken
-// before a wait, it names the updates the wait was for.
-static SweepMark sweep_mark(orion_case_t c) {
-  return SweepMark{c->sweeps_sent, c->group ? c->group->proxy->sweeps_sent.load() : 0};
-}
-
-// An error word that was read (the stream is idle), put back; the edge records
-// may hold increments nobody read.
-static int sweep_clear(orion_case_t c, int word) {
-  if (!word) return 0;
+// Takes a report that device waits of the case's (or group's) sweeps gave up;
+// the edge records may then hold increments nobody read.
+static int take_report(orion_case_t c, bool* any) {
+  *any = __atomic_exchange_n(c->gave_up, 0, __ATOMIC_ACQ_REL) != 0;
+  if (!*any) return 0;
   c->sweep_arrays = -1;
-  CUDA_TRY(cudaMemsetAsync(c->L.sweep_ctl, 0, 2 * sizeof(int), c->stream));
+  CUDA_TRY(cudaMemsetAsync(c->L.sweep_ctl, 0, offsetof(SweepCtl, host), c->stream));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   return 0;
-}
-
-// Reads the sweeps' error word when updates up to `sent` have run since it was
-// last read.
-static int sweep_word(orion_case_t c, long long sent, int* word) {
-  *word = 0;
-  if (c->sweeps_read >= sent) return 0;
-  int ctl[2] = {0, 0};
-  CUDA_TRY(cudaMemcpy(ctl, c->L.sweep_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
-  c->sweeps_read = sent;
-  *word = ctl[1];
-  return sweep_clear(c, ctl[1]);
 }
 
 static int gave_up() {
   return fail(ORION_E_TIMEOUT, "a bounded wait of the implicit sweeps (grid barrier or tile progress) gave up waiting");
 }
 
-// The group's error word: whoever reads it, the group and every member have it
-// to report.
-static int group_word(orion_group_t g, long long sent) {
-  int word;
-  const int rc = sweep_word(g->proxy, sent, &word);
-  if (!word) return rc;
+// A group's report: whoever takes it, the group and every member have it to make.
+static int take_group_report(orion_group_t g) {
+  bool any;
+  const int rc = take_report(g->proxy, &any);
+  if (!any) return rc;
   g->failed = true;
   for (auto c : g->members) {
     c->sweep_arrays = -1;
@@ -1405,32 +1406,19 @@ static int group_word(orion_group_t g, long long sent) {
   return rc;
 }
 
-// Reports sweeps that gave up, once, as far as they were enqueued at the mark
-// (the stream was found idle since).
-static int sweep_status(orion_case_t c, SweepMark m) {
-  int word, rc = sweep_word(c, m.own, &word);
-  if (!rc && c->group) rc = group_word(c->group, m.group);
+// Reports sweeps that gave up, once (the stream is idle).
+static int sweep_status(orion_case_t c) {
+  bool own;
+  int rc = take_report(c, &own);
+  if (!rc && c->group) rc = take_group_report(c->group);
   const bool grouped = c->group_failed.exchange(false);
-  return rc ? rc : (word || grouped ? gave_up() : 0);
+  return rc ? rc : (own || grouped ? gave_up() : 0);
 }
 
 // The wait of every call that hands out what the steps left.
 static int wait_checked(orion_case_t c) {
-  const SweepMark m = sweep_mark(c);
   CUDA_TRY(cudaStreamSynchronize(c->stream));
-  return sweep_status(c, m);
-}
-
-// The same with the history counter, in one copy.
-static int wait_checked_counter(orion_case_t c, int* cnt) {
-  const SweepMark m = sweep_mark(c);
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
-  int ctl[3] = {0, 0, 0};
-  CUDA_TRY(cudaMemcpy(ctl, c->L.sweep_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
-  c->sweeps_read = m.own;
-  *cnt = ctl[2];
-  const int rc = sweep_clear(c, ctl[1]), other = sweep_status(c, m);
-  return rc ? rc : (ctl[1] ? gave_up() : other);
+  return sweep_status(c);
 }
 
 static int read_hist(orion_case_t c, long long first, int n, orion_residual_t* out) {
@@ -1452,8 +1440,10 @@ int orion_residual_compute(orion_case_t c, orion_residual_t* out) {
   if (!c || !out) return fail(ORION_E_INVALID, "null argument");
   if (c->shard.nranks > 1) return fail(ORION_E_INVALID, "a shard's residual is orion_shard_residual, reduced over the shards");
   int cnt = 0;
-  int rc = wait_checked_counter(c, &cnt);
-  if (!rc) rc = dispatch(c, [&](const StageOps& o) { return o.residual(c); });
+  int rc = wait_checked(c);
+  if (rc) return rc;
+  CUDA_TRY(cudaMemcpy(&cnt, c->L.counter, sizeof(int), cudaMemcpyDeviceToHost));
+  rc = dispatch(c, [&](const StageOps& o) { return o.residual(c); });
   if (rc) return rc;
   c->hist_count = cnt + 1;
   return read_hist(c, cnt, 1, out);
@@ -1478,7 +1468,6 @@ static int launch_steps(orion_case_t c, int nsteps) {
   if (!rc && !c->L.group) rc = use_sweep_arrays(c, c->L.tiles_on);  // a group's: its members' (orion_group_submit)
   if (rc) return rc;
   for (int s = 0; s < nsteps; ++s) CUDA_TRY(cudaGraphLaunch(c->graph, c->stream));
-  sweeps_enqueued(c, nsteps);
   c->steps_done += nsteps;
   return 0;
 }
@@ -1556,7 +1545,6 @@ static int enqueue_hist_copy(orion_case_t c, int nsteps, cudaStream_t st) {
 int orion_case_poll(orion_case_t c, orion_residual_t* out, int cap, int* n) {
   if (!c || !n || (cap > 0 && !out)) return fail(ORION_E_INVALID, "null argument");
   *n = 0;
-  const SweepMark m = sweep_mark(c);
   if (c->io) {  // pipelined I/O copies the history on the output copy stream
     const cudaError_t qo = cudaStreamQuery(c->io->out);
     if (qo == cudaErrorNotReady) return 0;
@@ -1571,7 +1559,7 @@ int orion_case_poll(orion_case_t c, orion_residual_t* out, int cap, int* n) {
     cudaGetLastError();
     return fail(ORION_E_CUDA, std::string("case stream: ") + cudaGetErrorString(q));
   }
-  const int rc = sweep_status(c, m);
+  const int rc = sweep_status(c);
   if (rc == ORION_E_TIMEOUT) c->pending_n = 0;  // the history of sweeps that gave up is not given out
   if (rc) return rc;
   const int take = std::min(cap, c->pending_n);
@@ -1713,8 +1701,9 @@ extern "C" {
 int orion_last_residual(orion_case_t c, orion_residual_t* out) {
   if (!c || !out) return fail(ORION_E_INVALID, "null argument");
   int cnt = 0;
-  const int rc = wait_checked_counter(c, &cnt);
+  const int rc = wait_checked(c);
   if (rc) return rc;
+  CUDA_TRY(cudaMemcpy(&cnt, c->L.counter, sizeof(int), cudaMemcpyDeviceToHost));
   if (cnt <= 0) return fail(ORION_E_INVALID, "no step has run");
   return read_hist(c, cnt - 1, 1, out);
 }
@@ -2040,9 +2029,7 @@ int build_group(orion_group_t g, orion_case_t px) {
     L.tile_rows = rows;
     L.n_tile_rows = (int)trows.size();
     L.tile_ctl = ctl;
-    int* sctl = nullptr;
-    if ((rc = dev_alloc(px, &sctl, 4))) return rc;
-    L.sweep_ctl = sctl;
+    if ((rc = make_sweep_ctl(px))) return rc;
   }
   if ((rc = dev_alloc(px, &L.partials, (size_t)std::max(L.n_int_chunks, 1)))) return rc;
   if ((rc = dev_alloc(px, &L.dt_part, (size_t)std::max(L.n_pad_chunks, 1)))) return rc;
@@ -2113,7 +2100,7 @@ int orion_group_destroy(orion_group_t g) {
   if (!g) return 0;
   std::lock_guard<std::mutex> lk(g_struct_mu);
   cudaStreamSynchronize(g->proxy->stream);
-  group_word(g, g->proxy->sweeps_sent);  // the members report what nobody asked for
+  take_group_report(g);  // the members report what nobody asked for
   for (size_t m = 0; m < g->members.size(); ++m) {
     g->members[m]->stream = g->saved_streams[m];
     g->members[m]->group = nullptr;
@@ -2158,9 +2145,8 @@ int orion_group_submit(orion_group_t g, int nsteps) {
 
 int orion_group_sync(orion_group_t g) {
   if (!g) return fail(ORION_E_INVALID, "null group");
-  const long long sent = g->proxy->sweeps_sent;
   CUDA_TRY(cudaStreamSynchronize(g->proxy->stream));
-  const int rc = group_word(g, sent);
+  const int rc = take_group_report(g);
   if (rc || !g->failed.exchange(false)) return rc;
   g->told = true;
   return gave_up();

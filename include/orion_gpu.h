@@ -155,7 +155,9 @@ int orion_case_step_launches(orion_case_t c, int* n);
  * wavefront), out[1] = CTAs (grid), clusters or forward tiles, out[2] = CTAs per cluster, out[3] = threads
  * per CTA, out[4] = hyperplanes of the longest sweep.  Waits for set-up only. */
 int orion_case_sweep_schedule(orion_case_t c, int out[5]);
-/* Device bytes held by the case (the HBM footprint used for admission). */
+/* Device bytes held by the case's fields, operands and packed output's staging;
+ * the estimate (the HBM footprint used for admission) is the most they come to,
+ * with the work lists. */
 int orion_case_footprint(orion_case_t c, size_t* bytes);
 size_t orion_footprint_estimate(int nblocks, const orion_block_desc_t* blocks, int precision);
 

@@ -200,6 +200,7 @@ struct orion_case_s {
   std::unordered_map<const void*, std::vector<unsigned char>> list_mirror;
   IoPipe* io = nullptr;  // orion_io_*, made on first use
   float* pack_stage = nullptr;  // orion_case_pack_output, made on first use
+  std::atomic<size_t> pack_bytes{0};  // its size
   std::mutex pack_mu;           // of pack_stage
 };
 

@@ -56,6 +56,14 @@ int dev_alloc(orion_case_t c, T** dptr, size_t n) {
   return 0;
 }
 
+// The packed output's staging: seven floats a point of the largest block.
+constexpr size_t kPackBytes = 7 * sizeof(float);
+size_t pack_stage_bytes(orion_case_t c) {
+  size_t most = 0;
+  for (const auto& b : c->hb) most = std::max(most, (size_t)b.idim * b.jdim * b.kdim);
+  return kPackBytes * most;
+}
+
 // Bytes of one block's fields for storage size ssz.
 size_t block_bytes(const HostBlock& b, size_t ssz, int tile_lines) {
   const size_t np = (size_t)b.npad;
@@ -934,7 +942,7 @@ int orion_gpu_init(int device) {
 size_t orion_footprint_estimate(int nblocks, const orion_block_desc_t* blocks, int precision) {
   if (nblocks <= 0 || !blocks) return 0;
   const size_t ssz = precision == ORION_PREC_FP64 ? 8 : 4;
-  size_t s = 0;
+  size_t s = 0, most = 0;
   long long lines = 0;
   for (int b = 0; b < nblocks; ++b) lines += (long long)blocks[b].jdim * blocks[b].kdim;
   const int tile_lines = tile_max_lines(ssz, lines <= kTileSmallCase);
@@ -948,8 +956,10 @@ size_t orion_footprint_estimate(int nblocks, const orion_block_desc_t* blocks, i
     h.nz = h.kdim + 2 * NG;
     h.npad = (long long)h.nx * h.ny * h.nz;
     s += block_bytes(h, ssz, tile_lines);
+    most = std::max(most, (size_t)h.idim * h.jdim * h.kdim);
   }
-  return s + (s / 64);  // work lists and buffers are a small fraction
+  // work lists and buffers are a small fraction; the packed output's staging is kept from its first call on
+  return s + (s / 64) + kPackBytes * most;
 }
 
 int orion_case_create(int nblocks, const orion_block_desc_t* blocks, const orion_params_t* params, int precision,
@@ -1206,7 +1216,7 @@ int orion_case_sweep_schedule(orion_case_t c, int out[5]) {
 
 int orion_case_footprint(orion_case_t c, size_t* bytes) {
   if (!c || !bytes) return fail(ORION_E_INVALID, "null argument");
-  *bytes = c->arena_bytes;
+  *bytes = c->arena_bytes + c->pack_bytes;
   return 0;
 }
 
@@ -1322,13 +1332,12 @@ int orion_case_pack_output(orion_case_t c, int block, float* host) {
   }
   std::lock_guard<std::mutex> lk(c->pack_mu);
   if (!c->pack_stage) {
-    long long most = 0;
-    for (const auto& b : c->hb) most = std::max(most, (long long)b.idim * b.jdim * b.kdim);
-    if (cudaMallocAsync((void**)&c->pack_stage, sizeof(float) * 7 * most, c->stream) != cudaSuccess) {
+    if (cudaMallocAsync((void**)&c->pack_stage, pack_stage_bytes(c), c->stream) != cudaSuccess) {
       cudaGetLastError();
       c->pack_stage = nullptr;
       return fail(ORION_E_NOMEM, "output staging buffer");
     }
+    c->pack_bytes = pack_stage_bytes(c);
   }
   float* const stage = c->pack_stage;
   out::k_pack_output<<<148 * 4, kThreads, 0, c->stream>>>(static_cast<const double*>(dprim), h.npad, h.idim, h.jdim,

@@ -42,3 +42,17 @@ def test_a_capturing_stream_is_refused():
     del g
     assert np.isfinite(output.pack_block(fs, 0)).all()
     fs.close()
+
+
+@pytest.mark.parametrize("split", [(1, 1, 1), (2, 1, 1)])
+@pytest.mark.parametrize("precision", [_lib.PREC_FP64, _lib.PREC_MIXED], ids=["plain", "mixed"])
+def test_the_footprint_counts_the_staging_buffer(precision, split):
+    case = cases.small_case("pack_fp", dims=(49, 45, 41), split=split, noise_seed=3)
+    fs = solver.FlowFieldSet(case, precision=precision)
+    before = fs.footprint()
+    for b in range(len(case.blocks)):
+        output.pack_block(fs, b)
+    assert fs.footprint() == before + 28 * max(int(np.prod(b.dims)) for b in case.blocks)
+    # the work lists too: 1/64 of the arena
+    assert solver.footprint_estimate(case, precision) >= fs.footprint() + before // 64
+    fs.close()

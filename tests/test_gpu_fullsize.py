@@ -77,3 +77,15 @@ def test_mixed_c3_tracks_plain(c3):
     assert (num / den) ** 0.5 <= 1e-6
     fm.close()
     fp.close()
+
+
+def test_plain_c3_tiles_match_the_hyperplane_launches(c3):
+    runs = []
+    for form in ("planes", "tiles"):
+        fs = solver.FlowFieldSet(c3, precision=_lib.PREC_FP64)
+        fs.set_schedule(form, 0, 32)
+        h = fs.step(STEPS)
+        runs.append((h, [fs.download(b, "prim") for b in range(0, len(c3.blocks), 5)]))
+        fs.close()
+    assert np.array_equal(runs[0][0], runs[1][0])
+    assert all(np.array_equal(a, b) for a, b in zip(runs[0][1], runs[1][1]))

@@ -47,3 +47,37 @@ def test_switching_forms_keeps_the_arrays_apart():
         got.append(fs.step(1))
     fs.close()
     assert np.array_equal(np.vstack(got), ref)
+
+
+# More than 9,472 lines, the least that FP64 cases take tiles of up to 96 lines for
+LARGE = [((25, 131, 97), (1, 1, 1), 1), ((17, 140, 143), (1, 2, 3), 0), ((13, 12, 797), (1, 1, 1), 1)]
+
+
+@pytest.mark.parametrize("dims,split,nvis", LARGE, ids=["x".join(map(str, s[0])) for s in LARGE])
+def test_large_tiles_match_the_hyperplane_launches(dims, split, nvis):
+    case = cases.small_case("tiles_large", dims=dims, split=split, uneven_seed=3 if max(split) > 1 else None,
+                            noise_seed=3, moo=0.7, nvis=nvis)
+    assert sum(b.jdim * b.kdim for b in case.blocks) > 9472
+    a, b = (_run(case, _lib.PREC_FP64, s) for s in ("planes", "tiles"))
+    assert np.array_equal(a[0], b[0])
+    assert all(np.array_equal(x, y) for x, y in zip(a[1], b[1]))
+
+
+@pytest.mark.parametrize("precision", [_lib.PREC_FP64, _lib.PREC_MIXED], ids=["plain", "mixed"])
+def test_a_group_of_small_and_large_tiles_steps_as_its_members_alone(precision):
+    """Plain: members of 64-line tiles run in the launch of the 96-line ones."""
+    specs = [dict(name="tl", dims=(25, 131, 97), noise_seed=3), dict(name="ts", dims=(33, 25, 23), split=(2, 1, 1), noise_seed=4),
+             dict(name="to", dims=(13, 47, 12), noise_seed=5, moo=0.7)]
+    sets = [solver.FlowFieldSet(cases.small_case(**sp), precision=precision) for sp in specs]
+    alone = []
+    for sp in specs:
+        fs = solver.FlowFieldSet(cases.small_case(**sp), precision=precision)
+        alone.append((fs.step(3), [fs.download(b, "prim") for b in range(len(fs.case.blocks))]))
+        fs.close()
+    g = solver.CaseGroup(sets)
+    hists = g.step(3)
+    g.close()
+    for (h, st), hg, fs in zip(alone, hists, sets):
+        assert np.array_equal(h, hg)
+        assert all(np.array_equal(x, fs.download(b, "prim")) for b, x in enumerate(st))
+        fs.close()

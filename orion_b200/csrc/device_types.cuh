@@ -107,14 +107,6 @@ struct RegionDev {
   int is2d;     // symmetry in a k-thin block
 };
 
-// Wavefront plane work: for plane s of a block, jj,kk of the line set.
-struct PlaneChunk {
-  int block;
-  int start;  // first (jj + nj*kk) index
-  int count;
-  int pad;
-};
-
 // Residual partial of one CTA.
 struct ResPartial {
   double sum;

@@ -640,21 +640,6 @@ __global__ void k_iface_apply(const BlockDev<S>* __restrict__ blocks, const int*
 // upper ones reproduces the lexicographic sweeps exactly; the hyperplane order
 // does, and each hyperplane is a contiguous, coalesced range here.
 // ===========================================================================
-template <typename S>
-__device__ __forceinline__ int jlo_of(const BlockDev<S>& B, int s, int kk) {
-  const int v = s - kk - (B.ni - 1);
-  return v > 0 ? v : 0;
-}
-
-template <typename S>
-__device__ __forceinline__ void decode_nat(const BlockDev<S>& B, int nat, int& ii, int& jj, int& kk) {
-  const int i = nat % B.nx;
-  const int r = nat / B.nx;
-  ii = i - NG;
-  jj = r % B.ny - NG;
-  kk = r / B.ny - NG;
-}
-
 __device__ __forceinline__ double sqrt_s(double x) { return sqrt(x); }
 __device__ __forceinline__ float sqrt_s(float x) { return sqrtf(x); }
 

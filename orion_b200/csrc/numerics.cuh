@@ -160,8 +160,7 @@ __device__ __forceinline__ T flux_diff_at(F f, int t, int ni) {
 }
 
 // ---------------------------------------------------------------------------
-// Spectral radii and flux splitting of the implicit sweeps
-// (src/solver/StateUpdater.cpp:175-265).
+// Spectral radii of the implicit sweeps (src/solver/StateUpdater.cpp:175-215).
 // ---------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ T spectral_radius(T rho, T u, T v, T w, T p, T gamma, T kx, T ky, T kz) {
@@ -181,47 +180,6 @@ __device__ __forceinline__ T visc_spectral_radius(T rho, T mu, T vol, T reynolds
   const T rm_vol = rho * vol;
   const T coef = T(2) * mu / (tabs(reynolds) * rm_vol + T(1.0e-30));
   return coef * grad2;
-}
-
-// compute_flux_splitting with nt = 0; sign is +1 or -1.
-template <typename T>
-__device__ __forceinline__ void flux_split(const T prim[5], const T dq[5], T nx, T ny, T nz, T r, T sign,
-                                           T gamma, T out[5]) {
-  T rm = prim[0];
-  const T um = prim[1], vm = prim[2], wm = prim[3];
-  T pm = prim[4];
-  const T drm = dq[0], dum = dq[1], dvm = dq[2], dwm = dq[3], dEm = dq[4];
-  const T nt = T(0);
-  const T v2 = um * um + vm * vm + wm * wm;
-  if (rm < T(1e-30)) rm = T(1e-30);
-  if (pm < T(1e-30)) pm = T(1e-30);
-  const T c2 = gamma * pm / rm;
-  const T cm = tsqrt(c2);
-  const T H = (gamma / (gamma - T(1))) * (pm / rm) + T(0.5) * v2;
-  const T ct = nx * um + ny * vm + nz * wm + nt;
-  T grad_mag = tsqrt(nx * nx + ny * ny + nz * nz);
-  if (grad_mag < T(1.0e-30)) grad_mag = T(1.0e-30);
-  T l1 = ct;
-  T l4 = ct + cm * grad_mag;
-  T l5 = ct - cm * grad_mag;
-  l1 = T(0.5) * (l1 + sign * r);
-  l4 = T(0.5) * (l4 + sign * r);
-  l5 = T(0.5) * (l5 + sign * r);
-  const T x1 = (T(2) * l1 - l4 - l5) / (T(2) * c2);
-  const T x2 = (l4 - l5) / (T(2) * cm);
-  const T inv_mag = T(1) / grad_mag;
-  const T nx_n = nx * inv_mag, ny_n = ny * inv_mag, nz_n = nz * inv_mag;
-  const T ct_n = (ct - nt) * inv_mag;
-  const T gm1 = gamma - T(1);
-  const T af = T(0.5) * gm1 * v2;
-  const T dc = ct_n * drm - (nx_n * dum + ny_n * dvm + nz_n * dwm);
-  const T dh = af * drm - gm1 * (um * dum + vm * dvm + wm * dwm - dEm);
-  const T c2dc = c2 * dc;
-  out[0] = l1 * drm - dh * x1 - dc * x2;
-  out[1] = l1 * dum + (nx_n * c2dc - um * dh) * x1 + (nx_n * dh - um * dc) * x2;
-  out[2] = l1 * dvm + (ny_n * c2dc - vm * dh) * x1 + (ny_n * dh - vm * dc) * x2;
-  out[3] = l1 * dwm + (nz_n * c2dc - wm * dh) * x1 + (nz_n * dh - wm * dc) * x2;
-  out[4] = l1 * dEm + (ct_n * c2dc - H * dh) * x1 + (ct_n * dh - H * dc) * x2;
 }
 
 }  // namespace orion

@@ -363,7 +363,7 @@ struct Stages {
     auto launch = [&](auto kernel, int tt) {
       kernel<<<n, tt * (MODE == SW_GS && TileLayout<T>::split ? 2 : 1) + 64, smem, c->stream>>>(
           blocks(c), static_cast<const SweepTile*>(L.sweep_tiles[d]), n, L.tile_lines,
-          static_cast<TileCtl*>(L.tile_ctl), sc, L.spin_limit);
+          static_cast<TileCtl*>(L.tile_ctl), &sc->error, L.spin_limit);
     };
     if (L.tile_small) launch(k_sweep_tiles<S, T, MODE, DIR, tile_threads(true)>, tile_threads(true));
     else launch(k_sweep_tiles<S, T, MODE, DIR, tile_threads(false)>, tile_threads(false));

@@ -196,10 +196,10 @@ __device__ __forceinline__ bool mbar_try(unsigned m, unsigned parity) {
   return ok != 0;
 }
 // A copy of this CTA's own always arrives; the bound is there all the same.
-__device__ __forceinline__ void mbar_wait(unsigned m, unsigned parity, SweepCtl* sc) {
+__device__ __forceinline__ void mbar_wait(unsigned m, unsigned parity, int* err) {
   for (int it = 0; !mbar_try(m, parity); ++it)
     if (it > (1 << 24)) {
-      sweep_gave_up(sc);
+      sweep_gave_up(err);
       return;
     }
 }
@@ -409,7 +409,7 @@ struct TilePoint<double, MODE> {
 template <typename S, typename T, int MODE, int DIR, int TT>
 __global__ void __launch_bounds__(TT * (MODE == SW_GS && TileLayout<T>::split ? 2 : 1) + 64, TileLayout<T>::minb)
     k_sweep_tiles(const BlockDev<S>* __restrict__ blocks, const SweepTile* __restrict__ tiles, int ntiles, int lines,
-                  TileCtl* __restrict__ ctl, SweepCtl* __restrict__ sc, long long spin_limit) {
+                  TileCtl* __restrict__ ctl, int* __restrict__ err, long long spin_limit) {
   static_assert(sizeof(S) == sizeof(T), "the tile sweeps keep operands in their storage precision");
   using L = TileLayout<T>;
   using U = typename EdgeBits<T>::type;
@@ -499,14 +499,14 @@ __global__ void __launch_bounds__(TT * (MODE == SW_GS && TileLayout<T>::split ? 
       }
       pown = pown + oplane == own + (R - 1) * oplane ? own : pown + oplane;
     };
-    mbar_wait(full0, 0, sc);
+    mbar_wait(full0, 0, err);
     __syncthreads();
     if constexpr (SPLIT) {
       if (helper) {
         // step s: the terms of wave s's ahead neighbours (wave s + 1), read by
         // the other warps at step s, formed while they are at step s - 1
         for (int s = 0; s < nsteps; ++s) {
-          mbar_wait(full0 + 8 * ra, parity, sc);
+          mbar_wait(full0 + 8 * ra, parity, err);
           if ((unsigned)i < (unsigned)ni) {
             TilePoint<T, MODE> cur;
             cur.load(pown, nl, l, po);
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(TT * (MODE == SW_GS && TileLayout<T>::split ? 
     if (!helper) {
       if (SPLIT) __syncthreads();  // wave 0's ahead terms
       for (int t = 0; t < nsteps; ++t) {
-        mbar_wait(full0 + 8 * ra, parity, sc);
+        mbar_wait(full0 + 8 * ra, parity, err);
         if ((unsigned)i < (unsigned)ni) {
           const uint4* const fr = fresh + ((t + 1) & 1) * fplane;  // wave t-1's
           TilePoint<T, MODE> cur;
@@ -658,9 +658,9 @@ __global__ void __launch_bounds__(TT * (MODE == SW_GS && TileLayout<T>::split ? 
         long long it = 0;
         while (!dead && __any_sync(0xffffffffu, !full)) {
           bool stop = ++it > spin_limit;
-          if ((it & 31) == 0 && *(volatile int*)&sc->error) stop = true;
+          if ((it & 31) == 0 && *(volatile int*)err) stop = true;
           if (__any_sync(0xffffffffu, stop)) {
-            if (lane == 0) sweep_gave_up(sc);
+            if (lane == 0) sweep_gave_up(err);
             dead = true;
             break;
           }

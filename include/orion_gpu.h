@@ -152,8 +152,9 @@ int orion_case_stream(orion_case_t c, void** stream);
 int orion_case_step_launches(orion_case_t c, int* n);
 /* How the implicit sweeps are scheduled: out[0] = mode (0 one launch per
  * hyperplane, 1 persistent cooperative grid, 2 thread-block clusters, 3 tile
- * wavefront), out[1] = CTAs (grid), clusters or forward tiles, out[2] = CTAs per cluster, out[3] = threads
- * per CTA, out[4] = hyperplanes of the longest sweep.  Waits for set-up only. */
+ * wavefront), out[1] = CTAs (grid), clusters or forward tiles, out[2] = CTAs
+ * per cluster, out[3] = threads per CTA (tiles: grid lines per tile at most),
+ * out[4] = hyperplanes of the longest sweep.  Waits for set-up only. */
 int orion_case_sweep_schedule(orion_case_t c, int out[5]);
 /* Device bytes held by the case's fields, operands and packed output's staging;
  * the estimate (the HBM footprint used for admission) is the most they come to,

@@ -44,7 +44,9 @@ constexpr int kHistCap = 4096;      // residual history ring
 #define ORION_SWEEP_THREADS 128
 #endif
 constexpr int kSweepThreads = ORION_SWEEP_THREADS;
-constexpr size_t kLineBudget = 96 * 1024;  // five face values of the longest grid line a case may have
+// The longest grid line a case may have: five face values of it in 96 KB (2,456
+// points in FP64, 4,914 in FP32), refused beyond; no kernel holds a whole line.
+constexpr size_t kLineBudget = 96 * 1024;
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 

@@ -12,7 +12,10 @@
 //           rounds (:377-521), one thread each;
 //   output  the flux difference, or at the three points of a flagged end the
 //           rounds' sums, added to dq.
-// What bounds it: arithmetic (the FP64 pipe, and instruction issue in FP32).
+// What bounds it: the phases' latency.  Neither pipe is full (193x97x65: an
+// instruction issues in 57-62% of the cycles in FP32 and 42-46% in FP64, the
+// FP64 pipe works in 40-44%), and the first stall is the barrier between the
+// phases, with four (FP32) or three CTAs an SM to fill in for one another.
 // Each prim and metric value is read from global memory once per chunk into
 // shared memory (a face used to read 30 and 12, with their addresses).  A
 // chunk needs two or three faces more than points on each inner side, so lines

@@ -408,11 +408,10 @@ __device__ __forceinline__ void dtmin_final_body(const double* __restrict__ part
   }
 }
 
-// CTAs per SM (256 threads each) the sweep-preparation kernels are
-// compiled for (register cap 65536 / (256 n)), per precision.  Measured on C3
-// against the compiler's own choice (80-109 registers): FP32 six, FP64 four
-// (a few spilled registers each) took the mixed step from 16.7 to 15.9 ms and
-// the plain step from 32.7 to 31.7 ms.
+// CTAs per SM (256 threads each) the sweep-preparation kernels are compiled for
+// (register cap 65536 / (256 n)), per precision: 385x257x129 in 64 blocks,
+// k_tile_prep in FP32 0.62 ms at five, 0.573 at six, 0.560 at seven; in FP64
+// 1.23 at three, 1.106 at four, 1.24 at five.
 #ifndef ORION_PTWISE_MINB_F32
 #define ORION_PTWISE_MINB_F32 6
 #endif
@@ -429,8 +428,8 @@ template <> struct PointwiseMinBlocks<double> { static constexpr int n = ORION_P
 // One point a thread, every value it needs asked for before the first is used:
 // what bounds it is the latency of its loads, and stores in between held the
 // later ones back (385x257x129 mixed 0.83 -> 0.57 ms, plain 1.06 -> 0.72; at four
-// CTAs an SM, three the same).  Arithmetic in the storage precision S of c, mu,
-// dt (FP64 on the plain path).
+// CTAs an SM, three 0.57 and 0.74, five 0.52 and 0.82).  Arithmetic in the
+// storage precision S of c, mu, dt (FP64 on the plain path).
 template <typename S, bool DO_Q, bool DO_DT>
 __global__ void __launch_bounds__(256, ORION_STATE_MINB) k_state(const BlockDev<S>* __restrict__ blocks, const Chunk* __restrict__ chunks,
                         double* __restrict__ dt_part) {
@@ -576,10 +575,12 @@ __global__ void k_node_derivs(const BlockDev<S>* __restrict__ blocks, const Chun
   }
 }
 
-// CTAs per SM the line kernels are compiled for (register cap 65536/(256*n)),
+// Register caps of the line kernels, as CTAs per SM of 256 threads (65536/(256*n)),
 // per compute precision, measured on 385x257x129 in 64 blocks, the three
-// directions: viscous FP32 four (2.49 ms; five 2.59), FP64 two (4.50 ms without
-// spills; three 5.70); inviscid FP32 four, FP64 three (inviscid.cuh).
+// directions: viscous FP32 four (2.45 ms; three 2.49, five 2.54), where its
+// shared memory lets three CTAs be resident; FP64 two (4.55 ms without spills;
+// three 5.68); inviscid FP32 four, FP64 three, as many as are resident
+// (inviscid.cuh).
 #ifndef ORION_VISC_MINB_F32
 #define ORION_VISC_MINB_F32 4
 #endif
@@ -1331,9 +1332,8 @@ __device__ __forceinline__ void block_reduce_res(double& sum, double& mx, long l
 
 // The finish kernel asks for every value before its first store (385x257x129
 // mixed 0.67 -> 0.50 ms, plain 0.81 -> 0.66).
-// CTAs per SM it is compiled for (register cap 65536 / (NT n)):
-// on C3 four (64 registers, a few spilled) took the update stage from 7.43 to
-// 7.04 ms mixed and 11.93 to 11.54 ms plain against no cap (105 registers).
+// CTAs per SM it is compiled for (register cap 65536 / (NT n)), 385x257x129:
+// mixed 0.55 ms at three, 0.50 at four, 0.515 at five; plain 0.65, 0.65, 0.755.
 #ifndef ORION_FINISH_MINB
 #define ORION_FINISH_MINB 4
 #endif

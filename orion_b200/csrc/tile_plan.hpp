@@ -11,7 +11,7 @@ namespace orion {
 // keep their waves in 227 KB of shared memory.  An FP64 case with few lines
 // takes tiles of 64: it has SMs to spare, and a wave of two warps is shorter
 // than one of three (they share the SM's load path).  Few: at most 148 x 64
-// grid lines along i in all blocks, one small tile an SM (97x49x33 by stages
+// grid lines along i in all blocks, one small tile on each of a B200's SMs (97x49x33 by stages
 // 5.29 ms against 5.71, Euler 111x53x47 3.97 against 4.15; 193x97x65, 12,936
 // lines, 2.63 against 2.54; FP32 gained nothing).
 constexpr int kTileLinesSmall = 64;

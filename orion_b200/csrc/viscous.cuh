@@ -7,11 +7,14 @@
 // along them.  It stages the 23 values a face interpolates (velocity and
 // temperature, viscosity, Jacobian, metrics, cross derivatives) once per point
 // in shared memory, forms the faces' fluxes from them, and adds the 6th-order
-// difference to dq.  What bounds it: issue of the interpolations (FP32: a face
-// used to read 92 values from L1 and L2, each with a 64-bit address) and the
-// FP64 pipe.  The divisions by 24 and 1920 are products with the rounded
+// difference to dq (a face used to read 92 values from L1 and L2, each with a
+// 64-bit address).  What bounds it: the phases' latency and shared-memory reads,
+// 92 a face, with three (FP32) or two CTAs an SM: on 193x97x65 an instruction
+// issues in 30-48% of the cycles (FP64 23-32%), the shared-memory pipe works in
+// 33-56% and the FP64 pipe in 17-25%; the stalls are the barriers between the
+// phases and the shared-memory queue.  The divisions by 24 and 1920 are products with the rounded
 // reciprocal, corrected to the division's rounding (quotient).  385x257x129 in
-// 64 blocks, the three directions: mixed 3.34 -> 2.49 ms, plain 6.19 -> 4.50;
+// 64 blocks, the three directions: mixed 3.34 -> 2.45 ms, plain 6.19 -> 4.55;
 // 97x49x33 mixed 0.146 -> 0.054 (chunks give small grids more CTAs).
 #pragma once
 

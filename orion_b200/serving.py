@@ -9,11 +9,13 @@ own CUDA stream in quanta of graph-captured steps (orion_step_submit), so the
 work of all resident cases overlaps on the device.  With batched=True every
 resident case is stepped in one group instead, one launch per stage over the
 blocks of all of them (orion_group_*), rebuilt between quanta when cases join
-or retire.  Streams are the default: a case
-joins and retires without the others waiting, and one case's line kernels
-overlap other cases' sweep chains.  On the C4 request mix the two serve alike
-(24 requests: 8.1e8 cell-updates/s on streams, 8.5e8 in one group).  A case retires at the end
-of the first quantum in which its residual has dropped to `drop` times its
+or retire.  Streams are the default: a case joins and retires without the
+others waiting, and one case's line kernels overlap other cases' sweep chains.
+The two serve alike: 24 requests of the C4 mix, ten runs of each in turn on two
+machines, 4.9e8 to 9.2e8 cell-updates/s on streams (median 7.3e8) and 5.1e8 to
+9.3e8 in one group (7.1e8); the spread is the host's, which builds the cases
+meanwhile.  A case retires at the end of the first quantum in which its
+residual has dropped to `drop` times its
 first-step residual (rms, ResidualMonitor::compute), or after max_steps, or
 as diverged when its residual stops being finite or grows past diverge_growth
 (1e3) times the first step's; its memory is freed in stream order and the
